@@ -122,6 +122,7 @@ PowTab view(const HostPowTab& h) {
     t.log2slots = h.log2slots;
     t.lo_bits = h.lo_bits;
     t.hi_bits = h.hi_bits;
+    t.margin = h.margin;
     return t;
 }
 

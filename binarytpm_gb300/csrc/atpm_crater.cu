@@ -52,7 +52,7 @@ template <> struct Ca<MODE_FAST> {
 
 __device__ __forceinline__ float cpow4_exact(const PowTab& t, float x, int* st) {
     // x^4 corrected to this host's libm powf (atpm_powtab.cpp)
-    return pow_table_fix(t, x, dev_pow4(x), st);
+    return libm_pow4(t, x, st);
 }
 
 template <int MODE>
@@ -309,7 +309,7 @@ __global__ void __launch_bounds__(128) k_crater_equilibrium(CraterDev c, PowTab 
             float inc = c.RGH[o];
             for (int i = 0; i != nsf; ++i) inc = A::add(inc, A::mul(W[i], Vs[i * nsf + j]));
             const float x = A::div(A::add(A::mul(oma, c.RI[o]), inc), es);
-            c.stemp1[o] = (MODE == MODE_REF) ? pow_table_fix(pq, x, dev_qroot(x), c.status) : dev_qroot(x);
+            c.stemp1[o] = (MODE == MODE_REF) ? libm_qroot(pq, x, c.status) : dev_qroot(x);
         }
         __syncthreads();
     }
@@ -363,7 +363,7 @@ __global__ void k_crater_root(CraterDev c, PowTab pq, float es, float* t) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= c.nf * c.nsf) return;
     const float x = __fdiv_rn(t[i], es);
-    t[i] = (MODE == MODE_REF) ? pow_table_fix(pq, x, dev_qroot(x), c.status) : dev_qroot(x);
+    t[i] = (MODE == MODE_REF) ? libm_qroot(pq, x, c.status) : dev_qroot(x);
 }
 
 __global__ void k_crater_fill(CraterDev c, const float* t) {

@@ -59,6 +59,7 @@ atpm_status launch(atpm_crater* c, int what, std::initializer_list<float> f, voi
         t.log2slots = h.log2slots;
         t.lo_bits = h.lo_bits;
         t.hi_bits = h.hi_bits;
+        t.margin = h.margin;
         return t;
     };
     if (crater_launch(what, c->d, view(c->ctx->p4), view(c->ctx->pq), fa.data(), p0, p1, c->st))

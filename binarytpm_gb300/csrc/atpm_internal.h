@@ -36,6 +36,8 @@ struct PowTab {
     uint32_t log2slots;
     uint32_t lo_bits;     // first float (bits) covered
     uint32_t hi_bits;     // one past the last float covered
+    float margin;         // least rounding margin of any exception (below): a result
+                          // whose margin is smaller has no exception; 0 consults always
 };
 
 #ifdef __CUDACC__
@@ -57,36 +59,66 @@ __device__ __forceinline__ float pow_table_fix(const PowTab& t, float x, float v
     if (x != 0.0f) atomicOr(status, 4 /* ST_POW_RANGE */);
     return v;
 }
-// x^4 and x^3 as the device evaluates them before the exception table
-// (host twins emu_pow4 / emu_pow3): a double-float product from 2^-4 up, and
+// The rounding margin of a result s: what rounding discarded over half an
+// ulp, 1 at a tie.  powf is within a few thousandths of an ulp of the exact
+// power before its own rounding, so it differs from the correctly rounded
+// value only beside a tie; the table's build takes the least margin over all
+// its exceptions (0.9966 with this glibc, where 0.34 % of all floats lie above
+// it), and only results at or above that are looked up.  The lookup is a
+// dependent load into a table of tens of MB: eight REFERENCE revolutions of
+// 6,280 facets x 613 steps, NX 48, took 29.5 ms with a lookup for every power
+// and 13.6 ms with the margin test in front (a thread per facet both times).
+__device__ __forceinline__ bool beside_tie(float discarded, float s, float margin) {
+    return __fmul_rn(fabsf(discarded), 16777216.0f) >=
+           __fmul_rn(margin, __uint_as_float(__float_as_uint(s) & 0x7f800000u));
+}
+// libm's powf(x, 4) and powf(x, 3): a double-float product from 2^-4 up, and
 // below 2^-4, where that product underflows, one double product rounded to
-// float (x^2 is exact in double)
-__device__ __forceinline__ float dev_pow4(float x) {
+// float (x^2 is exact in double), each corrected by the exception table
+// (host twins of the uncorrected values: emu_pow4 / emu_pow3)
+__device__ __forceinline__ float libm_pow4(const PowTab& t, float x, int* status) {
     if (x < 0.0625f) {
         const double d = (double)x, d2 = __dmul_rn(d, d);
-        return __double2float_rn(__dmul_rn(d2, d2));
+        return pow_table_fix(t, x, __double2float_rn(__dmul_rn(d2, d2)), status);
     }
     const float h = __fmul_rn(x, x);
     const float l = __fmaf_rn(x, x, -h);
     const float p = __fmul_rn(h, h);
     const float e = __fmaf_rn(h, h, -p);
     const float c = __fmaf_rn(__fmul_rn(2.0f, h), l, e);
-    return __fadd_rn(p, c);
+    const float s = __fadd_rn(p, c);
+    const bool covered = x < __uint_as_float(t.hi_bits);  // false for NaN
+    if (covered && !beside_tie(__fadd_rn(__fsub_rn(p, s), c), s, t.margin)) return s;
+    return pow_table_fix(t, x, s, status);
 }
-__device__ __forceinline__ float dev_pow3(float x) {
+__device__ __forceinline__ float libm_pow3(const PowTab& t, float x, int* status) {
     if (x < 0.0625f) {
         const double d = (double)x;
-        return __double2float_rn(__dmul_rn(__dmul_rn(d, d), d));
+        return pow_table_fix(t, x, __double2float_rn(__dmul_rn(__dmul_rn(d, d), d)), status);
     }
     const float h = __fmul_rn(x, x);
     const float l = __fmaf_rn(x, x, -h);
     const float p = __fmul_rn(h, x);
     const float e = __fmaf_rn(h, x, -p);
     const float c = __fmaf_rn(l, x, e);
-    return __fadd_rn(p, c);
+    const float s = __fadd_rn(p, c);
+    const bool covered = x < __uint_as_float(t.hi_bits);
+    if (covered && !beside_tie(__fadd_rn(__fsub_rn(p, s), c), s, t.margin)) return s;
+    return pow_table_fix(t, x, s, status);
 }
 // x^0.25 through two correctly rounded double square roots (host: emu_qroot)
 __device__ __forceinline__ float dev_qroot(float x) { return (float)__dsqrt_rn(__dsqrt_rn((double)x)); }
+// libm's powf(x, 0.25)
+__device__ __forceinline__ float libm_qroot(const PowTab& t, float x, int* status) {
+    const double r = __dsqrt_rn(__dsqrt_rn((double)x));
+    const float s = __double2float_rn(r);
+    const double ulp = (double)__uint_as_float(__float_as_uint(s) & 0x7f800000u);
+    const uint32_t b = __float_as_uint(x);
+    if (b - t.lo_bits < t.hi_bits - t.lo_bits &&
+        __dmul_rn(fabs(__dsub_rn(r, (double)s)), 16777216.0) < __dmul_rn((double)t.margin, ulp))
+        return s;
+    return pow_table_fix(t, x, s, status);
+}
 #endif
 
 // per-solve control words (device memory, updated by the advance kernel)
@@ -357,15 +389,12 @@ int launch_transpose_sf(const float* in, int ntau, int nf, float* out, stream_t 
 struct HostPowTab {
     uint2* slots_dev = nullptr;
     uint32_t log2slots = 0, lo_bits = 0, hi_bits = 0;
+    float margin = 0.0f;
     int64_t exceptions = 0;
 };
 // builds the table for exponent e in {3, 4} over the positive floats below
 // 2^12, or for the quarter power (e = -4) below 2^44 (subnormals included),
 // and uploads it
 int build_pow_table(int e, HostPowTab* out, char* err, size_t errlen);
-// host emulation of the device's double-float x^e (exact IEEE ops)
-float emu_pow3(float x);
-float emu_pow4(float x);
-float emu_qroot(float x);
 
 }  // namespace atpm

@@ -15,7 +15,9 @@
 // temperatures (about 0.02 % of the low-range powers differ).
 // The table is built here by calling powf itself on every float of that
 // range (multi-threaded), so it reproduces whatever libm the host links; no
-// libm code or constant is restated.
+// libm code or constant is restated.  The build also finds the least rounding
+// margin of any exception, which lets the device skip the lookup of nearly
+// every result (atpm_internal.h).
 //
 // x^0.25 (e = -4) is evaluated on the device as (float)sqrt(sqrt((double)x))
 // (two correctly rounded square roots); about 0.06 % of glibc's powf(x, 0.25f)
@@ -27,6 +29,7 @@
 // Build with -ffp-contract=off: the emulation must round each operation.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -39,9 +42,19 @@
 
 namespace atpm {
 
+static inline uint32_t fbits(float f) { uint32_t u; std::memcpy(&u, &f, 4); return u; }
+static inline float bitsf(uint32_t u) { float f; std::memcpy(&f, &u, 4); return f; }
+
+// what rounding to s discarded, over half an ulp of s (powers of two: exact)
+static inline float margin_of(float discarded, float s) {
+    return std::fabs(discarded) * 16777216.0f / bitsf(fbits(s) & 0x7f800000u);
+}
+
 // double-float evaluation shared bit-for-bit with the device code
-// (atpm_thermal.cu: dev_pow4 / dev_pow3)
-float emu_pow4(float x) {
+// (atpm_internal.h: libm_pow4 / libm_pow3), and the result's rounding margin
+// (2, above every threshold, for the double products below 2^-4)
+static float emu_pow4(float x, float* margin) {
+    *margin = 2.0f;
     if (x < 0.0625f) {  // below 2^-4 the double-float product underflows
         const double d = (double)x, d2 = d * d;
         return (float)(d2 * d2);
@@ -51,10 +64,13 @@ float emu_pow4(float x) {
     float p = h * h;
     float e = std::fma(h, h, -p);        // h^2 = p + e exactly
     float c = std::fma(2.0f * h, l, e);  // 2hl + e (l^2 below the result's ulp)
-    return p + c;
+    float s = p + c;
+    *margin = margin_of((p - s) + c, s);
+    return s;
 }
 
-float emu_pow3(float x) {
+static float emu_pow3(float x, float* margin) {
+    *margin = 2.0f;
     if (x < 0.0625f) {
         const double d = (double)x;
         return (float)((d * d) * d);
@@ -64,13 +80,19 @@ float emu_pow3(float x) {
     float p = h * x;
     float e = std::fma(h, x, -p);        // h x = p + e exactly
     float c = std::fma(l, x, e);
-    return p + c;
+    float s = p + c;
+    *margin = margin_of((p - s) + c, s);
+    return s;
 }
 
-float emu_qroot(float x) { return (float)std::sqrt(std::sqrt((double)x)); }
-
-static inline uint32_t fbits(float f) { uint32_t u; std::memcpy(&u, &f, 4); return u; }
-static inline float bitsf(uint32_t u) { float f; std::memcpy(&f, &u, 4); return f; }
+static float emu_qroot(float x, float* margin) {
+    double r = std::sqrt(std::sqrt((double)x));
+    float s = (float)r;
+    double m = std::fabs(r - (double)s) * 16777216.0 / (double)bitsf(fbits(s) & 0x7f800000u);
+    *margin = (float)m;
+    if ((double)*margin > m) *margin = std::nextafter(*margin, 0.0f);  // never above the margin itself
+    return s;
+}
 
 static inline uint32_t slot_of(uint32_t key, uint32_t log2slots) {
     return (key * 2654435761u) >> (32 - log2slots);
@@ -86,19 +108,26 @@ int build_pow_table(int e, HostPowTab* out, char* err, size_t errlen) {
     if (nth == 0) nth = 4;
     if (nth > 64) nth = 64;
     std::vector<std::vector<uint2>> found(nth);
+    std::vector<float> least(nth, 2.0f);
     std::vector<std::thread> th;
     const uint32_t span = hi_bits - lo_bits;
     for (unsigned t = 0; t < nth; ++t) {
         th.emplace_back([&, t]() {
             uint32_t a = lo_bits + (uint32_t)((uint64_t)span * t / nth);
             uint32_t b = lo_bits + (uint32_t)((uint64_t)span * (t + 1) / nth);
+            float lo = 2.0f;
             for (uint32_t u = a; u < b; ++u) {
                 float x = bitsf(u);
                 volatile float xv = x;
                 float ref = std::pow((float)xv, ef);  // libm powf, as the reference
-                float dev = q ? emu_qroot(x) : (e == 4) ? emu_pow4(x) : emu_pow3(x);
-                if (fbits(ref) != fbits(dev)) found[t].push_back(make_uint2(u, fbits(ref)));
+                float margin;
+                float dev = q ? emu_qroot(x, &margin) : (e == 4) ? emu_pow4(x, &margin) : emu_pow3(x, &margin);
+                if (fbits(ref) != fbits(dev)) {
+                    found[t].push_back(make_uint2(u, fbits(ref)));
+                    if (margin < lo) lo = margin;
+                }
             }
+            least[t] = lo;
         });
     }
     for (auto& x : th) x.join();
@@ -130,6 +159,7 @@ int build_pow_table(int e, HostPowTab* out, char* err, size_t errlen) {
     out->log2slots = log2slots;
     out->lo_bits = lo_bits;
     out->hi_bits = hi_bits;
+    out->margin = *std::min_element(least.begin(), least.end());
     out->exceptions = (int64_t)n;
     return 0;
 }

@@ -55,14 +55,10 @@ template <> struct Ar<MODE_FAST> {
     static __device__ __forceinline__ R fabs_(R a) { return fabsf(a); }
 };
 
-__device__ __forceinline__ float pow_fix(const PowTab& t, float x, float v, int* status) {
-    return pow_table_fix(t, x, v, status);
-}
-
 template <int MODE> struct Pw;
 template <> struct Pw<MODE_REF> {
-    static __device__ __forceinline__ float p4(const PowTab& t, float x, int* st) { return pow_fix(t, x, dev_pow4(x), st); }
-    static __device__ __forceinline__ float p3(const PowTab& t, float x, int* st) { return pow_fix(t, x, dev_pow3(x), st); }
+    static __device__ __forceinline__ float p4(const PowTab& t, float x, int* st) { return libm_pow4(t, x, st); }
+    static __device__ __forceinline__ float p3(const PowTab& t, float x, int* st) { return libm_pow3(t, x, st); }
 };
 template <> struct Pw<MODE_FP64> {
     static __device__ __forceinline__ double p4(const PowTab&, double x, int*) {
@@ -771,7 +767,7 @@ __device__ __forceinline__ void column_equilibrium(const DevSolve& sv, const Bat
         const R x = A::div(A::add(A::mul(c.oma, E[o]), Q[o]), c.es);
         R tn;
         if constexpr (MODE == MODE_FP64) tn = sqrt(sqrt(x));
-        else if constexpr (MODE == MODE_REF) tn = pow_fix(b.pq, x, dev_qroot(x), sv.status);  // powf(x, 0.25f)
+        else if constexpr (MODE == MODE_REF) tn = libm_qroot(b.pq, x, sv.status);  // powf(x, 0.25f)
         else tn = dev_qroot(x);
         S1[o] = tn;
         if constexpr (MODE == MODE_FAST) {
@@ -946,7 +942,7 @@ __global__ void k_fill_initial(DevSolve sv, const void* mean, PowTab pq) {
         v = sqrt(sqrt(__ddiv_rn(__dmul_rn(sv.oma_d, m), sv.es_d)));
     } else {
         const float x = __fdiv_rn(__fmul_rn(sv.oma, m), sv.es);
-        v = (MODE == MODE_REF) ? pow_fix(pq, x, dev_qroot(x), sv.status) : dev_qroot(x);  // powf(x, 0.25f)
+        v = (MODE == MODE_REF) ? libm_qroot(pq, x, sv.status) : dev_qroot(x);  // powf(x, 0.25f)
     }
     R* temp = static_cast<R*>(sv.temp);
     R* S0 = static_cast<R*>(sv.stemp0);
