@@ -21,7 +21,7 @@ LIB = PKG / "libatpm.so"
 CUDA_HOME = Path(os.environ.get("CUDA_HOME", "/usr/local/cuda"))
 NVCC = str(CUDA_HOME / "bin" / "nvcc")
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
-CU_SOURCES = ["atpm_thermal.cu", "atpm_scatter.cu", "atpm_geom.cu", "atpm_viewfactor.cu", "atpm_spmm_tc.cu", "atpm_crater.cu", "atpm_crater_forcing.cu", "atpm_flux.cu"]
+CU_SOURCES = ["atpm_thermal.cu", "atpm_conduction_split.cu", "atpm_scatter.cu", "atpm_geom.cu", "atpm_viewfactor.cu", "atpm_spmm_tc.cu", "atpm_crater.cu", "atpm_crater_forcing.cu", "atpm_flux.cu"]
 CPP_SOURCES = ["atpm_capi.cpp", "atpm_powtab.cpp", "atpm_vfapi.cpp", "atpm_server.cpp", "atpm_crater_api.cpp"]
 
 
@@ -33,7 +33,7 @@ def _stale() -> bool:
     if not LIB.exists():
         return True
     t = LIB.stat().st_mtime
-    deps = _sources() + list(CSRC.glob("*.h")) + [PKG.parent / "include" / "atpm.h", Path(__file__)]
+    deps = _sources() + list(CSRC.glob("*.h")) + list(CSRC.glob("*.cuh")) + [PKG.parent / "include" / "atpm.h", Path(__file__)]
     return any(p.stat().st_mtime > t for p in deps if p.exists())
 
 

@@ -160,7 +160,7 @@ Layout layout(int nv, int nf, int nnz, const atpm_params& P) {
     sz[B_STATUS] = 4;
     sz[B_CTL] = sizeof(Ctl);
     sz[B_DIAG] = 4 * 8;
-    sz[B_ACT] = ((size_t)2 * nf + 5) * 4;
+    sz[B_ACT] = ((size_t)2 * nf + ACT_N) * 4;
     sz[B_MEAN] = (size_t)nf * rs;
     sz[B_RBACT] = (size_t)(nf + 127) / 128;
     Layout L;
@@ -306,12 +306,20 @@ bool warp_tail_enabled() {
     return !(e && e[0] == '0');
 }
 
-// active facets per SM up to which a revolution runs warp per facet
-// (ATPM_WARP_TAIL_PER_SM, 1..64; both forms give identical results)
+// Advancing facets per SM up to which a FAST revolution runs with 16 lanes per
+// facet (ATPM_WARP_TAIL_PER_SM, 1..64) and with 4 (kFewPerSm); every form gives
+// identical results.  ms per revolution (self-heating included) with 1 / 4 / 16
+// lanes per facet, all facets active: 0.279 / 0.184 / 0.146 at 1,280 facets (8
+// per SM; NX 56, 720 steps), 0.193 / 0.148 / 0.136 at 2,740 (18 per SM; NX 32,
+// 400 steps), 0.350 / 0.276 / 0.277 at 5,440 (36 per SM; NX 56, 720 steps),
+// 0.347 / 0.348 at 9,280 with 1 / 4 (61 per SM; NX 48, 600 steps).  Four solves
+// of 6,400 facets to convergence: 0.332 ms a revolution with a thread per facet
+// throughout, 0.202 with the split forms.
+constexpr int kFewPerSm = 56;
 int warp_tail_per_sm() {
     const char* e = std::getenv("ATPM_WARP_TAIL_PER_SM");
     const int v = e ? std::atoi(e) : 0;
-    return v >= 1 && v <= 64 ? v : 12;
+    return v >= 1 && v <= 64 ? v : 24;
 }
 
 // Device memory of solves and batches comes from the device's
@@ -567,6 +575,7 @@ Batch make_batch(atpm_context* ctx, const DevSolve* tab, int n, const int4* wm, 
     // facet: about a dozen warps per SM, where one warp per facet still beats
     // the thread-per-facet sweep's latency-bound last warps
     b.tail_limit = warp_tail_per_sm() * ctx->sm_count;
+    b.few_limit = std::max(b.tail_limit, kFewPerSm * ctx->sm_count);
     b.sms = ctx->sm_count;
     b.rem_nmb = 0;
     b.rem_ntau = 0;

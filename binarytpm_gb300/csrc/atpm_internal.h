@@ -129,6 +129,11 @@ struct Ctl {
     int numconv;    // facets converged after the last revolution
 };
 
+// act_cnt beyond the lists: lanes per facet of the split sweep (batch leader; 0:
+// the thread-per-facet kernels run), its warps in all (batch leader), and this
+// solve's first warp
+enum : int { ACT_LANES = 4, ACT_WARPS = 5, ACT_START = 6, ACT_N = 7 };
+
 struct DevSolve {
     int nf, nv, ntau, nx, revcap, mode;
     int nnz;
@@ -158,8 +163,8 @@ struct DevSolve {
     // list (r+1)&1, the conduction of r+1 reads it, k_advance of r+1 clears it
     uint8_t* rb_act;         // [ceil(nf/128)] some facet of the 128-facet row block active (FAST)
     int* act_list;           // [2][nf]
-    int* act_cnt;            // [5]: counts of the two lists, the revolution each list is for, and
-                             // (batch leader) whether this revolution runs warp per facet
+    int* act_cnt;            // [ACT_N]: counts of the two lists, the revolution each list is for, then
+                             // this revolution's split sweep (k_tail_mode)
     int* counts;             // [revcap] numconverged after each revolution
     int* status;             // ST_* bits
     Ctl* ctl;
@@ -260,9 +265,10 @@ struct Batch {
     int tc_nmax;             // largest step chunk in the batch
     int cond_variant;        // FAST conduction register/occupancy variant (1, 2, 3)
     int tc_stages;           // tensor-core pipeline depth (0: deepest that fits)
-    int warp_tail;           // 1: FAST revolutions with few active facets sweep the active list
-                             // (thread per facet; warp per facet below tail_limit)
-    int tail_limit;          // active facets of the batch up to which they do
+    int warp_tail;           // 1: FAST revolutions with few advancing facets run the lane-split sweep, and
+                             // solves at most half active sweep the list of their active facets
+    int tail_limit;          // advancing facets of the batch up to which 16 lanes share a facet,
+    int few_limit;           // and up to which 4 do
     int sms;                 // SMs of the device (persistent tensor-core grid)
     int rem_nmb, rem_ntau;   // largest row-block count / steps of the batch's solves with a
                              // sparse remainder (0: none; the remainder kernel's grid)
@@ -297,6 +303,9 @@ int launch_tc_fill(const DevSolve& s, int nkb, const int* slot, const int* lo_of
                    stream_t st);
 // part 0 W, 1 Q, 2 conduction, 3 convergence, 4 advance
 int launch_revolution_part(const Batch& b, int part, stream_t st);
+// REFERENCE / FP64 conduction of one revolution (atpm_conduction_split.cu)
+int launch_conduction_split(const Batch& b, stream_t st);
+int launch_conduction_few(const Batch& b, stream_t st);  // FAST, few advancing facets
 int launch_initial_mean(const DevSolve& s, void* mean_out, stream_t st);
 // T0 = ((1-A) mean / (eps sigma))^0.25 (x^0.25 exact to libm through pq in REFERENCE)
 int launch_fill_initial(const DevSolve& s, const void* mean, const PowTab& pq, stream_t st);

@@ -12,8 +12,9 @@
 //   k_conduction   depth column in registers, NTAU steps, Newton BC -- A1
 //                  (FAST: over the active-facet list once at most half a
 //                  solve is active)
-//   k_tail_mode, k_conduction_warp   FAST late revolutions: one warp per
-//                  active facet once the batch has few of them
+//   k_tail_mode, k_conduction_few   FAST revolutions with few advancing facets:
+//                  several lanes per facet (atpm_conduction_split.cu, as the
+//                  REFERENCE and FP64 sweeps)
 //   k_converge     shape_converged (main.cpp:1876-1909)             -- A4
 //                  (+ the active-facet lists and row-block activity)
 //   k_advance      revolution counter / stop rule (main.cpp:2522-2539)
@@ -24,74 +25,10 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
+#include "atpm_column.cuh"
 #include "atpm_internal.h"
 
 namespace atpm {
-
-// ------------------------------------------------------------------ arithmetic
-template <int MODE> struct Ar;
-template <> struct Ar<MODE_REF> {
-    using R = float;
-    static __device__ __forceinline__ R add(R a, R b) { return __fadd_rn(a, b); }
-    static __device__ __forceinline__ R sub(R a, R b) { return __fsub_rn(a, b); }
-    static __device__ __forceinline__ R mul(R a, R b) { return __fmul_rn(a, b); }
-    static __device__ __forceinline__ R div(R a, R b) { return __fdiv_rn(a, b); }
-    static __device__ __forceinline__ R fabs_(R a) { return fabsf(a); }
-};
-template <> struct Ar<MODE_FP64> {
-    using R = double;
-    static __device__ __forceinline__ R add(R a, R b) { return __dadd_rn(a, b); }
-    static __device__ __forceinline__ R sub(R a, R b) { return __dsub_rn(a, b); }
-    static __device__ __forceinline__ R mul(R a, R b) { return __dmul_rn(a, b); }
-    static __device__ __forceinline__ R div(R a, R b) { return __ddiv_rn(a, b); }
-    static __device__ __forceinline__ R fabs_(R a) { return fabs(a); }
-};
-template <> struct Ar<MODE_FAST> {
-    using R = float;
-    static __device__ __forceinline__ R add(R a, R b) { return a + b; }
-    static __device__ __forceinline__ R sub(R a, R b) { return a - b; }
-    static __device__ __forceinline__ R mul(R a, R b) { return a * b; }
-    static __device__ __forceinline__ R div(R a, R b) { return a / b; }
-    static __device__ __forceinline__ R fabs_(R a) { return fabsf(a); }
-};
-
-template <int MODE> struct Pw;
-template <> struct Pw<MODE_REF> {
-    static __device__ __forceinline__ float p4(const PowTab& t, float x, int* st) { return libm_pow4(t, x, st); }
-    static __device__ __forceinline__ float p3(const PowTab& t, float x, int* st) { return libm_pow3(t, x, st); }
-};
-template <> struct Pw<MODE_FP64> {
-    static __device__ __forceinline__ double p4(const PowTab&, double x, int*) {
-        double t2 = __dmul_rn(x, x);
-        return __dmul_rn(t2, t2);
-    }
-    static __device__ __forceinline__ double p3(const PowTab&, double x, int*) { return __dmul_rn(__dmul_rn(x, x), x); }
-};
-template <> struct Pw<MODE_FAST> {
-    static __device__ __forceinline__ float p4(const PowTab&, float x, int*) { float t2 = x * x; return t2 * t2; }
-    static __device__ __forceinline__ float p3(const PowTab&, float x, int*) { return x * x * x; }
-};
-
-// per-mode scalar views of DevSolve
-template <int MODE> struct Sc {
-    using R = typename Ar<MODE>::R;
-    R ti, oma, es, es4, m1, r, tacc, tacc10, esw;
-    __device__ __forceinline__ void load(const DevSolve& s) {
-        if constexpr (MODE == MODE_FP64) {
-            ti = s.ti_d; oma = s.oma_d; es = s.es_d; es4 = s.es4_d; m1 = s.m1_d; r = s.r_d;
-            tacc = s.tacc_d; tacc10 = s.tacc10_d; esw = s.es_w_d;
-        } else {
-            ti = s.ti; oma = s.oma; es = s.es; es4 = s.es4; m1 = s.m1; r = s.r;
-            tacc = s.tacc; tacc10 = s.tacc10; esw = s.es_w;
-        }
-    }
-    // facet f's own rotation rate (the secondary of a non-synchronous binary)
-    __device__ __forceinline__ void body(const DevSolve& s, int f) {
-        if (f < s.fsplit) return;
-        if constexpr (MODE == MODE_FP64) { m1 = s.m1_2_d; r = s.r2_d; }
-        else { m1 = s.m1_2; r = s.r2; }
-    }
-};
 
 // ------------------------------------------------------------- self-heating
 // W[f][s] = (eps*sigma) * T[s][f]^4 over a 32x32 tile, transposed in shared memory
@@ -153,96 +90,10 @@ __global__ void __launch_bounds__(1024) k_selfheat_q(Batch b) {
 }
 
 // --------------------------------------------------------------- conduction
-// One thread owns one facet's depth column (NX+1 nodes in registers) for a
-// whole revolution.  Per step it reads E, Q and the previous-revolution
-// surface temperature (coalesced across the warp), applies the FTCS update of
-// main.cpp:1510-1515, the Newton boundary of main.cpp:1533-1542 and the
-// Neumann bottom of main.cpp:1549, and records whether |stemp1-stemp0| >= TACC
-// (the shape_converged test) so no stemp history has to be re-read.
-template <int MODE, int NX>
-__device__ __forceinline__ void column_revolution(const DevSolve& sv, const Batch& b, int f) {
-    using A = Ar<MODE>;
-    using R = typename A::R;
-    const int nf = sv.nf, ntau = sv.ntau;
-    Sc<MODE> c;
-    c.load(sv);
-    c.body(sv, f);
-    R* temp = static_cast<R*>(sv.temp);
-    const R* E = static_cast<const R*>(sv.E);
-    const R* Q = static_cast<const R*>(sv.Q);
-    R* S0 = static_cast<R*>(sv.stemp0);
-    R* S1 = static_cast<R*>(sv.stemp1);
-    R T[NX + 1];
-#pragma unroll
-    for (int i = 0; i <= NX; ++i) T[i] = temp[(size_t)i * nf + f];
-    bool hot = false;
-    const int cap = sv.newton_cap;
-    int flags = 0;
-    for (int s = 0; s < ntau; ++s) {
-        const size_t o = (size_t)s * nf + f;
-        const R old = S1[o];
-        S0[o] = old;
-        R t0 = T[0];
-#pragma unroll
-        for (int i = 1; i < NX; ++i) {
-            const R t1 = T[i];
-            T[i] = A::add(T[i], A::mul(c.r, A::add(A::sub(T[i + 1], A::mul(R(2), T[i])), t0)));
-            t0 = t1;
-        }
-        const R a = A::add(A::mul(c.oma, E[o]), Q[o]);
-        R TR0 = T[0], TR1 = T[0], DT = R(1);
-        int it = 0;
-        while (DT >= c.tacc10) {
-            if (it == cap) { flags |= ST_NEWTON_CAP; break; }
-            const R sbc = A::sub(A::add(a, A::mul(c.m1, A::sub(T[1], TR0))),
-                                 A::mul(c.es, Pw<MODE>::p4(b.p4, TR0, sv.status)));
-            const R sbcd = A::add(c.m1, A::mul(c.es4, Pw<MODE>::p3(b.p3, TR0, sv.status)));
-            TR1 = A::add(TR0, A::div(sbc, sbcd));
-            DT = A::fabs_(A::sub(TR1, TR0));
-            TR0 = TR1;
-            ++it;
-        }
-        T[0] = TR1;
-        S1[o] = TR1;
-        T[NX] = T[NX - 1];
-        hot = hot || (A::fabs_(A::sub(TR1, old)) >= c.tacc);
-        if (!isfinite(TR1)) flags |= ST_NONFINITE;
-    }
-#pragma unroll
-    for (int i = 0; i <= NX; ++i) temp[(size_t)i * nf + f] = T[i];
-    sv.hot[f] = hot ? 1 : 0;
-    if (flags) atomicOr(sv.status, flags);
-}
-
-// FAST + tensor-core self-heating: eps*sigma*T^4 of the new surface
-// temperature goes straight into the hi/lo BF16 tiles the next revolution's
-// product reads (atpm_spmm_tc.cu), so no separate pass re-reads stemp1.
-// FAST arithmetic is written with explicitly rounded operations (the _rn
-// intrinsics are never contracted into a multiply-add), so the scalar, the
-// warp-per-facet and the paired forms of the sweep round alike, operation by
-// operation, whatever the compiler schedules.
-// eps sigma T^4 (with the IR absorptivity folded into es_w)
-__device__ __forceinline__ float fast_w(float es_w, float t) {
-    const float t2 = __fmul_rn(t, t);
-    return __fmul_rn(es_w, __fmul_rn(t2, t2));
-}
-// the BF16 pair of W: hi = bf16(w), lo = bf16(w - hi)
-__device__ __forceinline__ __nv_bfloat16 w_lo(float w, __nv_bfloat16 hi) {
-    return __float2bfloat16_rn(__fsub_rn(w, __bfloat162float(hi)));
-}
-
-__device__ __forceinline__ void store_w(const DevSolve& sv, int f, int s, float t) {
-    const int N = sv.tc_n;
-    const float w = fast_w(sv.es_w, t);
-    __nv_bfloat16* W = static_cast<__nv_bfloat16*>(sv.Wb);
-    const size_t base = ((size_t)(f >> 6) * sv.tc_nchunks + s / N) * (size_t)2 * N * 64;
-    const uint32_t o = swz((uint32_t)(s % N), (uint32_t)(f & 63));
-    const __nv_bfloat16 hi = __float2bfloat16_rn(w);
-    W[base + o] = hi;
-    W[base + (size_t)N * 64 + o] = w_lo(w, hi);
-    if (sv.W32) sv.W32[(size_t)f * sv.w32_ld + s] = w;
-}
-
+// REFERENCE and FP64 run the lane-split sweep (atpm_conduction_split.cu).  The
+// sweeps record whether |stemp1-stemp0| >= TACC at some step (the
+// shape_converged test), so no stemp history has to be re-read.
+//
 // FAST precision: the same update, scheduled for the FP32 pipes.
 //  * The column is advanced as offsets theta_i = T_i - T_ref from a per-facet
 //    reference (the bottom node at the start of the revolution).  The FTCS
@@ -267,27 +118,6 @@ template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
 constexpr int kFastPrefetch = 8;  // steps of forcing / flux / previous temperature in flight per facet
-
-// One FTCS node update and one Newton step of the FAST sweep, shared by the
-// thread-per-facet and the warp-per-facet forms so both round alike.
-// (up + dn) - 2 t is formed as one fma: 2 t is exact, so this is the
-// rounding of the plain expression
-__device__ __forceinline__ float ftcs_node(float r, float up, float dn, float t) {
-    return __fmaf_rn(r, __fmaf_rn(-2.0f, t, __fadd_rn(up, dn)), t);
-}
-
-// one Newton step on theta_0: sbc = (m1 (t1 - th) + a) - es TR^4 with the
-// emission folded into one multiply-add
-__device__ __forceinline__ float newton_fast(float th, float Tref, float t1, float a, float m1, float es, float es4,
-                                             float& DT) {
-    const float TR = __fadd_rn(Tref, th);
-    const float t2 = __fmul_rn(TR, TR);
-    const float sbc = __fmaf_rn(-es, __fmul_rn(t2, t2), __fmaf_rn(m1, __fsub_rn(t1, th), a));
-    const float sbcd = __fmaf_rn(es4, __fmul_rn(t2, TR), m1);
-    const float th1 = __fadd_rn(th, __fdividef(sbc, sbcd));
-    DT = fabsf(__fsub_rn(th1, th));
-    return th1;
-}
 
 template <int NX>
 __device__ __forceinline__ void column_revolution_fast(const DevSolve& sv, int f) {
@@ -429,7 +259,7 @@ __device__ __forceinline__ float2 newton_fast2(float2 th, float2 Tref, float2 t1
     const float2 t2 = f2mul(TR, TR);
     const float2 sbc = f2fma(nes, f2mul(t2, t2), f2fma(m1, f2sub(t1, th), a));
     const float2 sbcd = f2fma(es4, f2mul(t2, TR), m1);
-    const float2 th1 = f2add(th, make_float2(__fdividef(sbc.x, sbcd.x), __fdividef(sbc.y, sbcd.y)));
+    const float2 th1 = f2add(th, make_float2(quotient(sbc.x, sbcd.x), quotient(sbc.y, sbcd.y)));
     const float2 d = f2sub(th1, th);
     DT = make_float2(fabsf(d.x), fabsf(d.y));
     return th1;
@@ -571,209 +401,66 @@ __device__ __forceinline__ void column_revolution_fast2(const DevSolve& sv, int 
     if (flags) atomicOr(sv.status, flags);
 }
 
-// FAST, late revolutions: one warp per active facet.  Lane l holds depth
-// nodes 2l and 2l+1 (theta offsets, as above), and every lane also carries
-// nodes 0..3, so a step's boundary chain (node 1, then the Newton solve)
-// waits on no shuffle: the new node 3 and the next step's absorbed flux are
-// shuffled while the Newton solve runs.  The bottom node is a copy of node
-// NX-1 after every step, so node NX-1 reads its own old value for it and the
-// bottom is written once, after the revolution.  The arithmetic is that of
-// column_revolution_fast step for step.  Forcing, flux and the previous
-// temperature come in blocks of 32 steps (lane j holds step s0 + j, the next
-// block loading while this one runs); the step's outputs collect in the lane
-// of that step and are stored once per block.
-constexpr int kWarpNodes = 64;  // nodes 0..NX a warp can hold
-
-template <int NX>
-__device__ __forceinline__ void column_revolution_warp(const DevSolve& sv, int f) {
-    static_assert(NX + 1 <= kWarpNodes, "two nodes per lane");
-    static_assert(NX >= 4, "nodes 0..3 above the bottom node");
-    constexpr unsigned FULL = 0xffffffffu;
-    const int nf = sv.nf, ntau = sv.ntau;
-    const int lane = threadIdx.x & 31;
-    const bool sec = f >= sv.fsplit;
-    const float r = sec ? sv.r2 : sv.r, oma = sv.oma, es = sv.es, es4 = sv.es4, m1 = sec ? sv.m1_2 : sv.m1,
-                tacc = sv.tacc, tacc10 = sv.tacc10;
-    float* temp = static_cast<float*>(sv.temp);
-    const float* __restrict__ E = static_cast<const float*>(sv.E);
-    const float* __restrict__ Q = static_cast<const float*>(sv.Q);
-    float* __restrict__ S0 = static_cast<float*>(sv.stemp0);
-    float* __restrict__ S1 = static_cast<float*>(sv.stemp1);
-    __nv_bfloat16* Wb = static_cast<__nv_bfloat16*>(sv.Wb);
-    const int N = sv.tc_n;
-    const int na = 2 * lane, nb = 2 * lane + 1;
-    const float Tref = temp[(size_t)NX * nf + f];
-    float Ta = na <= NX ? __fsub_rn(temp[(size_t)na * nf + f], Tref) : 0.0f;
-    float Tb = nb <= NX ? __fsub_rn(temp[(size_t)nb * nf + f], Tref) : 0.0f;
-    bool hot = false;
-    int flags = 0;
-    const int cap = sv.newton_cap;
-    // nodes 0..3 on every lane (lane 0 owns 0 and 1, lane 1 owns 2 and 3)
-    float th_u = __shfl_sync(FULL, Ta, 0), t1_u = __shfl_sync(FULL, Tb, 0);
-    float t2_u = __shfl_sync(FULL, Ta, 1), t3_u = __shfl_sync(FULL, Tb, 1);
-    // lane j: (1 - A) E + Q and the previous surface temperature of step s0 + j
-    float ca = 0.0f, co = 0.0f;
-    if (lane < ntau) {
-        const size_t o = (size_t)lane * nf + f;
-        ca = __fmaf_rn(oma, E[o], Q[o]);
-        co = S1[o];
-    }
-    for (int s0 = 0; s0 < ntau; s0 += 32) {
-        float ne = 0.0f, nq = 0.0f, no = 0.0f;
-        if (s0 + 32 + lane < ntau) {
-            const size_t o = (size_t)(s0 + 32 + lane) * nf + f;
-            ne = E[o];
-            nq = Q[o];
-            no = S1[o];
-        }
-        float ts = 0.0f;
-        const int nstep = min(32, ntau - s0);
-        float a = __shfl_sync(FULL, ca, 0);
-#pragma unroll 4
-        for (int j = 0; j < nstep; ++j) {
-            const float old = __shfl_sync(FULL, co, j);
-            const float a_next = __shfl_sync(FULL, ca, (j + 1) & 31);  // unused after the block's last step
-            const float lft = __shfl_up_sync(FULL, Tb, 1);    // node na - 1
-            const float rgt = __shfl_down_sync(FULL, Ta, 1);  // node nb + 1
-            // nodes 2 .. NX-1 from old values; node NX-1 reads itself for the bottom
-            float Ta_n = Ta, Tb_n = Tb;
-            if (na >= 2 && na <= NX - 1) Ta_n = ftcs_node(r, Tb, lft, Ta);
-            if (nb >= 2 && nb <= NX - 1) Tb_n = ftcs_node(r, nb == NX - 1 ? Tb : rgt, Ta, Tb);
-            if (nb == NX) Tb_n = Ta_n;  // odd NX: the bottom copy beside node NX-1
-            // nodes 1 and 2 on every lane (uniform values)
-            const float t1n = ftcs_node(r, t2_u, th_u, t1_u);
-            const float t2n = ftcs_node(r, t3_u, t1_u, t2_u);
-            if (lane == 0) Tb_n = t1n;  // node 1, read by lane 1 next step
-            const float t3n = __shfl_sync(FULL, Tb_n, 1);
-            // the boundary solve on every lane
-            float DT;
-            float th1 = newton_fast(th_u, Tref, t1n, a, m1, es, es4, DT);
-            if (DT >= tacc10) th1 = newton_fast(th1, Tref, t1n, a, m1, es, es4, DT);
-            int it = 2;
-            while (DT >= tacc10) {
-                if (it >= cap) { flags |= ST_NEWTON_CAP; break; }
-                th1 = newton_fast(th1, Tref, t1n, a, m1, es, es4, DT);
-                ++it;
-            }
-            Ta = Ta_n;
-            Tb = Tb_n;
-            th_u = th1;
-            t1_u = t1n;
-            t2_u = t2n;
-            t3_u = t3n;
-            a = a_next;
-            const float Tsurf = __fadd_rn(Tref, th1);
-            if (lane == j) ts = Tsurf;
-            hot = hot || (fabsf(__fsub_rn(Tsurf, old)) >= tacc);
-        }
-        if (lane < nstep) {
-            const int s = s0 + lane;
-            const size_t o = (size_t)s * nf + f;
-            S0[o] = co;
-            S1[o] = ts;
-            if (Wb) {
-                const float w = fast_w(sv.es_w, ts);
-                const size_t base = ((size_t)(f >> 6) * sv.tc_nchunks + s / N) * (size_t)2 * N * 64;
-                const uint32_t off = swz((uint32_t)(s % N), (uint32_t)(f & 63));
-                const __nv_bfloat16 hi = __float2bfloat16_rn(w);
-                Wb[base + off] = hi;
-                Wb[base + (size_t)N * 64 + off] = w_lo(w, hi);
-                if (sv.W32) sv.W32[(size_t)f * sv.w32_ld + s] = w;  // 32 lanes: one 128-byte row segment
-            }
-        }
-        ca = __fmaf_rn(oma, ne, nq);
-        co = no;
-    }
-    if (!isfinite(__fadd_rn(th_u, Tref))) flags |= ST_NONFINITE;
-    if (lane == 0) Ta = th_u;  // node 0 lives in the uniform copy during the sweep
-    if constexpr ((NX & 1) == 0) {
-        const float bot = __shfl_sync(FULL, Tb, (NX - 1) >> 1);  // node NX-1
-        if (lane == (NX >> 1)) Ta = bot;
-    }
-    if (na <= NX) temp[(size_t)na * nf + f] = __fadd_rn(Tref, Ta);
-    if (nb <= NX) temp[(size_t)nb * nf + f] = __fadd_rn(Tref, Tb);
-    if (lane == 0) {
-        sv.hot[f] = hot ? 1 : 0;
-        if (flags) atomicOr(sv.status, flags);
-    }
-}
-
-// A revolution of the batch runs warp per facet when every active solve with
-// a depth sweep (TI > 0) freezes converged facets, fits a warp's nodes and
-// has the list of its active facets built for this revolution, and those
-// lists hold at most b.tail_limit facets together.  k_tail_mode decides once
-// per revolution (one warp over the solves) and leaves the answer in the
-// batch's first solve (act_cnt[4]), where both conduction kernels read it:
-// exactly one of them advances each facet.
+// How a FAST revolution's depth sweep runs, decided once per revolution from
+// the facets that advance (one warp over the solves): with few of them the
+// lane-split sweep takes every solve (k_conduction_few; its warps are dealt
+// out here, solve by solve), else the thread-per-facet kernels do.  The answer
+// goes to the batch's first solve, where all of them read it: exactly one of
+// the forms advances each facet.
 __global__ void k_tail_mode(Batch b) {
     const int lane = threadIdx.x;
-    bool ok = b.warp_tail != 0;
-    int total = 0;
-    for (int i = lane; i < b.n; i += 32) {
+    auto advancing = [&](int i) {
+        if (i >= b.n) return 0;
         const DevSolve& s = b.tab[i];
-        if (!s.ctl->active || s.ti == 0.0f) continue;
+        if (!s.ctl->active || s.ti == 0.0f) return 0;
         const int rev = s.ctl->rev;
-        if (!s.freeze || s.nx + 1 > kWarpNodes || rev < 7 || s.act_cnt[2 + (rev & 1)] != rev) ok = false;
-        else total += s.act_cnt[rev & 1];
-    }
-    ok = __all_sync(0xffffffffu, ok);
+        return active_listed(s, rev) ? s.act_cnt[rev & 1] : s.nf;
+    };
+    int total = 0;
+    for (int i = lane; i < b.n; i += 32) total += advancing(i);
     for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-    if (lane == 0) b.tab[0].act_cnt[4] = (ok && total <= b.tail_limit) ? 1 : 0;
-}
-
-__device__ __forceinline__ bool warp_tail_now(const Batch& b) { return b.tab[0].act_cnt[4] != 0; }
-
-// CTAs (4 warps each) per solve: in the late revolutions most active facets
-// belong to the one or two solves of highest thermal inertia, so one solve
-// may hold most of the batch's b.tail_limit facets (12 per SM, 1,824 on 152
-// SMs); 384 x 4 = 1,536 warps give nearly every one of them its own warp, and
-// the CTAs beyond a solve's list exit at once
-constexpr int kSparseCtas = 384;
-
-template <int NX>
-__global__ void __launch_bounds__(128) k_conduction_warp(Batch b) {
-    const int si = blockIdx.x / kSparseCtas;
-    // the batch-wide decision first: one load, and most revolutions stop here
-    if (si >= b.n || !b.warp_tail || !warp_tail_now(b)) return;
-    const DevSolve& sv = b.tab[si];
-    if (!sv.ctl->active || sv.ti == 0.0f) return;
-    const int rev = sv.ctl->rev;
-    if (rev < 7 || sv.act_cnt[2 + (rev & 1)] != rev || sv.act_cnt[rev & 1] == 0) return;
-    if constexpr (NX + 1 <= kWarpNodes) {
-        const int n = sv.act_cnt[rev & 1];
-        const int* list = sv.act_list + (size_t)(rev & 1) * sv.nf;
-        for (int k = (blockIdx.x % kSparseCtas) * 4 + (threadIdx.x >> 5); k < n; k += 4 * kSparseCtas)
-            column_revolution_warp<NX>(sv, list[k]);
+    int lanes = 0;
+    if (b.warp_tail && total <= b.few_limit) lanes = split_lanes(b.nx, total <= b.tail_limit ? kFewestLanes : kFewLanes);
+    int start = 0;
+    if (lanes) {
+        const int per = 32 / lanes;  // facets per warp
+        for (int i0 = 0; i0 < b.n; i0 += 32) {
+            const int w = (advancing(i0 + lane) + per - 1) / per;
+            int x = w;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (i0 + lane < b.n) b.tab[i0 + lane].act_cnt[ACT_START] = start + x - w;
+            start += __shfl_sync(0xffffffffu, x, 31);
+        }
+    }
+    if (lane == 0) {
+        b.tab[0].act_cnt[ACT_LANES] = lanes;
+        b.tab[0].act_cnt[ACT_WARPS] = start;
     }
 }
+
+__device__ __forceinline__ bool few_now(const Batch& b) { return b.tab[0].act_cnt[ACT_LANES] != 0; }
 
 // instequilibrium (main.cpp:1563-1612): every facet, every step, no depth
-template <int MODE>
-__device__ __forceinline__ void column_equilibrium(const DevSolve& sv, const Batch& b, int f) {
-    using A = Ar<MODE>;
-    using R = typename A::R;
+__device__ __forceinline__ void column_equilibrium_fast(const DevSolve& sv, int f) {
     const int nf = sv.nf, ntau = sv.ntau;
-    Sc<MODE> c;
-    c.load(sv);
-    const R* E = static_cast<const R*>(sv.E);
-    const R* Q = static_cast<const R*>(sv.Q);
-    R* S0 = static_cast<R*>(sv.stemp0);
-    R* S1 = static_cast<R*>(sv.stemp1);
+    const float* E = static_cast<const float*>(sv.E);
+    const float* Q = static_cast<const float*>(sv.Q);
+    float* S0 = static_cast<float*>(sv.stemp0);
+    float* S1 = static_cast<float*>(sv.stemp1);
     bool hot = false;
+    WOut w;
+    w.open(sv, f);
     for (int s = 0; s < ntau; ++s) {
         const size_t o = (size_t)s * nf + f;
-        const R old = S1[o];
+        const float old = S1[o];
         S0[o] = old;
-        const R x = A::div(A::add(A::mul(c.oma, E[o]), Q[o]), c.es);
-        R tn;
-        if constexpr (MODE == MODE_FP64) tn = sqrt(sqrt(x));
-        else if constexpr (MODE == MODE_REF) tn = libm_qroot(b.pq, x, sv.status);  // powf(x, 0.25f)
-        else tn = dev_qroot(x);
+        const float tn = dev_qroot((sv.oma * E[o] + Q[o]) / sv.es);
         S1[o] = tn;
-        if constexpr (MODE == MODE_FAST) {
-            if (sv.Wb) store_w(sv, f, s, tn);
-        }
-        hot = hot || (A::fabs_(A::sub(tn, old)) >= c.tacc);
+        if (w.tiles) w.store(s, tn);
+        hot = hot || (fabsf(tn - old) >= sv.tacc);
     }
     sv.hot[f] = hot ? 1 : 0;
 }
@@ -782,7 +469,7 @@ __device__ __forceinline__ void column_equilibrium(const DevSolve& sv, const Bat
 // of them active, freeze protocol, list built for this revolution)
 __device__ __forceinline__ bool list_mode(const Batch& b, const DevSolve& sv) {
     const int rev = sv.ctl->rev;
-    return b.warp_tail && sv.freeze && rev >= 7 && sv.act_cnt[2 + (rev & 1)] == rev && 2 * sv.act_cnt[rev & 1] <= sv.nf;
+    return b.warp_tail && active_listed(sv, rev) && 2 * sv.act_cnt[rev & 1] <= sv.nf;
 }
 // the facet-range sweep of this solve runs as pairs (variant 4, even facet
 // count) while at least 90 % of its facets are active: once facets freeze,
@@ -795,46 +482,38 @@ __device__ __forceinline__ bool pairs_here(const Batch& b, const DevSolve& sv) {
     const int rev = sv.ctl->rev;
     // no count for this revolution (every facet active before revolution 7,
     // or no lists kept): pairs; split pairs fall to the scalar sweep
-    if (!sv.freeze || rev < 7 || sv.act_cnt[2 + (rev & 1)] != rev) return true;
+    if (!active_listed(sv, rev)) return true;
     return 10 * sv.act_cnt[rev & 1] >= 9 * sv.nf;
 }
 
 // MINB: minimum resident blocks per SM requested from the register allocator
-// (FAST only; the variants trade registers for occupancy, picked at run time)
-template <int MODE, int NX, int MINB = 1>
+// (the variants trade registers for occupancy, picked at run time)
+template <int NX, int MINB>
 __global__ void __launch_bounds__(128, MINB) k_conduction(Batch b) {
     const int2 fb = b.fmap[blockIdx.x];
     const DevSolve& sv = b.tab[fb.x];
     if (!sv.ctl->active) return;
-    if constexpr (MODE == MODE_FAST) {
-        if (sv.ti != 0.0f) {
-            if (warp_tail_now(b)) return;  // k_conduction_warp runs this revolution
-            // at most half the facets active: the solve's blocks sweep its
-            // list of active facets instead of its facet range, so active
-            // facets fill whole warps and the remaining blocks exit
-            const int rev = sv.ctl->rev;
-            if (list_mode(b, sv)) {
-                const int k = fb.y + threadIdx.x;
-                if (k >= sv.act_cnt[rev & 1]) return;
-                column_revolution_fast<NX>(sv, sv.act_list[(size_t)(rev & 1) * sv.nf + k]);
-                return;
-            }
+    if (sv.ti != 0.0f) {
+        if (few_now(b)) return;  // k_conduction_few runs this revolution
+        // at most half the facets active: the solve's blocks sweep its
+        // list of active facets instead of its facet range, so active
+        // facets fill whole warps and the remaining blocks exit
+        const int rev = sv.ctl->rev;
+        if (list_mode(b, sv)) {
+            const int k = fb.y + threadIdx.x;
+            if (k >= sv.act_cnt[rev & 1]) return;
+            column_revolution_fast<NX>(sv, sv.act_list[(size_t)(rev & 1) * sv.nf + k]);
+            return;
         }
     }
     const int f = fb.y + threadIdx.x;
     if (f >= sv.nf) return;
-    if constexpr (MODE == MODE_FAST) {
-        // k_conduction_pairs sweeps the pairs whose facets are both active;
-        // a facet whose partner is frozen is swept here
-        if (sv.ti != 0.0f && pairs_here(b, sv) && !(sv.freeze && sv.conv[f ^ 1])) return;
-    }
-    const bool inst = (MODE == MODE_FP64) ? (sv.ti_d == 0.0) : (sv.ti == 0.0f);
-    if (inst) { column_equilibrium<MODE>(sv, b, f); return; }
+    // k_conduction_pairs sweeps the pairs whose facets are both active;
+    // a facet whose partner is frozen is swept here
+    if (sv.ti != 0.0f && pairs_here(b, sv) && !(sv.freeze && sv.conv[f ^ 1])) return;
+    if (sv.ti == 0.0f) { column_equilibrium_fast(sv, f); return; }
     if (sv.freeze && sv.conv[f]) return;
-    if constexpr (MODE == MODE_FAST) {
-        column_revolution_fast<NX>(sv, f);
-    }
-    else column_revolution<MODE, NX>(sv, b, f);
+    column_revolution_fast<NX>(sv, f);
 }
 
 // FAST conduction variant 4: the facet-range sweep (every revolution before
@@ -847,7 +526,7 @@ template <int NX>
 __global__ void __launch_bounds__(64, 4) k_conduction_pairs(Batch b) {
     const int2 fb = b.fmap[blockIdx.x];
     const DevSolve& sv = b.tab[fb.x];
-    if (!sv.ctl->active || sv.ti == 0.0f || !pairs_here(b, sv) || warp_tail_now(b) || list_mode(b, sv)) return;
+    if (!sv.ctl->active || sv.ti == 0.0f || !pairs_here(b, sv) || few_now(b) || list_mode(b, sv)) return;
     const int f = fb.y + 2 * threadIdx.x;
     if (f >= sv.nf || (sv.freeze && (sv.conv[f] || sv.conv[f + 1]))) return;
     column_revolution_fast2<NX>(sv, f);
@@ -1002,50 +681,21 @@ static int launch_rev_part(const Batch& b, int part, cudaStream_t st) {
         case 0: if (b.nw > 0) k_selfheat_w<MODE><<<b.nw, dim3(32, 8), 0, st>>>(b); break;
         case 1: if (b.nw > 0) k_selfheat_q<MODE><<<b.nw, dim3(32, 32), 0, st>>>(b); break;
         case 2:
-            if (MODE == MODE_FAST) k_tail_mode<<<1, 32, 0, st>>>(b);
-            if (MODE == MODE_FAST && b.cond_variant == 4) {
-                switch (b.nx) {
-#define NX_CASE(n)                                                \
-    case n:                                                       \
-        k_conduction<MODE, n, 3><<<b.nfb, 128, 0, st>>>(b);       \
-        k_conduction_pairs<n><<<b.nfb, 64, 0, st>>>(b);           \
+            if (MODE != MODE_FAST) return launch_conduction_split(b, st);
+            k_tail_mode<<<1, 32, 0, st>>>(b);
+            switch (b.nx) {
+#define NX_CASE(N)                                                                       \
+    case N:                                                                               \
+        if (b.cond_variant >= 3) k_conduction<N, 3><<<b.nfb, 128, 0, st>>>(b);            \
+        else if (b.cond_variant == 2) k_conduction<N, 2><<<b.nfb, 128, 0, st>>>(b);       \
+        else k_conduction<N, 1><<<b.nfb, 128, 0, st>>>(b);                                \
+        if (b.cond_variant == 4) k_conduction_pairs<N><<<b.nfb, 64, 0, st>>>(b);          \
         break;
-                    NX_LIST(NX_CASE)
+                NX_LIST(NX_CASE)
 #undef NX_CASE
-                    default: return 1;
-                }
-            } else if (MODE == MODE_FAST && b.cond_variant == 3) {
-                switch (b.nx) {
-#define NX_CASE(n) case n: k_conduction<MODE, n, 3><<<b.nfb, 128, 0, st>>>(b); break;
-                    NX_LIST(NX_CASE)
-#undef NX_CASE
-                    default: return 1;
-                }
-            } else if (MODE == MODE_FAST && b.cond_variant == 2) {
-                switch (b.nx) {
-#define NX_CASE(n) case n: k_conduction<MODE, n, 2><<<b.nfb, 128, 0, st>>>(b); break;
-                    NX_LIST(NX_CASE)
-#undef NX_CASE
-                    default: return 1;
-                }
-            } else {
-                switch (b.nx) {
-#define NX_CASE(n) case n: k_conduction<MODE, n><<<b.nfb, 128, 0, st>>>(b); break;
-                    NX_LIST(NX_CASE)
-#undef NX_CASE
-                    default: return 1;
-                }
+                default: return 1;
             }
-            if (MODE == MODE_FAST) {
-                const int wgrid = b.n * kSparseCtas;
-                switch (b.nx) {
-#define NX_CASE(n) case n: k_conduction_warp<n><<<wgrid, 128, 0, st>>>(b); break;
-                    NX_LIST(NX_CASE)
-#undef NX_CASE
-                    default: return 1;
-                }
-            }
-            break;
+            return launch_conduction_few(b, st);
         case 3: k_converge<<<b.nfb, 128, 0, st>>>(b); break;
         case 4: k_advance<<<(b.n + 127) / 128, 128, 0, st>>>(b); break;
         default: return 1;
@@ -1067,7 +717,7 @@ int kernels_per_revolution(const Batch& b) {
     const bool tc = b.mode == MODE_FAST && b.nq > 0;
     // k_tc_compact + k_spmm_tc (+ k_spmm_rem, k_rem_add), or W + Q
     const int selfheat = tc ? 2 + (b.rem_nmb > 0 ? 2 : 0) : (b.nw > 0 ? 2 : 0);
-    // + k_tail_mode, k_conduction_warp (+ k_conduction_pairs)
+    // + k_tail_mode, k_conduction_few (+ k_conduction_pairs)
     const int conduction = b.mode == MODE_FAST ? (b.cond_variant == 4 ? 4 : 3) : 1;
     return selfheat + conduction + 2;                    // + k_converge, k_advance
 }
