@@ -159,128 +159,247 @@ __global__ void __launch_bounds__(128) k_crater_scatter(CraterDev c, float solar
     }
 }
 
-// one revolution of finite_difference + boundary_condition for every step:
-// block = one facet, thread j = sub-facet j (its depth column in registers)
-template <int MODE, int NX>
-__global__ void __launch_bounds__(128) k_crater_revolution(CraterDev c, PowTab p4, float es, float es4, float m0,
-                                                           float dz, float tacc, float tacc2) {
-    using A = Ca<MODE>;
-    extern __shared__ float sm[];
-    const int nsf = c.nsf, ntau = c.ntau, f = blockIdx.x;
-    if (c.conv[f]) return;  // block-uniform (sfc_converged)
-    float* Vs = sm;                           // nsf*nsf
-    float* W = Vs + ((nsf * nsf + 3) & ~3);   // nsf, 16-byte aligned: eps sigma T_prev^4 of this step
-    for (int k = threadIdx.x; k < nsf * nsf; k += blockDim.x) Vs[k] = c.V[k];
-    const int j = threadIdx.x;
-    const bool act = j < nsf;
-    const float alb = c.albedo[f];
-    // the facet body's revolutions per model period scale the time step and
-    // the skin factor (175706/Run-04/thermal_GPU.cu:448-450, 539); with none
-    // given the expressions are the synchronous module's (GPU_code.cu:392-393)
-    const float w2pi = c.numrevs ? A::mul(A::mul(2.0f, c.PI), c.numrevs[f]) : A::mul(2.0f, c.PI);
-    const float m0f = c.numrevs ? A::div(A::div(w2pi, (float)ntau), A::mul(dz, dz)) : m0;
-    const float m1 = A::div(A::mul(c.ti[f], A::sqrt_(A::div(w2pi, c.rot_period))), dz);
-    const float esw = A::mul(c.ir_abs, es);  // IR_ABS * EPSSIGMA (thermal_GPU.cu:521): es when ir_abs = 1
-    const float oma = A::sub(1.0f, alb);
-    float T[NX + 1];
-    float* tp = c.temp + (size_t)f * (NX + 1) * nsf;
+// steps whose crater sums are formed together
+constexpr int kBatch = 8;
+
+// acc[k] += V[i][j] x w[i][k] over i = i0, i0 + step, ... < n, in order, on the
+// packed FP32 instructions (two steps an instruction), each lane rounded as the
+// scalar operations
+template <int MODE>
+__device__ __forceinline__ void add_view(float2 (&acc)[kBatch / 2], const float* V, const float* w, int nsf, int j,
+                                         int i0, int step, int n) {
+#pragma unroll 5
+    for (int i = i0; i < n; i += step) {
+        const float v = __ldg(V + i * nsf + j);
+        const float4 lo = *reinterpret_cast<const float4*>(w + i * kBatch);
+        const float4 hi = *reinterpret_cast<const float4*>(w + i * kBatch + 4);
+        const float2 x[kBatch / 2] = {make_float2(lo.x, lo.y), make_float2(lo.z, lo.w), make_float2(hi.x, hi.y),
+                                      make_float2(hi.z, hi.w)};
+        const float2 vv = make_float2(v, v);
 #pragma unroll
-    for (int i = 0; i <= NX; ++i) T[i] = act ? tp[(size_t)i * nsf + j] : 0.0f;
-    bool hot = false;
-    int flags = 0;
-    const size_t base = (size_t)f * ntau * nsf;
-    // the step's forcing and previous-revolution temperature are loaded one
-    // step ahead (they are not written by the current step), so the HBM
-    // latency overlaps the current step's sweep
-    float nx_old = 0.0f, nx_rgh = 0.0f, nx_ri = 0.0f;
-    if (act) {
-        nx_old = c.stemp1[base + j];
-        nx_rgh = c.RGH[base + j];
-        nx_ri = c.RI[base + j];
-    }
-    for (int s = 0; s < ntau; ++s) {
-        const size_t o = base + (size_t)s * nsf + j;
-        const float old = nx_old, rgh = nx_rgh, ri = nx_ri;
-        if (act && s + 1 < ntau) {
-            nx_old = c.stemp1[o + nsf];
-            nx_rgh = c.RGH[o + nsf];
-            nx_ri = c.RI[o + nsf];
-        }
-        // finite_difference (GPU_code.cu:377-412)
-        if (act) {
-            float t0 = T[0];
-#pragma unroll
-            for (int i = 1; i < NX; ++i) {
-                const float t1 = T[i];
-                T[i] = A::add(t1, A::mul(m0f, A::add(A::sub(T[i + 1], A::mul(2.0f, t1)), t0)));
-                t0 = t1;
-            }
-            T[NX] = T[NX - 1];
-        }
-        // boundary_condition (GPU_code.cu:418-490)
-        if (act) {
-            c.stemp0[o] = old;
-            W[j] = A::mul(esw, cpow4<MODE>(p4, old, c.status));
-        }
-        __syncthreads();
-        if (act) {
-            // W is read four at a time (one broadcast 16-byte load); the
-            // sum keeps the module's order in REFERENCE precision
-            const float4* W4 = reinterpret_cast<const float4*>(W);
-            const int n4 = nsf >> 2;
-            float inc;
+        for (int k = 0; k < kBatch / 2; ++k) {
             if constexpr (MODE == MODE_REF) {
-                inc = rgh;
-                for (int q = 0; q < n4; ++q) {
-                    const float4 w = W4[q];
-                    const float* v = Vs + (4 * q) * nsf + j;
-                    inc = A::add(inc, A::mul(w.x, v[0]));
-                    inc = A::add(inc, A::mul(w.y, v[nsf]));
-                    inc = A::add(inc, A::mul(w.z, v[2 * nsf]));
-                    inc = A::add(inc, A::mul(w.w, v[3 * nsf]));
-                }
-                for (int i = 4 * n4; i < nsf; ++i) inc = A::add(inc, A::mul(W[i], Vs[i * nsf + j]));
+                // scalar additions: ptxas may fuse a packed product and sum
+                const float2 q = __fmul2_rn(x[k], vv);
+                acc[k] = make_float2(__fadd_rn(acc[k].x, q.x), __fadd_rn(acc[k].y, q.y));
             } else {
-                // four interleaved partial sums: a quarter of the dependent chain
-                float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-                for (int q = 0; q < n4; ++q) {
-                    const float4 w = W4[q];
-                    const float* v = Vs + (4 * q) * nsf + j;
-                    a0 += w.x * v[0];
-                    a1 += w.y * v[nsf];
-                    a2 += w.z * v[2 * nsf];
-                    a3 += w.w * v[3 * nsf];
+                acc[k] = __ffma2_rn(x[k], vv, acc[k]);
+            }
+        }
+    }
+}
+
+__device__ __forceinline__ void copy_word(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+
+// one revolution of finite_difference + boundary_condition for every step:
+// block = one facet, thread j = sub-facet j (its depth column in registers).
+// The crater's mutual heating of a step needs only the previous revolution's
+// temperatures, so it is summed for kBatch steps at a time: a view factor then
+// serves kBatch multiply-adds and the steps between two barriers (one a batch)
+// are independent per thread.  The next batch's forcing arrives by cp.async
+// while this batch's steps run.  The view factors are read through L1, which
+// all CTAs of an SM share: shared memory then leaves room for as many CTAs as
+// the registers do.
+//
+// A facet's revolution is long, so a last wave of few facets would cost as
+// much as a full one.  With more facets than resident CTAs the steps are
+// therefore dealt out in kSegments pieces (take_piece): a CTA takes the next
+// (segment, facet) ticket, and the facet's column waits in memory between its
+// segments.  A segment's predecessor was taken a whole grid of tickets
+// earlier by a CTA that is running or done, so the wait for it always ends
+// (it is bounded all the same).
+//
+// With one step at a time and the matrix in shared memory the kernel was bound
+// by shared memory (125 reads for 100 multiply-adds a step) and, in REFERENCE
+// precision, by the one chain of 100 additions.  Now it is bound by instruction
+// issue (470 a sub-facet step) and, for few facets, by a step's latency.  ms a
+// revolution, before and after (720 steps): FAST, NX 48: 0.92 and 0.56 at 152
+// facets, 1.50 and 1.03 at 608, 1.78 and 1.15 at 640 (1.85 without the
+// segments), 2.92 and 2.07 at 1,216; REFERENCE, NX 48, 200 facets: 1.76 and
+// 0.88.
+constexpr int kSegments = 8;
+constexpr long long kPieceWait = 2000000000LL;  // clock cycles (about a second)
+
+// the next piece of work: facet and first step in f, s0; false when none is
+// left.  Uniform over the block.  `work`: [nf] segments done, then the ticket.
+__device__ __forceinline__ bool take_piece(const CraterDev& c, int* work, int segs, int len, int& f, int& s0,
+                                           int& piece) {
+    __shared__ int next;
+    for (;;) {
+        __syncthreads();  // the last piece is done with shared memory
+        if (threadIdx.x == 0) {
+            int t = atomicAdd(&work[c.nf], 1);
+            if (t >= segs * c.nf) t = -1;
+            else if (t >= c.nf && t / c.nf * len < c.ntau && !c.conv[t % c.nf]) {
+                const volatile int* done = &work[t % c.nf];
+                const long long begin = clock64();
+                while (*done < t / c.nf) {
+                    __nanosleep(200);
+                    if (clock64() - begin > kPieceWait) {
+                        atomicOr(c.status, ST_TC_TIMEOUT);
+                        t = -1;
+                        break;
+                    }
                 }
-                for (int i = 4 * n4; i < nsf; ++i) a0 += W[i] * Vs[i * nsf + j];
-                inc = rgh + ((a0 + a1) + (a2 + a3));
+                __threadfence();
             }
-            const float m2 = A::add(A::mul(oma, ri), inc);
-            float TR0 = T[0], TR1 = T[0], DT = 1.0f;
-            int it = 0;
-            while (DT >= tacc2) {
-                if (it == 200) { flags |= ST_NEWTON_CAP; break; }
-                const float t3 = A::mul(A::mul(A::mul(es, TR0), TR0), TR0);
-                const float sbc = A::sub(A::add(m2, A::mul(m1, A::sub(T[1], TR0))), A::mul(t3, TR0));
-                const float sbcd = A::add(m1, A::mul(A::mul(A::mul(es4, TR0), TR0), TR0));
-                TR1 = A::add(TR0, A::div(sbc, sbcd));
-                DT = fabsf(A::sub(TR1, TR0));
-                TR0 = TR1;
-                ++it;
-            }
-            T[0] = TR1;
-            c.stemp1[o] = TR1;
-            hot = hot || (fabsf(A::sub(old, TR1)) >= tacc);
-            if (!isfinite(TR1)) flags |= ST_NONFINITE;
+            next = t;
         }
         __syncthreads();
+        const int t = next;
+        if (t < 0) return false;
+        f = t % c.nf;
+        piece = t / c.nf;
+        s0 = piece * len;
+        if (!c.conv[f] && s0 < c.ntau) return true;
     }
-    if (act) {
+}
+
+// RESIDENT: CTAs an SM holds (the register allocator's bound): 4, or 2 where no
+// SM gets more than two facets (200 facets, NX 56: 0.73 against 0.85 ms)
+template <int MODE, int NX, int RESIDENT>
+__global__ void __launch_bounds__(128, RESIDENT)
+    k_crater_revolution(CraterDev c, PowTab p4, float es, float es4, float m0, float dz, float tacc, float tacc2,
+                        int* work, int segs) {
+    using A = Ca<MODE>;
+    __shared__ float stage[2][3][kBatch][128];               // previous temperature, heating, illumination -> flux
+    __shared__ __align__(16) float W[2][128 * kBatch];       // eps sigma T_prev^4 of the batch's steps
+    const int nsf = c.nsf, ntau = c.ntau;
+    const int len = (ntau + segs * kBatch - 1) / (segs * kBatch) * kBatch;  // steps of a segment
+    int f = blockIdx.x, first = 0, piece = 0;
+    while (segs > 1 ? take_piece(c, work, segs, len, f, first, piece) : piece++ == 0 && !c.conv[f]) {
+        const int end = min(ntau, first + len);
+        const int j = threadIdx.x;
+        const bool act = j < nsf;
+        const float alb = c.albedo[f];
+        // the facet body's revolutions per model period scale the time step and
+        // the skin factor (175706/Run-04/thermal_GPU.cu:448-450, 539); with none
+        // given the expressions are the synchronous module's (GPU_code.cu:392-393)
+        const float w2pi = c.numrevs ? A::mul(A::mul(2.0f, c.PI), c.numrevs[f]) : A::mul(2.0f, c.PI);
+        const float m0f = c.numrevs ? A::div(A::div(w2pi, (float)ntau), A::mul(dz, dz)) : m0;
+        const float m1 = A::div(A::mul(c.ti[f], A::sqrt_(A::div(w2pi, c.rot_period))), dz);
+        const float esw = A::mul(c.ir_abs, es);  // IR_ABS * EPSSIGMA (thermal_GPU.cu:521): es when ir_abs = 1
+        const float oma = A::sub(1.0f, alb);
+        float T[NX + 1];
+        float* tp = c.temp + (size_t)f * (NX + 1) * nsf;
 #pragma unroll
-        for (int i = 0; i <= NX; ++i) tp[(size_t)i * nsf + j] = T[i];
+        for (int i = 0; i <= NX; ++i) T[i] = act ? __ldcg(tp + (size_t)i * nsf + j) : 0.0f;
+        bool hot = false;
+        int flags = 0;
+        const size_t base = (size_t)f * ntau * nsf + j;
+        const float* V = c.V;
+        // a thread copies and reads its own words only
+        auto fetch = [&](int s0, int buf) {
+            if (act)
+                for (int k = 0; k < kBatch && s0 + k < end; ++k) {
+                    const size_t o = base + (size_t)(s0 + k) * nsf;
+                    copy_word(&stage[buf][0][k][j], c.stemp1 + o);
+                    copy_word(&stage[buf][1][k][j], c.RGH + o);
+                    copy_word(&stage[buf][2][k][j], c.RI + o);
+                }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        fetch(first, 0);
+        for (int s0 = first, buf = 0; s0 < end; s0 += kBatch, buf ^= 1) {
+            const int cnt = min(kBatch, end - s0);
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            if (act) {
+                float w[kBatch];
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k)
+                    w[k] = k < cnt ? A::mul(esw, cpow4<MODE>(p4, stage[buf][0][k][j], c.status)) : 0.0f;
+                float4* d = reinterpret_cast<float4*>(&W[buf][j * kBatch]);
+                d[0] = make_float4(w[0], w[1], w[2], w[3]);
+                d[1] = make_float4(w[4], w[5], w[6], w[7]);
+            }
+            fetch(s0 + kBatch, buf ^ 1);
+            __syncthreads();
+            if (!act) continue;
+            {
+                // incident flux of boundary_condition (GPU_code.cu:418-490): the
+                // module's order in REFERENCE precision, four partial sums in FAST
+                const float* w = W[buf];
+                float2 inc[kBatch / 2];
+#pragma unroll
+                for (int k = 0; k < kBatch / 2; ++k)
+                    inc[k] = make_float2(stage[buf][1][2 * k][j], stage[buf][1][2 * k + 1][j]);
+                if constexpr (MODE == MODE_REF) {
+                    add_view<MODE>(inc, V, w, nsf, j, 0, 1, nsf);
+                } else {
+                    const int n4 = nsf & ~3;
+                    const float2 zero = make_float2(0.0f, 0.0f);
+                    float2 x[kBatch / 2], y[kBatch / 2], z[kBatch / 2];
+#pragma unroll
+                    for (int k = 0; k < kBatch / 2; ++k) x[k] = y[k] = zero;
+                    add_view<MODE>(x, V, w, nsf, j, 0, 4, n4);
+                    add_view<MODE>(x, V, w, nsf, j, n4, 1, nsf);
+                    add_view<MODE>(y, V, w, nsf, j, 1, 4, n4);
+#pragma unroll
+                    for (int k = 0; k < kBatch / 2; ++k) {
+                        x[k] = __fadd2_rn(x[k], y[k]);
+                        y[k] = z[k] = zero;
+                    }
+                    add_view<MODE>(y, V, w, nsf, j, 2, 4, n4);
+                    add_view<MODE>(z, V, w, nsf, j, 3, 4, n4);
+#pragma unroll
+                    for (int k = 0; k < kBatch / 2; ++k)
+                        inc[k] = __fadd2_rn(inc[k], __fadd2_rn(x[k], __fadd2_rn(y[k], z[k])));
+                }
+#pragma unroll
+                for (int k = 0; k < kBatch; ++k) {
+                    const float in = (k & 1) ? inc[k / 2].y : inc[k / 2].x;
+                    stage[buf][2][k][j] = A::add(A::mul(oma, stage[buf][2][k][j]), in);
+                }
+            }
+            size_t o = base + (size_t)s0 * nsf;
+#pragma unroll 2
+            for (int k = 0; k < cnt; ++k, o += nsf) {
+                const float old = stage[buf][0][k][j], m2 = stage[buf][2][k][j];
+                // finite_difference (GPU_code.cu:377-412)
+                float t0 = T[0];
+#pragma unroll
+                for (int i = 1; i < NX; ++i) {
+                    const float t1 = T[i];
+                    T[i] = A::add(t1, A::mul(m0f, A::add(A::sub(T[i + 1], A::mul(2.0f, t1)), t0)));
+                    t0 = t1;
+                }
+                T[NX] = T[NX - 1];
+                c.stemp0[o] = old;
+                float TR0 = T[0], TR1 = T[0], DT = 1.0f;
+                int it = 0;
+                while (DT >= tacc2) {
+                    if (it == 200) { flags |= ST_NEWTON_CAP; break; }
+                    const float t3 = A::mul(A::mul(A::mul(es, TR0), TR0), TR0);
+                    const float sbc = A::sub(A::add(m2, A::mul(m1, A::sub(T[1], TR0))), A::mul(t3, TR0));
+                    const float sbcd = A::add(m1, A::mul(A::mul(A::mul(es4, TR0), TR0), TR0));
+                    TR1 = A::add(TR0, A::div(sbc, sbcd));
+                    DT = fabsf(A::sub(TR1, TR0));
+                    TR0 = TR1;
+                    ++it;
+                }
+                T[0] = TR1;
+                c.stemp1[o] = TR1;
+                hot = hot || (fabsf(A::sub(old, TR1)) >= tacc);
+                if (!isfinite(TR1)) flags |= ST_NONFINITE;
+            }
+        }
+        if (act) {
+#pragma unroll
+            for (int i = 0; i <= NX; ++i) tp[(size_t)i * nsf + j] = T[i];
+        }
+        if (flags) atomicOr(c.status, flags);
+        const int any = __syncthreads_or(hot);
+        if (threadIdx.x == 0) {
+            if (any || first == 0) c.hot[f] = any ? 1 : 0;
+            if (segs > 1) {
+                __threadfence();  // the block's column and flags before the count
+                *static_cast<volatile int*>(&work[f]) = piece + 1;
+            }
+        }
     }
-    if (__syncthreads_or(hot) && threadIdx.x == 0) c.hot[f] = 1;
-    else if (threadIdx.x == 0) c.hot[f] = 0;
-    if (flags) atomicOr(c.status, flags);
 }
 
 // roughness_inst_equilibrium (GPU_code.cu:496-548)
@@ -315,15 +434,24 @@ __global__ void __launch_bounds__(128) k_crater_equilibrium(CraterDev c, PowTab 
     }
 }
 
-// converged (GPU_code.cu:554-594)
+// converged (GPU_code.cu:554-594); a facet still changing shows it in the first
+// few steps, so the block stops at the first kConvSpan values per thread that
+// hold a change (640 facets of 100 sub-facets, 720 steps, none converged: 313
+// -> 44 us)
+constexpr int kConvSpan = 8;
 __global__ void __launch_bounds__(128) k_crater_converged(CraterDev c, float tacc) {
     const int f = blockIdx.x;
     if (c.conv[f]) return;
     const size_t n = (size_t)c.ntau * c.nsf, base = (size_t)f * n;
     int bad = 0;
-    for (size_t k = threadIdx.x; k < n; k += blockDim.x)
-        if (fabsf(c.stemp0[base + k] - c.stemp1[base + k]) >= tacc) bad = 1;
-    bad = __syncthreads_or(bad);
+    for (size_t k0 = 0; k0 < n && !bad; k0 += (size_t)kConvSpan * blockDim.x) {
+#pragma unroll
+        for (int u = 0; u < kConvSpan; ++u) {
+            const size_t k = k0 + (size_t)u * blockDim.x + threadIdx.x;
+            if (k < n && fabsf(c.stemp0[base + k] - c.stemp1[base + k]) >= tacc) bad = 1;
+        }
+        bad = __syncthreads_or(bad);
+    }
     if (threadIdx.x == 0) c.conv[f] = bad ? 0 : 1;
 }
 
@@ -335,7 +463,8 @@ __global__ void k_crater_init_mean(CraterDev c, float* out, int with_self, const
     const float inv = __fdiv_rn(1.0f, (float)c.ntau);
     const float sh = with_self ? selfh[(size_t)f * c.nsf + j] : 0.0f;
     float t = 0.0f;
-    for (int s = 0; s != c.ntau; ++s) {
+#pragma unroll 8
+    for (int s = 0; s < c.ntau; ++s) {
         const size_t o = (size_t)f * c.ntau * c.nsf + (size_t)s * c.nsf + j;
         float x = __fadd_rn(__fmul_rn(__fsub_rn(1.0f, alb), c.RI[o]), c.RGH[o]);
         if (with_self) x = __fadd_rn(x, sh);
@@ -381,6 +510,26 @@ __global__ void k_crater_fill(CraterDev c, const float* t) {
 // ------------------------------------------------------------------ launchers
 #define CRATER_NX_LIST(X) X(8) X(12) X(16) X(24) X(32) X(40) X(48) X(56) X(64)
 
+namespace {
+template <int MODE, int NX>
+int launch_crater_revolution(const CraterDev& c, const PowTab& p4, const float* a, int* work, cudaStream_t st) {
+    int dev = 0, sms = 0, per = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_crater_revolution<MODE, NX, 4>, 128, 0) != cudaSuccess)
+        return 2;
+    const int resident = sms * per;
+    const int segs = c.nf > resident ? kSegments : 1;
+    if (segs > 1 && cudaMemsetAsync(work, 0, ((size_t)c.nf + 1) * sizeof(int), st) != cudaSuccess) return 2;
+    if (c.nf <= 2 * sms)
+        k_crater_revolution<MODE, NX, 2><<<c.nf, 128, 0, st>>>(c, p4, a[0], a[1], a[2], a[3], a[4], a[5], work, segs);
+    else
+        k_crater_revolution<MODE, NX, 4><<<segs > 1 ? resident : c.nf, 128, 0, st>>>(c, p4, a[0], a[1], a[2], a[3],
+                                                                                    a[4], a[5], work, segs);
+    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+}  // namespace
+
 int crater_launch(int what, const CraterDev& c, const PowTab& p4, const PowTab& pq, const float* fargs, void* p0,
                   void* p1, stream_t stv) {
     cudaStream_t st = static_cast<cudaStream_t>(stv);
@@ -401,25 +550,16 @@ int crater_launch(int what, const CraterDev& c, const PowTab& p4, const PowTab& 
                 k_crater_scatter<MODE_REF><<<grid_fs, 128, sm, st>>>(c, fargs[0], fargs[1], (int)fargs[2], 10000);
             break;
         }
-        case 2: {  // revolution: fargs = {es, es4, m0, dz, tacc, tacc2}
-            const size_t sm = (size_t)(((c.nsf * c.nsf + 3) & ~3) + c.nsf) * 4;
-#define NX_CASE(n)                                                                                         \
-    case n:                                                                                                \
-        if (c.mode == MODE_FAST) {                                                                         \
-            cudaFuncSetAttribute(k_crater_revolution<MODE_FAST, n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-            k_crater_revolution<MODE_FAST, n><<<c.nf, 128, sm, st>>>(c, p4, fargs[0], fargs[1], fargs[2], fargs[3], fargs[4], fargs[5]); \
-        } else {                                                                                           \
-            cudaFuncSetAttribute(k_crater_revolution<MODE_REF, n>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm); \
-            k_crater_revolution<MODE_REF, n><<<c.nf, 128, sm, st>>>(c, p4, fargs[0], fargs[1], fargs[2], fargs[3], fargs[4], fargs[5]); \
-        }                                                                                                  \
-        break;
+        case 2:  // revolution: fargs = {es, es4, m0, dz, tacc, tacc2}, p0 = [nf + 1] work words
+#define NX_CASE(n)                                                                                              \
+    case n:                                                                                                     \
+        return c.mode == MODE_FAST ? launch_crater_revolution<MODE_FAST, n>(c, p4, fargs, static_cast<int*>(p0), st) \
+                                   : launch_crater_revolution<MODE_REF, n>(c, p4, fargs, static_cast<int*>(p0), st);
             switch (c.nx) {
                 CRATER_NX_LIST(NX_CASE)
                 default: return 1;
             }
 #undef NX_CASE
-            break;
-        }
         case 3: {  // equilibrium: fargs = {es}
             const size_t sm = smv + c.nsf * 4;
             cudaFuncSetAttribute(k_crater_equilibrium<MODE_REF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);

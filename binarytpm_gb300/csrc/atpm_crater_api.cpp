@@ -20,6 +20,7 @@ struct atpm_crater {
     cudaStream_t st = nullptr;
     void* mem = nullptr;
     float* scratch = nullptr;  // 2 x nf x nsf (initialisation)
+    int* work = nullptr;       // [nf + 1] pieces of a revolution done per facet, next ticket
     float* numrevs = nullptr;  // [nf] revolutions per model period (non-synchronous binaries), once set
     float PI = 0.0f, rot = 0.0f;
     bool have_model = false;
@@ -68,7 +69,7 @@ atpm_status launch(atpm_crater* c, int what, std::initializer_list<float> f, voi
     int stw = 0;
     CC(cudaMemcpy(&stw, c->d.status, 4, cudaMemcpyDeviceToHost), "status");
     if (stw & ST_NONFINITE) return atpm::fail_status(ATPM_E_NONFINITE, "crater: non-finite temperature");
-    if (stw & (ST_NEWTON_CAP | ST_SCATTER_CAP)) return atpm::fail_status(ATPM_E_ITERATION, "crater: iteration cap");
+    if (stw & (ST_NEWTON_CAP | ST_SCATTER_CAP | ST_TC_TIMEOUT)) return atpm::fail_status(ATPM_E_ITERATION, "crater: iteration cap");
     return ATPM_OK;
 }
 }  // namespace
@@ -112,7 +113,7 @@ ATPM_API atpm_status atpm_crater_create(atpm_context* ctx, int32_t nf, int32_t n
     const size_t sz[] = {(size_t)nsf * nsf * 4, 128 * 3 * 4, (size_t)nsf * 3 * 4, (size_t)nsf * 6 * 4, 100 * 2 * 4,
                          (size_t)nf, (size_t)nf * 4, (size_t)nf * 4, (size_t)nf, fs * 4, fss * 4, fs * 12, fss * 4,
                          th, th, th, th, th, thermal ? (size_t)nf * (nx + 1) * nsf * 4 : 0, 16,
-                         thermal ? (size_t)nf * nsf * 8 : 0};
+                         thermal ? (size_t)nf * nsf * 8 : 0, thermal ? ((size_t)nf + 1) * 4 : 0};
     const int n = sizeof(sz) / sizeof(sz[0]);
     size_t total = 0;
     for (int i = 0; i < n; ++i) total += al(sz[i]);
@@ -139,6 +140,7 @@ ATPM_API atpm_status atpm_crater_create(atpm_context* ctx, int32_t nf, int32_t n
     d.illumangle = (float*)ptr[12]; d.RI = (float*)ptr[13]; d.RGI = (float*)ptr[14]; d.RGH = (float*)ptr[15];
     d.stemp0 = (float*)ptr[16]; d.stemp1 = (float*)ptr[17]; d.temp = (float*)ptr[18]; d.status = (int*)ptr[19];
     c->scratch = (float*)ptr[20];
+    c->work = (int*)ptr[21];
     // trivector multipliers of the 10x10 sub-points (GPU_code.cu:669-687)
     float mult[100][2];
     for (int k = 1; k != 11; ++k)
@@ -575,7 +577,7 @@ ATPM_API atpm_status atpm_crater_inertia_difference(atpm_crater* c, float eps, f
     const float dtau = (2.0f * c->PI) / c->ntau;
     const float m0 = dtau / (dz * dz);
     const float tacc2 = tacc / 10.0f;
-    return launch(c, 2, {es, es4, m0, dz, tacc, tacc2});
+    return launch(c, 2, {es, es4, m0, dz, tacc, tacc2}, c->work);
 }
 
 ATPM_API atpm_status atpm_crater_inst_equilibrium(atpm_crater* c, float eps, float sigma) {
