@@ -549,6 +549,56 @@ atpm_status build_tc(atpm_solve* s, const atpm_shape* sh) {
     return ATPM_OK;
 }
 
+// the Gauss-Seidel order of the solve's lists, once per shape (a host pass
+// over the list entries below each row's facet: 0.4 ms for 5,440 facets and
+// 0.7 M entries)
+atpm_status ensure_gs_plan(atpm_solve* s) {
+    if (s->gs || s->P.precision == ATPM_FAST || s->nnz == 0 || (size_t)s->nf * s->rs > kGsSharedBytes) return ATPM_OK;
+    const int nf = s->nf;
+    std::vector<int> ptr(nf + 1), idx(s->nnz), mid(nf), level(nf, -1);
+    CK(cudaMemcpyAsync(ptr.data(), s->ds.dep_ptr, ptr.size() * 4, cudaMemcpyDeviceToHost, s->st));
+    CK(cudaMemcpyAsync(idx.data(), s->ds.dep_idx, idx.size() * 4, cudaMemcpyDeviceToHost, s->st));
+    CK(cudaStreamSynchronize(s->st));
+    auto gs = std::make_shared<GsShared>();
+    bool sorted = true;
+    int levels = 0;
+    for (int c = 0; c < nf && sorted; ++c) {
+        int top = -1, e = ptr[c];
+        for (; e < ptr[c + 1] && idx[e] <= c; ++e) {
+            top = std::max(top, idx[e] < c ? level[idx[e]] : -1);
+            sorted = sorted && (e == ptr[c] || idx[e - 1] <= idx[e]);
+        }
+        mid[c] = e;
+        for (; e < ptr[c + 1]; ++e) sorted = sorted && (e == ptr[c] || idx[e - 1] <= idx[e]);
+        if (ptr[c] == ptr[c + 1]) continue;  // no list: the value never changes
+        level[c] = top + 1;
+        levels = std::max(levels, top + 2);
+    }
+    if (sorted) {
+        std::vector<int> off(levels + 1, 0);
+        for (int c = 0; c < nf; ++c)
+            if (level[c] >= 0) ++off[level[c] + 1];
+        for (int l = 0; l < levels; ++l) off[l + 1] += off[l];
+        std::vector<int> at(off.begin(), off.end());
+        std::vector<int4> rows(off[levels]);
+        for (int c = 0; c < nf; ++c)
+            if (level[c] >= 0) rows[at[level[c]]++] = make_int4(c, ptr[c], mid[c], 0);
+        const size_t b_rows = align256(rows.size() * sizeof(int4)), b_off = align256(off.size() * 4);
+        CK(pool_alloc(&gs->mem, b_rows + b_off + (size_t)nf * 4, s->st));
+        char* m = static_cast<char*>(gs->mem);
+        CK(cudaMemcpyAsync(m, rows.data(), rows.size() * sizeof(int4), cudaMemcpyHostToDevice, s->st));
+        CK(cudaMemcpyAsync(m + b_rows, off.data(), off.size() * 4, cudaMemcpyHostToDevice, s->st));
+        CK(cudaMemcpyAsync(m + b_rows + b_off, mid.data(), (size_t)nf * 4, cudaMemcpyHostToDevice, s->st));
+        CK(cudaStreamSynchronize(s->st));  // the host tables must outlive their copies
+        gs->plan.rows = reinterpret_cast<const int4*>(m);
+        gs->plan.off = reinterpret_cast<const int*>(m + b_rows);
+        gs->plan.mid = reinterpret_cast<const int*>(m + b_rows + b_off);
+        gs->plan.levels = levels;
+    }
+    s->gs = gs;
+    return ATPM_OK;
+}
+
 Batch make_batch(atpm_context* ctx, const DevSolve* tab, int n, const int4* wm, int nw, const int2* fm,
                  int nfb, int mode, int nx) {
     Batch b;
@@ -1040,6 +1090,8 @@ ATPM_API atpm_status atpm_solve_footprint(const atpm_shape* sh, const atpm_param
         wb = align256((size_t)((sh->nf + 63) / 64) * nch * N * 64 * 2 * 2);
         wb += align256((size_t)sh->nf * ((P->ntau + 31) & ~31) * 4);  // W32 of the sparse remainder (when it has one)
     }
+    // the Gauss-Seidel order (shared with the solve it is cloned from)
+    if (P->precision != ATPM_FAST && P->multiple_scattering) wb += align256((size_t)sh->nf * 28 + 512);
     *bytes = (uint64_t)(L.total + wb + std::max(geo, sct) + 64 * 1024);
     return ATPM_OK;
 }
@@ -1207,6 +1259,7 @@ ATPM_API atpm_status atpm_solve_clone(atpm_solve* src, atpm_solve** out) {
     s->P = src->P;
     s->nf = src->nf; s->nv = src->nv; s->nnz = src->nnz; s->rs = src->rs;
     s->nw = src->nw; s->nfb = src->nfb; s->nq = src->nq;
+    s->gs = src->gs;
     s->vert_h = src->vert_h;
     s->fac_h = src->fac_h;
     s->have_forcing = src->have_forcing; s->have_temps = src->have_temps;
@@ -1394,8 +1447,10 @@ ATPM_API atpm_status atpm_scattering(atpm_solve* s) {
     if (launch_single_scattering(s->ds, s->st)) return fail(ATPM_E_CUDA, "single scattering launch");
     if (s->P.multiple_scattering) {
         void* work = nullptr;
+        atpm_status rp = ensure_gs_plan(s);
+        if (rp) return rp;
         CK(cudaMallocAsync(&work, multiple_scattering_work_bytes(s->ds), s->st));
-        int rc = launch_multiple_scattering(s->ds, work, s->st);
+        int rc = launch_multiple_scattering(s->ds, s->gs ? s->gs->plan : GsPlan{}, work, s->st);
         cudaFreeAsync(work, s->st);
         if (rc) return fail(ATPM_E_CUDA, "multiple scattering launch");
     }

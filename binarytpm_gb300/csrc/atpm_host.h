@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <atomic>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -47,6 +48,16 @@ struct TcShared {
     void* rem_mem = nullptr;    // the remainder's row offsets, columns and view factors
 };
 
+// A shape's Gauss-Seidel order (REFERENCE and FP64 multiple scattering), made
+// on the first scattering and shared by a solve and its clones.
+struct GsShared {
+    atpm::GsPlan plan{};
+    void* mem = nullptr;
+    ~GsShared() {
+        if (mem) cudaFree(mem);
+    }
+};
+
 struct atpm_solve {
     atpm_context* ctx = nullptr;
     atpm_params P{};
@@ -65,6 +76,7 @@ struct atpm_solve {
     size_t wb_bytes = 0;
     void* w32_mem = nullptr;  // this solve's FP32 W rows for the sparse remainder
     size_t w32_bytes = 0;
+    std::shared_ptr<const GsShared> gs;  // null until the first multiple scattering needs it
     // the stream the sparse remainder of a batch this solve leads runs on
     // beside the tensor-core product, and its fork / join events (made on
     // first use)

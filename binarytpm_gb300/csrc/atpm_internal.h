@@ -240,7 +240,16 @@ int launch_shadow_culled(const DevSolve& s, const GeomWork& g, bool all_pairs, s
 
 // scattering (atpm_scatter.cu)
 int launch_single_scattering(const DevSolve& s, stream_t st);
-int launch_multiple_scattering(const DevSolve& s, void* work, stream_t st);
+// Gauss-Seidel order of a shape's lists (ascending rows): the facets with a
+// list sorted by level, {facet, first entry, first entry above the facet, 0}
+struct GsPlan {
+    const int4* rows;  // null: no plan (unsorted lists or no lists)
+    const int* off;    // [levels + 1] first row of each level
+    const int* mid;    // [nf] first entry above the facet
+    int levels;
+};
+constexpr size_t kGsSharedBytes = 220 * 1024;  // one CTA's values (k_multi_levels)
+int launch_multiple_scattering(const DevSolve& s, const GsPlan& plan, void* work, stream_t st);
 size_t multiple_scattering_work_bytes(const DevSolve& s);
 int launch_forcing_transpose(const DevSolve& s, stream_t st);
 int launch_set_forcing(const DevSolve& s, const int32_t* shadow_d, const float* illum_d, stream_t st);
