@@ -1340,30 +1340,30 @@ ATPM_API atpm_status atpm_geometry_shadow(atpm_solve* s) {
     g.vsplit = s->sec_vertex >= 0 ? s->sec_vertex : s->nv;
     if (s->has_position)
         for (int k = 0; k < 3; ++k) g.car[k] = s->position[k];
-    const size_t nt = (size_t)s->nf * ntau;
-    const size_t bytes = align256((size_t)s->nv * ntau * 24) + align256(nt * 24) * 2 + align256(nt * 8) +
-                         align256((size_t)ntau * 32) + 64 * 8;
-    void* tmp = nullptr;
-    CK(cudaMallocAsync(&tmp, bytes, s->st));
+    const size_t nt = (size_t)s->nf * ntau, nvt = (size_t)s->nv * ntau;
+    // shadow drivers: through the central projection (the same flags);
+    // ATPM_SHADOW_CULL=0 runs the plain drivers
+    const bool shadows = (P.shadowing == 1 && s->nnz > 0) || P.shadowing == 2;
+    const bool cull = shadows && shadow_cull_enabled();
+    const size_t b_hp = align256(nvt * 24), b_rot = align256((size_t)ntau * 32), b_uv = cull ? align256(nvt * 8) : 0,
+                 b_w = cull ? align256(nvt * 4) : 0;
+    void *tmp = nullptr, *arrays = nullptr;
+    CK(cudaMallocAsync(&tmp, b_hp + b_rot + b_uv + b_w + 256 + 64 * 8, s->st));
     char* t = static_cast<char*>(tmp);
-    g.tests = reinterpret_cast<unsigned long long*>(t + bytes - 64 * 8);
-    CK(cudaMemsetAsync(g.tests, 0, 64 * 8, s->st));
     g.hp = reinterpret_cast<double*>(t);
-    t += align256((size_t)s->nv * ntau * 24);
-    g.hm = reinterpret_cast<double*>(t);
-    t += align256(nt * 24);
-    g.nrm = reinterpret_cast<double*>(t);
-    t += align256(nt * 24);
-    g.dist = reinterpret_cast<double*>(t);
-    t += align256(nt * 8);
-    g.rot = reinterpret_cast<double*>(t);
+    g.rot = reinterpret_cast<double*>(t + b_hp);
+    t += b_hp + b_rot;
+    if (cull) {
+        g.uv = t;
+        g.depth = reinterpret_cast<float*>(t + b_uv);
+    }
+    g.stats = reinterpret_cast<unsigned*>(t + b_uv + b_w);
+    g.tests = reinterpret_cast<unsigned long long*>(t + b_uv + b_w + 256);
+    CK(cudaMemsetAsync(g.tests, 0, 64 * 8, s->st));
     g.rot2 = g.rot + 2 * (size_t)ntau;
     cudaError_t e = cudaMemcpyAsync((void*)g.rot, rot.data(), rot.size() * 8, cudaMemcpyHostToDevice, s->st);
     int rc = 0;
     if (e == cudaSuccess) rc = launch_geometry(s->ds, g, s->st);
-    // shadow drivers: the projected-box cull in front of the exact test (the
-    // same flags); ATPM_SHADOW_CULL=0 runs the plain drivers
-    const bool shadows = (P.shadowing == 1 && s->nnz > 0) || P.shadowing == 2;
     // the shadow drivers' time (events) and exact-test count (culled drivers)
     cudaEvent_t sh0 = nullptr, sh1 = nullptr;
     unsigned long long counts[64] = {};
@@ -1371,14 +1371,27 @@ ATPM_API atpm_status atpm_geometry_shadow(atpm_solve* s) {
     if (e == cudaSuccess && !rc && shadows) {
         if (cudaEventCreate(&sh0) == cudaSuccess && cudaEventCreate(&sh1) == cudaSuccess)
             cudaEventRecord(sh0, s->st);
-        int cr = shadow_cull_enabled() ? launch_shadow_culled(s->ds, g, P.shadowing == 2, s->st) : -1;
-        culled = cr != -1;
-        if (cr == -1) cr = (P.shadowing == 2) ? launch_shadow_allpairs(s->ds, g, s->st)
-                                              : launch_shadow_deplist(s->ds, g, s->st);
-        rc = cr;
+        rc = cull ? launch_shadow_culled(s->ds, g, P.shadowing == 2, s->st) : -1;
+        culled = rc != -1;
+        if (!culled) {
+            rc = 0;
+            const size_t b_v = align256(nt * 24);
+            e = cudaMallocAsync(&arrays, 2 * b_v + align256(nt * 8), s->st);
+            if (e == cudaSuccess) {
+                char* p = static_cast<char*>(arrays);
+                g.hm = reinterpret_cast<double*>(p);
+                g.nrm = reinterpret_cast<double*>(p + b_v);
+                g.dist = reinterpret_cast<double*>(p + 2 * b_v);
+                rc = launch_geometry_arrays(s->ds, g, s->st);
+                if (!rc) rc = (P.shadowing == 2) ? launch_shadow_allpairs(s->ds, g, s->st)
+                                                 : launch_shadow_deplist(s->ds, g, s->st);
+            }
+        }
         if (sh1) cudaEventRecord(sh1, s->st);
-        if (!rc) e = cudaMemcpyAsync(counts, g.tests, sizeof counts, cudaMemcpyDeviceToHost, s->st);
+        if (!rc && e == cudaSuccess)
+            e = cudaMemcpyAsync(counts, g.tests, sizeof counts, cudaMemcpyDeviceToHost, s->st);
     }
+    if (arrays) cudaFreeAsync(arrays, s->st);
     cudaFreeAsync(tmp, s->st);
     cudaError_t e2 = cudaStreamSynchronize(s->st);  // `rot` must outlive the copy
     s->last_shadow_ms = 0.0;

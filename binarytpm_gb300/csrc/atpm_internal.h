@@ -216,26 +216,32 @@ using stream_t = void*;
 // geometry + shadowing (atpm_geom.cu)
 struct GeomWork {
     double* hp;      // [nv][ntau][3] heliocentric vertex positions
-    double* hm;      // [nf][ntau][3] heliocentric facet midpoints
-    double* nrm;     // [nf][ntau][3] unit normals
-    double* dist;    // [nf][ntau] |hm|
     const double* rot;  // [ntau][2] cos, sin of the rotation angle (host libm)
     const double* rot2; // the same for vertices >= vsplit (non-synchronous secondary)
     int vsplit;         // first vertex of the secondary (nv when synchronous)
     double tm[9];    // pole transformation matrix
     double car[3];   // heliocentric centre (km)
-    unsigned long long* tests;  // [64] exact ray-triangle tests of the culled drivers (or null)
+    unsigned long long* tests;  // [64] ray-triangle tests of the culled drivers (or null)
+    // the culled drivers' projection (null: not wanted)
+    void* uv;        // [nv][ntau] float2
+    float* depth;    // [nv][ntau]
+    unsigned* stats; // [4]
+    // the plain drivers' arrays (null until launch_geometry_arrays is wanted)
+    double* hm;      // [nf][ntau][3] heliocentric facet midpoints
+    double* nrm;     // [nf][ntau][3] unit normals
+    double* dist;    // [nf][ntau] |hm|
 };
 int launch_geometry(const DevSolve& s, const GeomWork& g, stream_t st);
+int launch_geometry_arrays(const DevSolve& s, const GeomWork& g, stream_t st);
 // vertex positions of every step (into g.hp), then the crater model's Sun
 // vector [nfc][ntau][3] and the facet shadow flags [nfc][ntau] of facets
 // f0 .. f0 + nfc - 1
 int launch_crater_sun(const DevSolve& s, const GeomWork& g, int f0, int nfc, float* sun, int* shadow, stream_t st);
 int launch_shadow_deplist(const DevSolve& s, const GeomWork& g, stream_t st);
 int launch_shadow_allpairs(const DevSolve& s, const GeomWork& g, stream_t st);
-// the same flags with the projected-box cull in front of the exact test
-// (dependent lists, or all pairs over a per-step grid); -1: not applicable
-// (body too close to the origin for a central projection), use the above
+// the same flags through the central projection (dependent lists, or all
+// pairs over a per-step grid); -1: not applicable (body too close to the
+// origin for a central projection), use the above
 int launch_shadow_culled(const DevSolve& s, const GeomWork& g, bool all_pairs, stream_t st);
 
 // scattering (atpm_scatter.cu)
