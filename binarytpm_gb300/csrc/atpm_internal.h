@@ -259,6 +259,7 @@ int launch_multiple_scattering(const DevSolve& s, const GsPlan& plan, void* work
 size_t multiple_scattering_work_bytes(const DevSolve& s);
 int launch_forcing_transpose(const DevSolve& s, stream_t st);
 int launch_set_forcing(const DevSolve& s, const int32_t* shadow_d, const float* illum_d, stream_t st);
+int launch_widen_flags(const uint8_t* src, int32_t* dst, size_t n, stream_t st);
 // [rows][cols] -> [cols][rows], element sizes 4 or 8 bytes (float / double)
 int launch_transpose(const void* src, int src_bytes, void* dst, int dst_bytes, size_t rows, size_t cols, stream_t st);
 

@@ -309,6 +309,17 @@ __global__ void __launch_bounds__(256) k_transpose(const Ri* src, Ro* dst, size_
     }
 }
 
+// flags [nf][ntau] as the 32-bit words of the host interface, four at a time
+__global__ void __launch_bounds__(256) k_widen_flags(const uint8_t* src, int32_t* dst, size_t n) {
+    const size_t i = 4 * ((size_t)blockIdx.x * blockDim.x + threadIdx.x);
+    if (i + 4 <= n) {
+        const uchar4 v = *reinterpret_cast<const uchar4*>(src + i);
+        *reinterpret_cast<int4*>(dst + i) = make_int4(v.x, v.y, v.z, v.w);
+    } else {
+        for (size_t j = i; j < n; ++j) dst[j] = src[j];
+    }
+}
+
 template <class R>
 __global__ void k_set_forcing(DevSolve sv, const int32_t* shadow, const float* illum) {
     const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -421,6 +432,11 @@ int launch_transpose(const void* src, int src_bytes, void* dst, int dst_bytes, s
         k_transpose<double, float><<<grd, blk, 0, st>>>(static_cast<const double*>(src), static_cast<float*>(dst), rows, cols);
     else
         return 1;
+    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+int launch_widen_flags(const uint8_t* src, int32_t* dst, size_t n, stream_t stv) {
+    k_widen_flags<<<(unsigned)((n / 4 + 256) / 256), 256, 0, static_cast<cudaStream_t>(stv)>>>(src, dst, n);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
