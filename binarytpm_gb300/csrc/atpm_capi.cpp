@@ -2004,32 +2004,38 @@ atpm_status disk_flux_impl(atpm_solve* s, const double* observer, const int32_t*
     a.eps = emissivity;
     const double cvel = 299792458.0, hcon = 6.626068963e-34, kcon = 1.380650424e-23;
     a.nwl = nwl;
-    a.hc = hcon * cvel;
     for (int l = 0; l < nwl; ++l) {
         const double wl = wavelength_um[l] * 1.0e-6;
         a.b1[l] = (2.0 * hcon * cvel * cvel) / std::pow(wl, 5.0);
-        a.lk[l] = wl * kcon;
+        a.hl[l] = (hcon * cvel) / (wl * kcon);
     }
-    std::vector<uint8_t> vis;
-    if (visibility) {
-        vis.resize((size_t)nf * ntau);
-        for (size_t i = 0; i < vis.size(); ++i) vis[i] = visibility[i] ? 1 : 0;
-    }
+    const size_t nt = (size_t)nf * ntau;
     const size_t b_rot = align256(rot.size() * 8), b_part = align256(flux_partial_bytes(s->ds, nwl)),
-                 b_out = align256((size_t)ntau * nwl * 8), b_vis = align256(vis.size()),
-                 b_geo = rough ? align256((size_t)rough->nsf * 4 * 8) : 0;
+                 b_out = align256((size_t)ntau * nwl * 8), b_vis = visibility ? align256(nt) : 0,
+                 b_flags = visibility ? align256(nt * 4) : 0, b_geo = rough ? align256((size_t)rough->nsf * 4 * 8) : 0,
+                 b_hp = align256((size_t)s->nv * ntau * 24), b_area = align256((size_t)nf * 8);
     void* tmp = nullptr;
-    CK(cudaMallocAsync(&tmp, b_rot + b_part + b_out + b_vis + b_geo, s->st));
+    CK(cudaMallocAsync(&tmp, b_rot + b_part + b_out + b_vis + b_flags + b_geo + b_hp + b_area, s->st));
     char* t = static_cast<char*>(tmp);
-    a.rot = reinterpret_cast<const double*>(t);
+    auto take = [&t](size_t bytes) {
+        char* p = t;
+        t += bytes;
+        return p;
+    };
+    a.rot = reinterpret_cast<const double*>(take(b_rot));
     a.rot2 = a.rot + 2 * (size_t)ntau;
-    a.partial = reinterpret_cast<double*>(t + b_rot);
-    a.out = reinterpret_cast<double*>(t + b_rot + b_part);
-    a.visible = visibility ? reinterpret_cast<const uint8_t*>(t + b_rot + b_part + b_out) : nullptr;
-    if (rough) a.sub_geo = reinterpret_cast<const double*>(t + b_rot + b_part + b_out + b_vis);
+    a.partial = reinterpret_cast<double*>(take(b_part));
+    a.out = reinterpret_cast<double*>(take(b_out));
+    a.hp = reinterpret_cast<double*>(take(b_hp));
+    a.area = reinterpret_cast<double*>(take(b_area));
+    if (visibility) {
+        a.visible = reinterpret_cast<const uint8_t*>(take(b_vis));
+        a.flags = reinterpret_cast<const int32_t*>(take(b_flags));
+    }
+    if (rough) a.sub_geo = reinterpret_cast<const double*>(take(b_geo));
     cudaError_t e = cudaMemcpyAsync((void*)a.rot, rot.data(), rot.size() * 8, cudaMemcpyHostToDevice, s->st);
     if (e == cudaSuccess && visibility)
-        e = cudaMemcpyAsync((void*)a.visible, vis.data(), vis.size(), cudaMemcpyHostToDevice, s->st);
+        e = cudaMemcpyAsync((void*)a.flags, visibility, nt * 4, cudaMemcpyHostToDevice, s->st);
     if (e == cudaSuccess && rough)
         e = cudaMemcpyAsync((void*)a.sub_geo, rough->sub_geo, (size_t)rough->nsf * 4 * 8, cudaMemcpyHostToDevice, s->st);
     int rc = 0;

@@ -11,12 +11,22 @@
 // to the observer, A_f the facet area as the stage leaves it (computed at the
 // last step of its geometry loop).
 //
-//   k_flux_partial  one thread per (facet, step): rotate the facet's three
-//                   vertices (host-libm rotation table, pole matrix), build
-//                   its frame, weight and Planck terms; a fixed-order
-//                   shared-memory tree sums each 256-facet block
+//   k_flux_vertices every vertex at every step (host-libm rotation table, pole
+//                   matrix), once instead of for each facet around it
+//   k_flux_area     the facets' areas
+//   k_flux_flags    the caller's visibility words, transposed to bytes
+//   k_flux_partial  one thread per (facet, step): weight and Planck terms; a
+//                   fixed-order sum over each 256-facet block
 //   k_flux_sum      sums the block partials of every (step, wavelength) in
 //                   block order: the result does not depend on scheduling
+//
+// All of it is FP64, on a part whose FP64 rate is 1/64 of FP32, so FP64
+// operations are what it costs.  The positions are the stage's, operand by
+// operand (its body lies 1e11 m away from an origin while its shape keeps its
+// own units, so their rounding shows in the normals); from them on, cosines come
+// from one reciprocal square root instead of a facet frame, acos and cos, and a
+// wavelength costs one exp and one reciprocal: 13.0 -> 4.0 ms for 21,760 facets,
+// 720 steps and three wavelengths.
 //
 // The rough-surface sum (observe, wise_main.cpp:695-727) replaces each
 // facet's own term by its crater's: the sub-facets with a visible fraction
@@ -37,7 +47,10 @@ __device__ __forceinline__ double temp_at(const DevSolve& s, int f, int step) {
     return (double)static_cast<const R*>(s.stemp1)[(size_t)step * s.nf + f];
 }
 
-__device__ __forceinline__ void vertex_at(const DevSolve& s, const FluxArgs& a, int v, int step, double* out) {
+__global__ void __launch_bounds__(256) k_flux_vertices(DevSolve s, FluxArgs a) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)s.nv * s.ntau) return;
+    const int step = (int)(i / s.nv), v = (int)(i % s.nv);
     const double* e = s.vert + 3 * v;
     const double* rt = (v < a.vsplit) ? a.rot : a.rot2;
     const double c = rt[2 * step], sn = rt[2 * step + 1];
@@ -47,120 +60,148 @@ __device__ __forceinline__ void vertex_at(const DevSolve& s, const FluxArgs& a, 
     rq[2] = e[2];
 #pragma unroll
     for (int k = 0; k < 3; ++k)
-        out[k] = __dadd_rn(a.car[k], __dadd_rn(__dadd_rn(__dmul_rn(a.tm[3 * k], rq[0]), __dmul_rn(a.tm[3 * k + 1], rq[1])),
-                                               __dmul_rn(a.tm[3 * k + 2], rq[2])));
+        a.hp[3 * i + k] =
+            __dadd_rn(a.car[k], __dadd_rn(__dadd_rn(__dmul_rn(a.tm[3 * k], rq[0]), __dmul_rn(a.tm[3 * k + 1], rq[1])),
+                                          __dmul_rn(a.tm[3 * k + 2], rq[2])));
 }
 
-__device__ __forceinline__ void edges_at(const DevSolve& s, const FluxArgs& a, int f, int step, double* hm, double* nc0,
-                                         double* nc1) {
-    const int* fv = s.fac + 3 * f;
-    double h0[3], h1[3], h2[3];
-    vertex_at(s, a, fv[0], step, h0);
-    vertex_at(s, a, fv[1], step, h1);
-    vertex_at(s, a, fv[2], step, h2);
+// a facet's corners at a step, its first edge and its normal (not scaled)
+struct Facet {
+    double sum[3], edge[3], n[3];
+    __device__ __forceinline__ Facet(const DevSolve& s, const FluxArgs& a, int f, int step) {
+        const double* hp = a.hp + (size_t)step * s.nv * 3;
+        const int* fv = s.fac + 3 * f;
+        const double *h0 = hp + 3 * (size_t)fv[0], *h1 = hp + 3 * (size_t)fv[1], *h2 = hp + 3 * (size_t)fv[2];
+        double nc1[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        hm[k] = __ddiv_rn(__dadd_rn(__dadd_rn(h0[k], h1[k]), h2[k]), 3.0);
-        nc0[k] = __dsub_rn(h1[k], h0[k]);
-        nc1[k] = __dsub_rn(h2[k], h0[k]);
+        for (int k = 0; k < 3; ++k) {
+            const double x = __ldg(h0 + k), y = __ldg(h1 + k), z = __ldg(h2 + k);
+            sum[k] = __dadd_rn(__dadd_rn(x, y), z);
+            edge[k] = __dsub_rn(y, x);
+            nc1[k] = __dsub_rn(z, x);
+        }
+        n[0] = __dsub_rn(__dmul_rn(edge[1], nc1[2]), __dmul_rn(edge[2], nc1[1]));
+        n[1] = __dsub_rn(__dmul_rn(edge[2], nc1[0]), __dmul_rn(edge[0], nc1[2]));
+        n[2] = __dsub_rn(__dmul_rn(edge[0], nc1[1]), __dmul_rn(edge[1], nc1[0]));
+    }
+};
+
+__device__ __forceinline__ double dot3(const double* a, const double* b) {
+    return __dadd_rn(__dadd_rn(__dmul_rn(a[0], b[0]), __dmul_rn(a[1], b[1])), __dmul_rn(a[2], b[2]));
+}
+
+// area as the stage leaves it: from the last step of its geometry loop
+__global__ void __launch_bounds__(256) k_flux_area(DevSolve s, FluxArgs a) {
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= s.nf) return;
+    const Facet t(s, a, f, s.ntau - 1);
+    a.area[f] = __ddiv_rn(__dsqrt_rn(dot3(t.n, t.n)), 2.0);
+}
+
+// [nf][ntau] words -> [ntau][nf] bytes
+__global__ void __launch_bounds__(256) k_flux_flags(const int32_t* src, uint8_t* dst, int nf, int ntau) {
+    __shared__ uint8_t t[32][33];
+    const int f0 = blockIdx.y * 32, s0 = blockIdx.x * 32;
+    for (int j = threadIdx.y; j < 32; j += 8) {
+        const int f = f0 + j, s = s0 + threadIdx.x;
+        if (f < nf && s < ntau) t[j][threadIdx.x] = src[(size_t)f * ntau + s] ? 1 : 0;
+    }
+    __syncthreads();
+    for (int j = threadIdx.y; j < 32; j += 8) {
+        const int s = s0 + j, f = f0 + threadIdx.x;
+        if (f < nf && s < ntau) dst[(size_t)s * nf + f] = t[threadIdx.x][j];
     }
 }
 
-__device__ __forceinline__ void cross(const double* a, const double* b, double* n) {
-    n[0] = __dsub_rn(__dmul_rn(a[1], b[2]), __dmul_rn(a[2], b[1]));
-    n[1] = __dsub_rn(__dmul_rn(a[2], b[0]), __dmul_rn(a[0], b[2]));
-    n[2] = __dsub_rn(__dmul_rn(a[0], b[1]), __dmul_rn(a[1], b[0]));
-}
-
-__device__ __forceinline__ double norm3(const double* v) {
-    return __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(v[0], v[0]), __dmul_rn(v[1], v[1])), __dmul_rn(v[2], v[2])));
+// (2hc^2 / lambda^5) * (1 / (exp(hc / (lambda k T)) - 1)), 0 where that is NaN
+__device__ __forceinline__ double planck(const FluxArgs& a, int l, double inv_t) {
+    const double b = a.b1[l] / (exp(a.hl[l] * inv_t) - 1.0);
+    return b == b ? b : 0.0;
 }
 
 template <class R, bool ROUGH>
 __global__ void __launch_bounds__(kFluxThreads) k_flux_partial(DevSolve s, FluxArgs a) {
-    __shared__ double red[kFluxThreads];
-    const int step = blockIdx.y;
+    constexpr int kWarps = kFluxThreads / 32;
+    __shared__ double red[kMaxFluxWavelengths][kWarps];
+    // rough: each facet's unit view vector in its frame and its weight
+    __shared__ double view[ROUGH ? kFluxThreads : 1][4];
+    const int step = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int f = blockIdx.x * kFluxThreads + threadIdx.x;
     double term[kMaxFluxWavelengths];
 #pragma unroll
     for (int l = 0; l < kMaxFluxWavelengths; ++l) term[l] = 0.0;
-    if (f < s.nf && (!a.visible || a.visible[(size_t)f * s.ntau + step])) {
-        double hm[3], nc0[3], nc1[3], n[3];
-        // area as the stage leaves it: from the last step of its geometry loop
-        edges_at(s, a, f, s.ntau - 1, hm, nc0, nc1);
-        cross(nc0, nc1, n);
-        const double area = __ddiv_rn(norm3(n), 2.0);
-        edges_at(s, a, f, step, hm, nc0, nc1);
-        cross(nc0, nc1, n);
-        const double nn = norm3(n);
+    double weight = 0.0;
+    if (f < s.nf && (!a.visible || a.visible[(size_t)step * s.nf + f])) {
+        const Facet t(s, a, f, step);
+        double ov[3];  // from the facet to the observer
 #pragma unroll
-        for (int k = 0; k < 3; ++k) n[k] = __ddiv_rn(n[k], nn);
-        const double x = norm3(nc0);
-        double xh[3], y[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) xh[k] = __ddiv_rn(nc0[k], x);
-        cross(n, xh, y);
-        double ov[3];
-#pragma unroll
-        for (int k = 0; k < 3; ++k) ov[k] = __dsub_rn(hm[k], a.obs[k]);
-        const double o = norm3(ov);
-        // view vector in the facet frame (rows x^, y, n)
-        const double v0 = -__dadd_rn(__dadd_rn(__dmul_rn(xh[0], ov[0]), __dmul_rn(xh[1], ov[1])), __dmul_rn(xh[2], ov[2]));
-        const double v1 = -__dadd_rn(__dadd_rn(__dmul_rn(y[0], ov[0]), __dmul_rn(y[1], ov[1])), __dmul_rn(y[2], ov[2]));
-        const double v2 = -__dadd_rn(__dadd_rn(__dmul_rn(n[0], ov[0]), __dmul_rn(n[1], ov[1])), __dmul_rn(n[2], ov[2]));
-        const double va = acos(__ddiv_rn(v2, o));
-        if (!(va > (3.141592653589793 / 2.0))) {
-            const double d = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(v0, v0), __dmul_rn(v1, v1)), __dmul_rn(v2, v2)));
+        for (int k = 0; k < 3; ++k) ov[k] = a.obs[k] - t.sum[k] * (1.0 / 3.0);
+        const double oo = dot3(ov, ov), nn = dot3(t.n, t.n), no = dot3(t.n, ov);
+        // cosine toward the observer; above 1 the stage's acos is NaN and the
+        // facet contributes nothing
+        const double c = no > 0.0 ? no * rsqrt(nn * oo) : -1.0;
+        if (c > 0.0 && c <= 1.0) {
+            weight = a.eps * a.area[f] / oo;
             if constexpr (!ROUGH) {
-                double mult = __ddiv_rn(__dmul_rn(__dmul_rn(a.eps, area), cos(va)), __dmul_rn(d, d));
-                if (mult != mult) mult = 0.0;
-                const double T = temp_at<R>(s, f, step);
-                for (int l = 0; l < a.nwl; ++l) {
-                    // (2hc^2 / lambda^5) * (1 / (exp(hc / (lambda k T)) - 1))
-                    const double arg = __ddiv_rn(a.hc, __dmul_rn(a.lk[l], T));
-                    double b = __dmul_rn(a.b1[l], __ddiv_rn(1.0, __dsub_rn(exp(arg), 1.0)));
-                    if (b != b) b = 0.0;
-                    term[l] = __dmul_rn(b, mult);
-                }
-            } else {
-                // the facet's crater: every sub-facet with a visible fraction
-                // > 0, its view angle from the view vector in the facet frame
-                // (wise_main.cpp:515), in sub-facet order; then the facet's
-                // share of the crater's projected area (wise_main.cpp:718)
-                const size_t base = ((size_t)f * s.ntau + step) * (size_t)a.nsf;
-                double sfc[kMaxFluxWavelengths];
+                weight *= c;
+                const double inv_t = 1.0 / temp_at<R>(s, f, step);
 #pragma unroll
-                for (int l = 0; l < kMaxFluxWavelengths; ++l) sfc[l] = 0.0;
-                const double dd = __dmul_rn(d, d);
-                for (int j = 0; j < a.nsf; ++j) {
-                    const double vis = (double)a.sub_vis[base + j];
-                    if (!(vis > 0.0)) continue;
-                    const double* g = a.sub_geo + 4 * j;
-                    const double c = __dadd_rn(__dadd_rn(__dmul_rn(v0, g[0]), __dmul_rn(v1, g[1])), __dmul_rn(v2, g[2]));
-                    const double vj = acos(__ddiv_rn(c, d));
-                    double mult = __ddiv_rn(__dmul_rn(__dmul_rn(__dmul_rn(a.eps, g[3]), vis), cos(vj)), dd);
-                    if (mult != mult) mult = 0.0;
-                    const double T = (double)a.sub_T[base + j];
-                    for (int l = 0; l < a.nwl; ++l) {
-                        const double arg = __ddiv_rn(a.hc, __dmul_rn(a.lk[l], T));
-                        double b = __dmul_rn(a.b1[l], __ddiv_rn(1.0, __dsub_rn(exp(arg), 1.0)));
-                        if (b != b) b = 0.0;
-                        sfc[l] = __dadd_rn(sfc[l], __dmul_rn(b, mult));
-                    }
+                for (int l = 0; l < kMaxFluxWavelengths; ++l)
+                    if (l < a.nwl) term[l] = planck(a, l, inv_t) * weight;
+            } else {
+                // the view vector in the facet's frame (rows x^, y, n)
+                const double rx = rsqrt(dot3(t.edge, t.edge)), rn = rsqrt(nn), ro = rsqrt(oo);
+                double x[3], n[3], u[3];
+#pragma unroll
+                for (int k = 0; k < 3; ++k) {
+                    x[k] = t.edge[k] * rx;
+                    n[k] = t.n[k] * rn;
+                    u[k] = ov[k] * ro;
                 }
-                for (int l = 0; l < a.nwl; ++l) term[l] = __ddiv_rn(__dmul_rn(sfc[l], area), a.sub_total);
+                const double y[3] = {n[1] * x[2] - n[2] * x[1], n[2] * x[0] - n[0] * x[2], n[0] * x[1] - n[1] * x[0]};
+                view[threadIdx.x][0] = dot3(x, u);
+                view[threadIdx.x][1] = dot3(y, u);
+                view[threadIdx.x][2] = dot3(n, u);
+                weight /= a.sub_total;
             }
         }
     }
-    for (int l = 0; l < a.nwl; ++l) {
-        red[threadIdx.x] = term[l];
-        __syncthreads();
-        for (int w = kFluxThreads / 2; w > 0; w >>= 1) {
-            if (threadIdx.x < w) red[threadIdx.x] = __dadd_rn(red[threadIdx.x], red[threadIdx.x + w]);
-            __syncthreads();
+    if constexpr (ROUGH) {
+        // each facet's crater, a lane per sub-facet: every one with a visible
+        // fraction > 0 at its own view angle (wise_main.cpp:515), the facet's
+        // total scaled by its share of the crater's projected area
+        // (wise_main.cpp:718)
+        view[threadIdx.x][3] = weight;
+        __syncwarp();
+        for (int i = 0; i < 32; ++i) {
+            const double* v = view[warp * 32 + i];
+            if (v[3] == 0.0) continue;
+            const size_t base =
+                ((size_t)(blockIdx.x * kFluxThreads + warp * 32 + i) * s.ntau + step) * (size_t)a.nsf;
+            for (int j = lane; j < a.nsf; j += 32) {
+                const double vis = (double)a.sub_vis[base + j];
+                const double* g = a.sub_geo + 4 * j;
+                const double c = v[0] * g[0] + v[1] * g[1] + v[2] * g[2];
+                if (!(vis > 0.0) || !(fabs(c) <= 1.0)) continue;
+                const double m = v[3] * g[3] * vis * c, inv_t = 1.0 / (double)a.sub_T[base + j];
+#pragma unroll
+                for (int l = 0; l < kMaxFluxWavelengths; ++l)
+                    if (l < a.nwl) term[l] += planck(a, l, inv_t) * m;
+            }
         }
-        if (threadIdx.x == 0) a.partial[((size_t)step * gridDim.x + blockIdx.x) * a.nwl + l] = red[0];
-        __syncthreads();
+    }
+#pragma unroll
+    for (int l = 0; l < kMaxFluxWavelengths; ++l) {
+        if (l >= a.nwl) break;
+        double t = term[l];
+        for (int o = 16; o > 0; o >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
+        if (lane == 0) red[l][warp] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x < a.nwl) {
+        double t = red[threadIdx.x][0];
+        for (int w = 1; w < kWarps; ++w) t = __dadd_rn(t, red[threadIdx.x][w]);
+        a.partial[((size_t)step * gridDim.x + blockIdx.x) * a.nwl + threadIdx.x] = t;
     }
 }
 
@@ -185,6 +226,12 @@ int launch_disk_flux(const DevSolve& s, const FluxArgs& a, stream_t stv) {
     if (a.nwl < 1 || a.nwl > kMaxFluxWavelengths) return 1;
     const int nblk = (s.nf + kFluxThreads - 1) / kFluxThreads;
     const dim3 grid(nblk, s.ntau);
+    const long long nvt = (long long)s.nv * s.ntau;
+    k_flux_vertices<<<(unsigned)((nvt + 255) / 256), 256, 0, st>>>(s, a);
+    k_flux_area<<<(s.nf + 255) / 256, 256, 0, st>>>(s, a);
+    if (a.visible)
+        k_flux_flags<<<dim3((s.ntau + 31) / 32, (s.nf + 31) / 32), dim3(32, 8), 0, st>>>(
+            a.flags, const_cast<uint8_t*>(a.visible), s.nf, s.ntau);
     if (a.sub_T) {
         if (s.mode == MODE_FP64) k_flux_partial<double, true><<<grid, kFluxThreads, 0, st>>>(s, a);
         else k_flux_partial<float, true><<<grid, kFluxThreads, 0, st>>>(s, a);

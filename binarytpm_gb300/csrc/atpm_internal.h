@@ -337,11 +337,13 @@ struct FluxArgs {
     double car[3];           // body centre (km)
     double obs[3];           // observer (km)
     double eps;
-    const uint8_t* visible;  // [nf][ntau] or null (horizon test only)
+    const int32_t* flags;    // [nf][ntau] visibility words, or null (horizon test only)
+    const uint8_t* visible;  // [ntau][nf] their bytes (k_flux_flags), or null
+    double* hp;              // [ntau][nv][3] vertex positions (k_flux_vertices)
+    double* area;            // [nf] (k_flux_area)
     int nwl;
     double b1[kMaxFluxWavelengths];  // 2 h c^2 / lambda^5
-    double lk[kMaxFluxWavelengths];  // lambda * k
-    double hc;                       // h * c
+    double hl[kMaxFluxWavelengths];  // h c / (lambda k)
     double* partial;         // [ntau][blocks][nwl]
     double* out;             // [ntau][nwl]
     // rough surface (crater sub-facets); null for the smooth-surface sum
