@@ -1,13 +1,12 @@
 // Host side of the view-factor precompute (Shape_Selfheating,
 // 3905/Shape_Selfheating/main.cpp:817-889): drives the kernels of
-// atpm_viewfactor.cu, compacts the occlusion-culled lists and forms the
-// photon-momentum vectors of main.cpp:824-835.  Built with -ffp-contract=off.
+// atpm_viewfactor.cu.  Lists, view factors and vectors stay on the device until
+// atpm_viewfactors_get copies them to the caller's arrays.
 #include <cuda_runtime.h>
 
-#include <cstdarg>
+#include <algorithm>
+#include <cmath>
 #include <cstdio>
-#include <cstring>
-#include <string>
 #include <vector>
 
 #include "../../include/atpm.h"
@@ -25,26 +24,40 @@ struct VfGeom {
 int vf_init(const VfGeom& g, cudaStream_t st);
 int vf_count(const VfGeom& g, int* count, cudaStream_t st);
 int vf_fill(const VfGeom& g, const long long* ptr, int* idx, float* vf, float* dir, cudaStream_t st);
-int vf_hidden(const VfGeom& g, const long long* ptr, const int* idx, uint8_t* keep, cudaStream_t st);
+int vf_hidden(const VfGeom& g, float size, const long long* ptr, const int* idx, uint8_t* keep, int* kept,
+              cudaStream_t st);
+int vf_compact(const VfGeom& g, const long long* ptr, const uint8_t* keep, const int* idx, const float* vf,
+               const float* dir, const long long* optr, int* oidx, float* ovf, float* odir, cudaStream_t st);
 int vf_refine(const VfGeom& g, const long long* ptr, const int* idx, float* vf, float* dir, cudaStream_t st);
+int vf_photo(const VfGeom& g, const long long* ptr, const float* dir, float* photo, cudaStream_t st);
 void set_last_error(const char* msg);
 }  // namespace atpm
 
-struct atpm_vf_result {
-    int nf = 0;
-    std::vector<int32_t> ptr, idx;
-    std::vector<float> vf, dir, photo;
-};
-
 namespace {
+// device memory from the stream-ordered pool (kept by the context's release
+// threshold from call to call), given back with its owner
 struct DevBufs {
     std::vector<void*> p;
-    ~DevBufs() { for (void* x : p) cudaFree(x); }
+    cudaStream_t st = nullptr;
+    ~DevBufs() {
+        for (void* x : p) cudaFreeAsync(x, st);
+    }
     template <class T> cudaError_t alloc(T** out, size_t n) {
         void* q = nullptr;
-        cudaError_t e = cudaMalloc(&q, n ? n * sizeof(T) : 1);
+        cudaError_t e = cudaMallocAsync(&q, n ? n * sizeof(T) : 1, st);
         if (e == cudaSuccess) { p.push_back(q); *out = static_cast<T*>(q); }
         return e;
+    }
+};
+// the device a result lives on is current within the scope
+struct OnDevice {
+    int before = -1;
+    explicit OnDevice(int device) {
+        if (cudaGetDevice(&before) != cudaSuccess) before = -1;
+        if (before != device) cudaSetDevice(device);
+    }
+    ~OnDevice() {
+        if (before >= 0) cudaSetDevice(before);
     }
 };
 atpm_status vfail(atpm_status s, const char* what, cudaError_t e) {
@@ -54,6 +67,14 @@ atpm_status vfail(atpm_status s, const char* what, cudaError_t e) {
     return s;
 }
 }  // namespace
+
+struct atpm_vf_result {
+    int nf = 0, device = 0;
+    std::vector<int32_t> ptr;
+    DevBufs bufs;
+    int* idx = nullptr;
+    float *vf = nullptr, *dir = nullptr, *photo = nullptr;
+};
 
 extern "C" {
 
@@ -70,6 +91,8 @@ ATPM_API atpm_status atpm_viewfactors_compute(atpm_context* ctx, int32_t nv, int
             atpm::set_last_error("viewfactors: facet vertex index out of range");
             return ATPM_E_INVALID;
         }
+    float size = 0.0f;  // the largest coordinate: the scale of the positions' rounding
+    for (int i = 0; i < 3 * nv; ++i) size = std::max(size, std::fabs(vertices[i]));
     cudaStream_t st = 0;
     DevBufs B;
     atpm::VfGeom g{};
@@ -91,66 +114,49 @@ ATPM_API atpm_status atpm_viewfactors_compute(atpm_context* ctx, int32_t nv, int
     g.fac = fac;
     if (atpm::vf_init(g, st)) return vfail(ATPM_E_CUDA, "init launch", cudaGetLastError());
     int* cnt = nullptr;
+    long long* dptr = nullptr;
     T(B.alloc(&cnt, (size_t)nf), "alloc");
+    T(B.alloc(&dptr, (size_t)nf + 1), "alloc");
     if (atpm::vf_count(g, cnt, st)) return vfail(ATPM_E_CUDA, "count launch", cudaGetLastError());
     std::vector<int> hc(nf);
-    T(cudaMemcpy(hc.data(), cnt, (size_t)nf * 4, cudaMemcpyDeviceToHost), "count");
     std::vector<long long> ptr(nf + 1, 0);
+    T(cudaMemcpy(hc.data(), cnt, (size_t)nf * 4, cudaMemcpyDeviceToHost), "count");
     for (int i = 0; i < nf; ++i) ptr[i + 1] = ptr[i] + hc[i];
     const size_t tot = (size_t)ptr[nf];
-    long long* dptr = nullptr;
     int* didx = nullptr;
     float *dvf = nullptr, *ddir = nullptr;
     uint8_t* keep = nullptr;
-    T(B.alloc(&dptr, (size_t)nf + 1), "alloc");
     T(B.alloc(&didx, tot), "alloc candidates");
     T(B.alloc(&dvf, tot), "alloc candidates");
     T(B.alloc(&ddir, 3 * tot), "alloc candidates");
     T(B.alloc(&keep, tot), "alloc candidates");
     T(cudaMemcpy(dptr, ptr.data(), (size_t)(nf + 1) * 8, cudaMemcpyHostToDevice), "upload");
     if (atpm::vf_fill(g, dptr, didx, dvf, ddir, st)) return vfail(ATPM_E_CUDA, "fill launch", cudaGetLastError());
-    if (atpm::vf_hidden(g, dptr, didx, keep, st)) return vfail(ATPM_E_CUDA, "hidden launch", cudaGetLastError());
-    std::vector<int> hidx(tot);
-    std::vector<float> hvf(tot), hdir(3 * tot);
-    std::vector<uint8_t> hk(tot);
-    T(cudaMemcpy(hidx.data(), didx, tot * 4, cudaMemcpyDeviceToHost), "download");
-    T(cudaMemcpy(hvf.data(), dvf, tot * 4, cudaMemcpyDeviceToHost), "download");
-    T(cudaMemcpy(hdir.data(), ddir, tot * 12, cudaMemcpyDeviceToHost), "download");
-    T(cudaMemcpy(hk.data(), keep, tot, cudaMemcpyDeviceToHost), "download");
+    if (atpm::vf_hidden(g, size, dptr, didx, keep, cnt, st))
+        return vfail(ATPM_E_CUDA, "hidden launch", cudaGetLastError());
+    T(cudaMemcpy(hc.data(), cnt, (size_t)nf * 4, cudaMemcpyDeviceToHost), "kept count");
     auto* r = new atpm_vf_result();
     r->nf = nf;
+    r->bufs.st = st;
     r->ptr.assign(nf + 1, 0);
-    for (int i = 0; i < nf; ++i) {
-        int c = 0;
-        for (long long k = ptr[i]; k < ptr[i + 1]; ++k)
-            if (hk[k]) {
-                r->idx.push_back(hidx[k]);
-                r->vf.push_back(hvf[k]);
-                r->dir.insert(r->dir.end(), &hdir[3 * k], &hdir[3 * k] + 3);
-                ++c;
-            }
-        r->ptr[i + 1] = r->ptr[i] + c;
-    }
-    const size_t n2 = r->idx.size();
-    if (refine && n2 > 0) {
-        std::vector<long long> p2(nf + 1);
-        for (int i = 0; i <= nf; ++i) p2[i] = r->ptr[i];
-        e = cudaMemcpy(dptr, p2.data(), (size_t)(nf + 1) * 8, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(didx, r->idx.data(), n2 * 4, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(dvf, r->vf.data(), n2 * 4, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess) e = cudaMemcpy(ddir, r->dir.data(), n2 * 12, cudaMemcpyHostToDevice);
-        if (e == cudaSuccess && atpm::vf_refine(g, dptr, didx, dvf, ddir, st)) e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpy(r->vf.data(), dvf, n2 * 4, cudaMemcpyDeviceToHost);
-        if (e == cudaSuccess) e = cudaMemcpy(r->dir.data(), ddir, n2 * 12, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) { delete r; return vfail(ATPM_E_CUDA, "refine", e); }
-    }
-    // photon-momentum vectors (main.cpp:824-835)
-    std::vector<float> area(nf);
-    T(cudaMemcpy(area.data(), g.area, (size_t)nf * 4, cudaMemcpyDeviceToHost), "download");
-    r->photo.assign((size_t)nf * 3, 0.0f);
-    for (int i = 0; i < nf; ++i)
-        for (int k = r->ptr[i]; k < r->ptr[i + 1]; ++k)
-            for (int c = 0; c < 3; ++c) r->photo[3 * i + c] = r->photo[3 * i + c] + (r->dir[3 * k + c] / area[i]);
+    for (int i = 0; i < nf; ++i) r->ptr[i + 1] = r->ptr[i] + hc[i];
+    const size_t n2 = (size_t)r->ptr[nf];
+    std::vector<long long> p2(r->ptr.begin(), r->ptr.end());
+    long long* optr = nullptr;
+    e = cudaGetDevice(&r->device);
+    if (e == cudaSuccess) e = B.alloc(&optr, (size_t)nf + 1);
+    if (e == cudaSuccess) e = r->bufs.alloc(&r->idx, n2);
+    if (e == cudaSuccess) e = r->bufs.alloc(&r->vf, n2);
+    if (e == cudaSuccess) e = r->bufs.alloc(&r->dir, 3 * n2);
+    if (e == cudaSuccess) e = r->bufs.alloc(&r->photo, 3 * (size_t)nf);
+    if (e == cudaSuccess) e = cudaMemcpy(optr, p2.data(), (size_t)(nf + 1) * 8, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && atpm::vf_compact(g, dptr, keep, didx, dvf, ddir, optr, r->idx, r->vf, r->dir, st))
+        e = cudaGetLastError();
+    if (e == cudaSuccess && refine && n2 > 0 && atpm::vf_refine(g, optr, r->idx, r->vf, r->dir, st))
+        e = cudaGetLastError();
+    if (e == cudaSuccess && atpm::vf_photo(g, optr, r->dir, r->photo, st)) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) { delete r; return vfail(ATPM_E_CUDA, "lists", e); }
 #undef T
     *out = r;
     if (nnz_out) *nnz_out = (int64_t)n2;
@@ -160,15 +166,23 @@ ATPM_API atpm_status atpm_viewfactors_compute(atpm_context* ctx, int32_t nv, int
 ATPM_API atpm_status atpm_viewfactors_get(const atpm_vf_result* r, int32_t* dep_ptr, int32_t* dep_idx, float* dep_vf,
                                           float* dep_vec, float* photovectors) {
     if (!r) { atpm::set_last_error("viewfactors_get: null result"); return ATPM_E_INVALID; }
-    if (dep_ptr) std::memcpy(dep_ptr, r->ptr.data(), r->ptr.size() * 4);
-    if (dep_idx && !r->idx.empty()) std::memcpy(dep_idx, r->idx.data(), r->idx.size() * 4);
-    if (dep_vf && !r->vf.empty()) std::memcpy(dep_vf, r->vf.data(), r->vf.size() * 4);
-    if (dep_vec && !r->dir.empty()) std::memcpy(dep_vec, r->dir.data(), r->dir.size() * 4);
-    if (photovectors) std::memcpy(photovectors, r->photo.data(), r->photo.size() * 4);
-    return ATPM_OK;
+    OnDevice on(r->device);
+    const size_t n = (size_t)r->ptr[r->nf];
+    cudaError_t e = cudaSuccess;
+    auto copy = [&](void* to, const void* from, size_t bytes) {
+        if (to && bytes && e == cudaSuccess) e = cudaMemcpy(to, from, bytes, cudaMemcpyDeviceToHost);
+    };
+    if (dep_ptr) std::copy(r->ptr.begin(), r->ptr.end(), dep_ptr);
+    copy(dep_idx, r->idx, n * 4);
+    copy(dep_vf, r->vf, n * 4);
+    copy(dep_vec, r->dir, n * 12);
+    copy(photovectors, r->photo, (size_t)r->nf * 12);
+    return e == cudaSuccess ? ATPM_OK : vfail(ATPM_E_CUDA, "download", e);
 }
 
 ATPM_API atpm_status atpm_viewfactors_free(atpm_vf_result* r) {
+    if (!r) return ATPM_OK;
+    OnDevice on(r->device);
     delete r;
     return ATPM_OK;
 }
