@@ -153,7 +153,7 @@ Layout layout(int nv, int nf, int nnz, const atpm_params& P) {
     sz[B_S1] = nt * rs;
     sz[B_TEMP] = (size_t)(P.nx + 1) * nf * rs;
     sz[B_Q] = nt * rs;
-    sz[B_W] = nt * rs;
+    sz[B_W] = (size_t)nf * ((P.ntau + 3) & ~3) * rs;  // rows of gather_ld(ntau)
     sz[B_CONV] = nf;
     sz[B_HOT] = nf;
     sz[B_COUNTS] = (size_t)std::max(P.revcap, 1) * 4;
@@ -1080,7 +1080,7 @@ ATPM_API atpm_status atpm_solve_footprint(const atpm_shape* sh, const atpm_param
     const size_t rs = (P->precision == ATPM_FP64) ? 8 : 4;
     // transient peak: geometry (hp, hm, nrm, dist) or scattering work
     const size_t geo = (size_t)sh->nv * P->ntau * 24 + nt * 56 + (size_t)P->ntau * 16;
-    const size_t sct = 3 * nt * rs;
+    const size_t sct = 3 * (nt + 4 * (size_t)sh->nf) * rs;
     // FAST with self-heating: this solve's BF16 W tiles (hi + lo; the view-
     // factor tiles are shared with the solve it is cloned from)
     size_t wb = 0;
@@ -1457,16 +1457,21 @@ ATPM_API atpm_status atpm_solve_solar(const atpm_solve* s, float* solar) {
 ATPM_API atpm_status atpm_scattering(atpm_solve* s) {
     if (!s) return fail(ATPM_E_INVALID, "null solve");
     CK(cudaSetDevice(s->ctx->device));
-    if (launch_single_scattering(s->ds, s->st)) return fail(ATPM_E_CUDA, "single scattering launch");
-    if (s->P.multiple_scattering) {
-        void* work = nullptr;
+    const bool multiple = s->P.multiple_scattering != 0;
+    if (multiple) {
         atpm_status rp = ensure_gs_plan(s);
         if (rp) return rp;
-        CK(cudaMallocAsync(&work, multiple_scattering_work_bytes(s->ds), s->st));
-        int rc = launch_multiple_scattering(s->ds, s->gs ? s->gs->plan : GsPlan{}, work, s->st);
-        cudaFreeAsync(work, s->st);
-        if (rc) return fail(ATPM_E_CUDA, "multiple scattering launch");
     }
+    void* work = nullptr;
+    CK(cudaMallocAsync(&work, scattering_work_bytes(s->ds, multiple), s->st));
+    int rc = launch_single_scattering(s->ds, work, multiple, s->st);
+    const char* what = "single scattering launch";
+    if (!rc && multiple) {
+        rc = launch_multiple_scattering(s->ds, s->gs ? s->gs->plan : GsPlan{}, work, s->st);
+        what = "multiple scattering launch";
+    }
+    cudaFreeAsync(work, s->st);
+    if (rc) return fail(ATPM_E_CUDA, "%s", what);
     if (launch_forcing_transpose(s->ds, s->st)) return fail(ATPM_E_CUDA, "forcing transpose launch");
     int st = 0;
     CK(cudaMemcpyAsync(&st, s->ds.status, 4, cudaMemcpyDeviceToHost, s->st));

@@ -5,8 +5,9 @@
 //                                       consecutive facets -> coalesced
 //   temp                   [nx+1][nf]   depth-major, read once per revolution
 //   W                      [nf][ntau]   facet-major eps*sigma*T^4 of the
-//                                       previous revolution: the self-heating
-//                                       gather reads 32 consecutive steps
+//                                       previous revolution, rows padded to 4
+//                                       steps: the self-heating gather reads
+//                                       16 bytes of consecutive steps a lane
 //   shadow, cosil          [nf][ntau]   facet-major (scattering gathers)
 //   dep_ptr/idx/vf         CSR view-factor lists in file order
 //
@@ -154,7 +155,7 @@ struct DevSolve {
     void* stemp1;            // [ntau][nf] R
     void* temp;              // [nx+1][nf] R
     void* Q;                 // [ntau][nf] R
-    void* W;                 // [nf][ntau] R (FAST with tensor-core tiles: the sparse remainder's
+    void* W;                 // [nf][gather_ld(ntau)] R (FAST with tensor-core tiles: the sparse remainder's
                              // sums, [ntau][nf] FP32, which k_rem_add adds to Q)
     uint8_t* conv;           // [nf] frozen (reference astconverged)
     uint8_t* hot;            // [nf] some |stemp1-stemp0| >= TACC this revolution
@@ -245,7 +246,8 @@ int launch_shadow_allpairs(const DevSolve& s, const GeomWork& g, stream_t st);
 int launch_shadow_culled(const DevSolve& s, const GeomWork& g, bool all_pairs, stream_t st);
 
 // scattering (atpm_scatter.cu)
-int launch_single_scattering(const DevSolve& s, stream_t st);
+size_t scattering_work_bytes(const DevSolve& s, bool multiple);
+int launch_single_scattering(const DevSolve& s, void* work, bool multiple, stream_t st);
 // Gauss-Seidel order of a shape's lists (ascending rows): the facets with a
 // list sorted by level, {facet, first entry, first entry above the facet, 0}
 struct GsPlan {
@@ -256,7 +258,6 @@ struct GsPlan {
 };
 constexpr size_t kGsSharedBytes = 220 * 1024;  // one CTA's values (k_multi_levels)
 int launch_multiple_scattering(const DevSolve& s, const GsPlan& plan, void* work, stream_t st);
-size_t multiple_scattering_work_bytes(const DevSolve& s);
 int launch_forcing_transpose(const DevSolve& s, stream_t st);
 int launch_set_forcing(const DevSolve& s, const int32_t* shadow_d, const float* illum_d, stream_t st);
 int launch_widen_flags(const uint8_t* src, int32_t* dst, size_t n, stream_t st);

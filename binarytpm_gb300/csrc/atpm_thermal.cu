@@ -26,6 +26,7 @@
 #include <cuda_bf16.h>
 
 #include "atpm_column.cuh"
+#include "atpm_gather.cuh"
 #include "atpm_internal.h"
 
 namespace atpm {
@@ -54,39 +55,49 @@ __global__ void __launch_bounds__(256) k_selfheat_w(Batch b) {
     __syncthreads();
     for (int j = threadIdx.y; j < 32; j += blockDim.y) {
         const int f = t.y + j, s = t.z + threadIdx.x;
-        if (f < nf && s < ntau) W[(size_t)f * ntau + s] = sm[threadIdx.x][j];
+        if (f < nf && s < ntau) W[(size_t)f * gather_ld(ntau) + s] = sm[threadIdx.x][j];
     }
 }
 
 // Q[s][f] = sum over f's list of W[g][s] * vf, accumulated in list order
-// (main.cpp:1519-1529).  Warp w of the block owns facet f0+w, lane l owns
-// step s0+l, so the list loop is warp-uniform and every W load is a
-// coalesced 128-byte row segment.
-template <int MODE>
-__global__ void __launch_bounds__(1024) k_selfheat_q(Batch b) {
+// (main.cpp:1519-1529), a warp per facet over rows of W (atpm_gather.cuh).  The
+// map's tiles of 32 facets x 32 steps are regrouped: the tiles of one span of
+// 32 lanes' steps (four in 32 bits, two in 64; fewer at the end) share its
+// facets.  Last facets first: a binary's secondary comes last and has its
+// longest rows.  REFERENCE, 6,280 facets, 613 steps: 0.44 -> 0.19 ms.
+template <int MODE, int N>
+__global__ void __launch_bounds__(N == 1 ? 1024 : 256) k_selfheat_q(Batch b) {
     using A = Ar<MODE>;
     using R = typename A::R;
-    const int4 t = b.wmap[blockIdx.x];
+    constexpr int SPAN = 32 * N, WARPS = N == 1 ? 32 : 8;
+    const int4 t = b.wmap[gridDim.x - 1 - blockIdx.x];
     const DevSolve& sv = b.tab[t.x];
     if (!sv.ctl->active) return;
-    __shared__ R sm[32][33];
-    const int nf = sv.nf, ntau = sv.ntau;
-    const int f = t.y + threadIdx.y, s = t.z + threadIdx.x;
+    __shared__ R sm[SPAN][33];
+    const int nf = sv.nf, ntau = sv.ntau, ld = gather_ld(ntau);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tile = t.z / 32, span = tile / N, share = min(N, (ntau + 31) / 32 - span * N);
+    const int f0 = t.y + 32 * (tile % N) / share, f1 = min(nf, t.y + 32 * (tile % N + 1) / share);
+    const int s0 = span * SPAN, s = s0 + lane * N;
     const bool inst = (MODE == MODE_FP64) ? (sv.ti_d == 0.0) : (sv.ti == 0.0f);
-    R q = R(0);
-    if (f < nf && s < ntau && (inst || !sv.freeze || !sv.conv[f])) {
-        const R* W = static_cast<const R*>(sv.W);
-        const int k1 = sv.dep_ptr[f + 1];
-        for (int k = sv.dep_ptr[f]; k < k1; ++k) {
-            const int g = __ldg(&sv.dep_idx[k]);
-            const R v = (R)__ldg(&sv.dep_vf[k]);
-            q = A::add(q, A::mul(W[(size_t)g * ntau + s], v));
-        }
+    const R* rows = static_cast<const R*>(sv.W) + (s < ntau ? s : 0);
+    for (int f = f0 + warp; f < f1; f += WARPS) {
+        R q[N] = {};
+        if (inst || !sv.freeze || !sv.conv[f])
+            gather<R, N>(sv.dep_idx, sv.dep_vf, sv.dep_ptr[f], sv.dep_ptr[f + 1], rows, ld, [](float v) { return (R)v; },
+                      [&](int, R c, const R(&x)[N]) {
+#pragma unroll
+                          for (int u = 0; u < N; ++u) q[u] = A::add(q[u], A::mul(x[u], c));
+                      });
+#pragma unroll
+        for (int u = 0; u < N; ++u) sm[lane * N + u][f - f0] = q[u];
     }
-    sm[threadIdx.y][threadIdx.x] = q;
     __syncthreads();
-    const int so = t.z + threadIdx.y, fo = t.y + threadIdx.x;
-    if (so < ntau && fo < nf) static_cast<R*>(sv.Q)[(size_t)so * nf + fo] = sm[threadIdx.x][threadIdx.y];
+    const int nw = f1 - f0;
+    for (int i = threadIdx.x; i < SPAN * 32; i += 32 * WARPS) {
+        const int so = i >> 5, fo = i & 31;
+        if (fo < nw && s0 + so < ntau) static_cast<R*>(sv.Q)[(size_t)(s0 + so) * nf + f0 + fo] = sm[so][fo];
+    }
 }
 
 // --------------------------------------------------------------- conduction
@@ -679,7 +690,12 @@ static int launch_rev_part(const Batch& b, int part, cudaStream_t st) {
     if (MODE == MODE_FAST && b.nq > 0 && part < 2) return part == 0 ? 0 : launch_spmm_tc(b, st);
     switch (part) {
         case 0: if (b.nw > 0) k_selfheat_w<MODE><<<b.nw, dim3(32, 8), 0, st>>>(b); break;
-        case 1: if (b.nw > 0) k_selfheat_q<MODE><<<b.nw, dim3(32, 32), 0, st>>>(b); break;
+        case 1: {
+            constexpr int W = kWide<typename Ar<MODE>::R>;
+            if (b.nw > 0 && gather_wide(b.nw, W, b.sms)) k_selfheat_q<MODE, W><<<b.nw, 256, 0, st>>>(b);
+            else if (b.nw > 0) k_selfheat_q<MODE, 1><<<b.nw, 1024, 0, st>>>(b);
+            break;
+        }
         case 2:
             if (MODE != MODE_FAST) return launch_conduction_split(b, st);
             k_tail_mode<<<1, 32, 0, st>>>(b);
