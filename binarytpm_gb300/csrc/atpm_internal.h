@@ -155,8 +155,8 @@ struct DevSolve {
     void* stemp1;            // [ntau][nf] R
     void* temp;              // [nx+1][nf] R
     void* Q;                 // [ntau][nf] R
-    void* W;                 // [nf][gather_ld(ntau)] R (FAST with tensor-core tiles: the sparse remainder's
-                             // sums, [ntau][nf] FP32, which k_rem_add adds to Q)
+    void* W;                 // [nf][gather_ld(ntau)] R (FAST with tensor-core tiles: the sparse
+                             // remainder's sums)
     uint8_t* conv;           // [nf] frozen (reference astconverged)
     uint8_t* hot;            // [nf] some |stemp1-stemp0| >= TACC this revolution
     // facets still active after each convergence test (FAST, freeze on),
@@ -201,7 +201,7 @@ struct DevSolve {
     const float* rem_vf;     // [rem_nnz]
     const uint8_t* rem_row;  // [rem_nnz] the entry's row within its 128-facet row block
     float* W32;              // [nf][w32_ld] FP32 (null without a remainder)
-    int w32_ld;              // row stride of W32: ntau rounded up to 32 (the remainder's step chunks)
+    int w32_ld;              // row stride of W32: ntau rounded up to 32
 };
 
 // element offset of (row, k) inside a 128-byte-swizzled K-major tile with 64
@@ -289,12 +289,6 @@ struct Batch {
     int sms;                 // SMs of the device (persistent tensor-core grid)
     int rem_nmb, rem_ntau;   // largest row-block count / steps of the batch's solves with a
                              // sparse remainder (0: none; the remainder kernel's grid)
-    // host handles: a second stream on which the remainder runs beside the
-    // tensor-core product (forked and joined with the two events; null: the
-    // remainder runs after the product on the batch's stream)
-    void* side;
-    void* ev_fork;
-    void* ev_join;
 };
 // deepest tensor-core pipeline that fits shared memory for step chunk N
 int tc_max_stages(int N);

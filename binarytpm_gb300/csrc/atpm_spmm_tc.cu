@@ -20,7 +20,7 @@
 // of the binary's entries, in 68 % of its cells: facets of one body seeing
 // each other across its relief) are the sparse remainder, summed in FP32 by
 // k_spmm_rem against W32 (eps sigma T^4 facet-major, written by the
-// conduction sweep beside the BF16 tiles) and added to the tiles' Q.
+// conduction sweep beside the BF16 tiles); the product's epilogue adds them.
 //
 // V is stored as 128 x 64 BF16 tiles (block-sparse rows: every 128-facet row
 // block keeps the 64-facet column blocks it has tiles in; one set per shape,
@@ -46,6 +46,7 @@
 #include <atomic>
 #include <cstdint>
 
+#include "atpm_gather.cuh"
 #include "atpm_internal.h"
 
 namespace atpm {
@@ -560,22 +561,33 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
             }
             tc_fence_after();
             const int f = w.y * TC_M + q * 32 + lane;
+            // the last segment adds the remainder's sums of the rows that
+            // have entries in it (k_spmm_rem)
+            const bool rem = f < nf && sv.rem_ptr && (w.w + 1) * TC_SEG >= T &&
+                             __ldg(&sv.rem_ptr[f]) != __ldg(&sv.rem_ptr[f + 1]);
+            const float* R = static_cast<const float*>(sv.W) + (size_t)(f < nf ? f : 0) * gather_ld(ntau);
             if (T == 0) {  // no tile in this row block
                 if (f < nf)
                     for (int n = 0; n < N; ++n) {
                         const int s = nc * N + n;
-                        if (s < ntau) Q[(size_t)s * nf + f] = 0.0f;
+                        if (s < ntau) Q[(size_t)s * nf + f] = rem ? R[s] : 0.0f;
                     }
             } else {
                 // the first segment stores, later ones add to Q in order
-                // (round to nearest); a batch's 16 loads all issue before
-                // its stores
+                // (round to nearest); a batch's loads all issue before its
+                // stores
                 const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + ab * kBufCols;
                 for (int c0 = 0; c0 < N; c0 += 16) {
                     float v[16];
                     tc_ld16(tbase + (uint32_t)c0, v);
                     if (f < nf) {
                         float prev[16];
+                        float4 more[4];
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const int s = nc * N + c0 + 4 * j;  // a multiple of 4: N is one of 16
+                            if (rem && s < ntau) more[j] = __ldg(reinterpret_cast<const float4*>(R + s));
+                        }
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
                             const int s = nc * N + c0 + j;
@@ -584,7 +596,9 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
 #pragma unroll
                         for (int j = 0; j < 16; ++j) {
                             const int s = nc * N + c0 + j;
-                            if (c0 + j < N && s < ntau) Q[(size_t)s * nf + f] = w.w == 0 ? v[j] : prev[j] + v[j];
+                            float x = w.w == 0 ? v[j] : prev[j] + v[j];
+                            if (rem) x += reinterpret_cast<const float*>(more)[j];
+                            if (c0 + j < N && s < ntau) Q[(size_t)s * nf + f] = x;
                         }
                     }
                 }
@@ -613,26 +627,23 @@ size_t spmm_tc_smem_bytes(int N, int stages) {
 int tc_max_stages(int N) { return tc_stages(N); }
 
 // The sparse remainder of the product: the list entries of the cells too
-// sparse for a tensor-core tile, added to the tiles' Q in FP32.  One CTA per
-// (solve, 128-facet row block, 32-step chunk), lane j of every warp on step
-// s0 + j, so each entry is one coalesced 128-byte load of its column facet's
-// W32 row.  The block's entries (rows in order, each row's in list order)
-// are cut into four contiguous ranges, one per warp; a warp reads 32
-// entries' column, value and row at once and keeps eight W32 loads in
-// flight across row boundaries, so the gather is not a chain of dependent
-// loads per row (a row holds ~3 remainder entries on average).  A row's sum
-// is the multiply-add chain over its entries in list order within each
-// warp's range; a row split between warps adds the warps' partial sums in
-// warp order after a barrier.  The block's 128 x 32 sums go through shared
-// memory into the remainder's own array (along facets, coalesced), which
-// k_rem_add adds to Q once the tensor-core product is complete.  Row blocks the
-// tensor-core product skips (all facets frozen) are skipped alike.
-// Earlier forms, a warp per facet row (one dependent index-then-W32 chain
-// per row: 1.80 ms for the product per batch revolution of the 8-inertia
-// binary), the same with the block's entries staged in shared memory first
-// (1.93 ms) and one CTA per row block looping over the chunks (2.43 ms),
-// were latency-bound.
-constexpr int REM_STEPS = 32;
+// sparse for a tensor-core tile, summed in FP32 into rows [facet][step] that
+// k_spmm_tc's epilogue adds to the tiles' sums.  One CTA per (solve, 128-facet
+// row block, 128-step chunk), four steps a lane: an entry is one coalesced
+// 512-byte load of its column facet's W32 row.  The block's entries (rows in
+// order, each row's in list order) are cut into four contiguous ranges, one per
+// warp; a warp reads 32 entries' column, value and row at once and keeps eight
+// W32 loads in flight across row boundaries, so the gather is not a chain of
+// dependent loads per row (a row holds ~3 entries on average).  A row's sum is
+// the multiply-add chain over its entries in list order within each warp's
+// range; the first and last row of a range, which neighbouring warps may share,
+// are added in warp order after a barrier.  Row blocks the tensor-core product
+// skips (all facets frozen) are skipped alike.
+// Bound by the W32 gathers from L2.  Eight inertias of the 21,760-facet binary,
+// 60,105 entries each: 0.46 -> 0.32 ms; with 4 bytes a lane, the sums
+// transposed in shared memory and a kernel of their own adding them to Q
+// (0.29 ms) it was bound by instruction issue.
+constexpr int REM_STEPS = 128;
 constexpr int REM_WARPS = 4;
 constexpr int REM_INFLIGHT = 8;
 
@@ -646,24 +657,25 @@ __global__ void __launch_bounds__(REM_WARPS * 32) k_spmm_rem(Batch b) {
     const int f_lo = rb * 128, f_hi = min(nf, f_lo + 128);
     const int e0 = __ldg(&sv.rem_ptr[f_lo]), e1 = __ldg(&sv.rem_ptr[f_hi]);
     if (e0 == e1) return;  // no remainder entry in this block
-    __shared__ float acc[128][REM_STEPS + 1];
-    __shared__ float edge[REM_WARPS][REM_STEPS];
-    __shared__ int edge_row[REM_WARPS];
+    __shared__ float4 part[2 * REM_WARPS][32];  // sums of the first and the last row of each warp's range
+    __shared__ int part_row[2 * REM_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int i = threadIdx.x; i < 128 * (REM_STEPS + 1); i += blockDim.x) (&acc[0][0])[i] = 0.0f;
-    __syncthreads();
-    const float* W32 = sv.W32;
+    const int s = s0 + 4 * lane;
+    const bool ok = s < ntau;
+    const float* W32 = sv.W32 + (ok ? s : 0);  // rows start and end on 16 bytes
+    float* R = static_cast<float*>(sv.W) + (size_t)f_lo * gather_ld(ntau) + s;
+    auto put = [&](int row, const float4& v) {
+        if (ok) *reinterpret_cast<float4*>(R + (size_t)row * gather_ld(ntau)) = v;
+    };
     const size_t ld = (size_t)sv.w32_ld;
-    const int s = s0 + lane;  // W32 rows are padded to the chunk grid: s < w32_ld
     const int n = e1 - e0;
     const int a0 = e0 + (int)(((long long)n * warp) / REM_WARPS);
     const int a1 = e0 + (int)(((long long)n * (warp + 1)) / REM_WARPS);
-    // the warp's first row goes to its edge slot, every later row (which
-    // starts inside this range) straight to acc
     int cur = -1;
     bool first = true;
-    float a = 0.0f;
-    if (lane == 0) edge_row[warp] = -1;
+    float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (lane < 2) part_row[2 * warp + lane] = -1;
+    __syncwarp();
     for (int kb = a0; kb < a1; kb += 32) {
         const int k = kb + lane;
         const bool in = k < a1;
@@ -672,11 +684,11 @@ __global__ void __launch_bounds__(REM_WARPS * 32) k_spmm_rem(Batch b) {
         const int rk = in ? (int)__ldg(&sv.rem_row[k]) : 0;
         const int cnt = min(32, a1 - kb);
         for (int j0 = 0; j0 < cnt; j0 += REM_INFLIGHT) {
-            float w[REM_INFLIGHT];
+            float4 w[REM_INFLIGHT];
 #pragma unroll
             for (int u = 0; u < REM_INFLIGHT; ++u) {
                 const int g = __shfl_sync(0xffffffffu, gk, (j0 + u) & 31);
-                w[u] = (j0 + u < cnt) ? W32[(size_t)g * ld + s] : 0.0f;
+                if (j0 + u < cnt) w[u] = __ldg(reinterpret_cast<const float4*>(W32 + (size_t)g * ld));
             }
 #pragma unroll
             for (int u = 0; u < REM_INFLIGHT; ++u) {
@@ -686,61 +698,49 @@ __global__ void __launch_bounds__(REM_WARPS * 32) k_spmm_rem(Batch b) {
                     if (r != cur) {  // warp-uniform: the entry's row is the same on every lane
                         if (cur >= 0) {
                             if (first) {
-                                edge[warp][lane] = a;
-                                if (lane == 0) edge_row[warp] = cur;
+                                part[2 * warp][lane] = a;
+                                if (lane == 0) part_row[2 * warp] = cur;
                                 first = false;
                             } else {
-                                acc[cur][lane] = a;
+                                put(cur, a);
                             }
                         }
                         cur = r;
-                        a = 0.0f;
+                        a = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
-                    a = fmaf(v, w[u], a);
+                    a.x = fmaf(v, w[u].x, a.x);
+                    a.y = fmaf(v, w[u].y, a.y);
+                    a.z = fmaf(v, w[u].z, a.z);
+                    a.w = fmaf(v, w[u].w, a.w);
                 }
             }
         }
     }
     if (cur >= 0) {
-        if (first) {
-            edge[warp][lane] = a;
-            if (lane == 0) edge_row[warp] = cur;
+        const int slot = 2 * warp + (first ? 0 : 1);
+        part[slot][lane] = a;
+        if (lane == 0) part_row[slot] = cur;
+    }
+    __syncthreads();
+    if (warp) return;
+    // the ranges' ends, in warp order
+    cur = -1;
+    for (int i = 0; i < 2 * REM_WARPS; ++i) {
+        const int r = part_row[i];
+        if (r < 0) continue;
+        const float4 v = part[i][lane];
+        if (r != cur) {
+            if (cur >= 0) put(cur, a);
+            cur = r;
+            a = v;
         } else {
-            acc[cur][lane] = a;
+            a.x += v.x;
+            a.y += v.y;
+            a.z += v.z;
+            a.w += v.w;
         }
     }
-    __syncthreads();
-    // the edge sums, in warp order
-    if (warp == 0)
-        for (int w = 0; w < REM_WARPS; ++w) {
-            const int r = edge_row[w];
-            if (r >= 0) acc[r][lane] = acc[r][lane] + edge[w][lane];
-        }
-    __syncthreads();
-    float* R = static_cast<float*>(sv.W);
-    const int f = f_lo + threadIdx.x;
-    if (f >= f_hi || __ldg(&sv.rem_ptr[f]) == __ldg(&sv.rem_ptr[f + 1])) return;
-    for (int j = 0; j < REM_STEPS && s0 + j < ntau; ++j) R[(size_t)(s0 + j) * nf + f] = acc[threadIdx.x][j];
-}
-
-// Q += the remainder's sums, for the rows k_spmm_rem summed (same grid and
-// the same tests): runs once both the tensor-core product and the remainder
-// are complete, so the two can run side by side.
-__global__ void __launch_bounds__(128) k_rem_add(Batch b) {
-    const DevSolve& sv = b.tab[blockIdx.z];
-    const int rb = blockIdx.x, s0 = blockIdx.y * REM_STEPS;
-    const int nf = sv.nf, ntau = sv.ntau;
-    if (!sv.rem_ptr || rb * 128 >= nf || s0 >= ntau || !sv.ctl->active) return;
-    const bool everyone = !sv.freeze || sv.ti == 0.0f;
-    if (!everyone && !sv.rb_act[rb]) return;
-    const int f = rb * 128 + threadIdx.x;
-    if (f >= nf || __ldg(&sv.rem_ptr[f]) == __ldg(&sv.rem_ptr[f + 1])) return;
-    float* Q = static_cast<float*>(sv.Q);
-    const float* R = static_cast<const float*>(sv.W);
-    for (int j = 0; j < REM_STEPS && s0 + j < ntau; ++j) {
-        const size_t o = (size_t)(s0 + j) * nf + f;
-        Q[o] = Q[o] + R[o];
-    }
+    put(cur, a);
 }
 
 int launch_spmm_tc(const Batch& b, stream_t stv) {
@@ -765,29 +765,14 @@ int launch_spmm_tc(const Batch& b, stream_t stv) {
     if (cudaMemsetAsync(b.tc_work, 0, 2 * sizeof(int), st) != cudaSuccess) return 2;
     k_tc_compact<<<(b.nq + 127) / 128, 128, 0, st>>>(b);
     const int grid = b.nq < b.sms ? b.nq : b.sms;  // one persistent CTA per SM
-    // The sparse remainder (latency-bound gathers) runs beside the product
-    // (latency-bound on its copy ring) on the side stream, into its own sums.
-    // Submitting the remainder first was measured faster on the 8-inertia
-    // binary (two batch groups): 16.1 against 17.2 ms for the 6-revolution
-    // step, 255.5 against 260.5 ms solved to convergence.
-    const dim3 g((unsigned)b.rem_nmb, (unsigned)((b.rem_ntau + REM_STEPS - 1) / REM_STEPS), (unsigned)b.n);
-    cudaStream_t side = static_cast<cudaStream_t>(b.side);
-    const bool fork = b.rem_nmb > 0 && side && b.ev_fork && b.ev_join;
-    if (fork) {
-        cudaEvent_t ef = static_cast<cudaEvent_t>(b.ev_fork), ej = static_cast<cudaEvent_t>(b.ev_join);
-        if (cudaEventRecord(ef, st) != cudaSuccess || cudaStreamWaitEvent(side, ef, 0) != cudaSuccess) return 2;
-        k_spmm_rem<<<g, REM_WARPS * 32, 0, side>>>(b);
-        if (cudaEventRecord(ej, side) != cudaSuccess) return 2;
+    // The remainder first: the product's epilogue adds its sums.  (Side by side
+    // on two streams the two hardly overlapped, the product's shared memory
+    // leaving no room, and the sums needed a pass over Q of their own.)
+    if (b.rem_nmb > 0) {
+        const dim3 g((unsigned)b.rem_nmb, (unsigned)((b.rem_ntau + REM_STEPS - 1) / REM_STEPS), (unsigned)b.n);
+        k_spmm_rem<<<g, REM_WARPS * 32, 0, st>>>(b);
     }
     k_spmm_tc<<<grid, TC_THREADS, smem, st>>>(b);
-    if (b.rem_nmb > 0) {
-        if (fork) {
-            if (cudaStreamWaitEvent(st, static_cast<cudaEvent_t>(b.ev_join), 0) != cudaSuccess) return 2;
-        } else {
-            k_spmm_rem<<<g, REM_WARPS * 32, 0, st>>>(b);
-        }
-        k_rem_add<<<g, 128, 0, st>>>(b);
-    }
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

@@ -88,3 +88,29 @@ def test_fast_multiple_scattering(gpu_ctx, nf, ntau):
         s.close()
     bound = 2 * prob.scattering_accuracy * 0.25 / prob.albedo + 2.0 ** -16 * np.abs(out[1])
     assert np.all(np.abs(out[0] - out[1]) <= bound)
+
+
+@pytest.mark.parametrize("nf,ntau", [(40, 14), (301, 129), (515, 258)])
+@pytest.mark.parametrize("min_entries,bound", [(8192, 2.0 ** -17), (8, 2.0 ** -14)])
+def test_remainder_rows(gpu_ctx, monkeypatch, nf, ntau, min_entries, bound):
+    """FAST self-heating with every entry in the sparse remainder (66 FP32
+    products of one sign) and split between tiles and remainder (W in two BF16
+    parts, 2^-17, and the tensor core's truncated sums, 66 of 2^-21); the view
+    factors are exact in BF16."""
+    from binarytpm_gb300 import lib
+
+    monkeypatch.setenv("ATPM_TC_MIN_ENTRIES", str(min_entries))
+    prob = _problem(nf, ntau, 0)
+    prob.dep_vf[:] = np.ceil(prob.dep_vf * 2.0 ** 14) / np.float32(2.0 ** 14)
+    rng = np.random.default_rng(ntau)
+    s = lib.Solve(gpu_ctx, prob, precision=lib.FAST)
+    s.set_forcing(rng.integers(0, 2, (nf, ntau)).astype(np.int32), (600 * rng.random((nf, ntau))).astype(np.float32))
+    s.set_thermal_inertia(200.0)
+    s.initialise_temperatures()
+    s.revolution(0)
+    t = s.surface_temperature64()
+    q = s.selfheating_flux().T
+    w = 0.9 * 5.67e-8 * t ** 4
+    want = _sums(prob, np.zeros_like(w), w, float)
+    assert np.all(np.abs(q - want) <= bound * want)
+    s.close()
