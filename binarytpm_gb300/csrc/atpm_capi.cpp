@@ -133,7 +133,7 @@ struct Layout {
 
 enum {
     B_VERT, B_FAC, B_DPTR, B_DIDX, B_DVF, B_SHADOW, B_COS, B_EFM, B_E, B_S0, B_S1, B_TEMP, B_Q, B_W,
-    B_CONV, B_HOT, B_COUNTS, B_STATUS, B_CTL, B_DIAG, B_ACT, B_MEAN, B_RBACT, B_N
+    B_CONV, B_HOT, B_COUNTS, B_STATUS, B_CTL, B_DIAG, B_ACT, B_RBACT, B_N
 };
 
 Layout layout(int nv, int nf, int nnz, const atpm_params& P) {
@@ -161,7 +161,6 @@ Layout layout(int nv, int nf, int nnz, const atpm_params& P) {
     sz[B_CTL] = sizeof(Ctl);
     sz[B_DIAG] = 4 * 8;
     sz[B_ACT] = ((size_t)2 * nf + ACT_N) * 4;
-    sz[B_MEAN] = (size_t)nf * rs;
     sz[B_RBACT] = (size_t)(nf + 127) / 128;
     Layout L;
     size_t o = 0;
@@ -1156,7 +1155,7 @@ ATPM_API atpm_status atpm_solve_create(atpm_context* ctx, const atpm_shape* sh, 
     UP(d.dep_idx, sh->dep_idx, (size_t)s->nnz * 4);
     UP(d.dep_vf, sh->dep_vf, (size_t)s->nnz * 4);
 #undef UP
-    e = cudaMemsetAsync(a + L.off[B_CONV], 0, L.off[B_MEAN] - L.off[B_CONV], s->st);
+    e = cudaMemsetAsync(a + L.off[B_CONV], 0, L.off[B_RBACT] - L.off[B_CONV], s->st);
     if (e != cudaSuccess) goto cuda_fail;
     e = cudaMemsetAsync(d.rb_act, 1, (size_t)(s->nf + 127) / 128, s->st);  // every row block active
     if (e != cudaSuccess) goto cuda_fail;
@@ -1522,16 +1521,12 @@ ATPM_API atpm_status atpm_initialise_temperatures(atpm_solve* s) {
     if (!s) return fail(ATPM_E_INVALID, "null solve");
     if (!s->have_forcing) return fail(ATPM_E_STATE, "no forcing: call atpm_scattering or atpm_set_forcing");
     CK(cudaSetDevice(s->ctx->device));
-    const int nf = s->nf;
-    void* mean = static_cast<char*>(s->arena) + layout(s->nv, s->nf, s->nnz, s->P).off[B_MEAN];
-    if (launch_initial_mean(s->ds, mean, s->st)) return fail(ATPM_E_CUDA, "initial mean launch");
-    const atpm_params& P = s->P;
-    if (P.precision == ATPM_REFERENCE) {
+    if (s->P.precision == ATPM_REFERENCE) {
         atpm_status r = ensure_qroot_table(s->ctx);
         if (r) return r;
     }
-    if (launch_fill_initial(s->ds, mean, view(s->ctx->pq), s->st)) return fail(ATPM_E_CUDA, "fill launch");
-    if (P.precision != ATPM_FP64 && launch_w_bf16_one(s->ds, s->st)) return fail(ATPM_E_CUDA, "W launch");
+    if (launch_initial(s->ds, view(s->ctx->pq), s->ctx->sm_count, s->st))
+        return fail(ATPM_E_CUDA, "initial temperatures launch");
     CK(cudaStreamSynchronize(s->st));
     s->have_temps = true;
     return ATPM_OK;

@@ -317,9 +317,8 @@ int launch_revolution_part(const Batch& b, int part, stream_t st);
 // REFERENCE / FP64 conduction of one revolution (atpm_conduction_split.cu)
 int launch_conduction_split(const Batch& b, stream_t st);
 int launch_conduction_few(const Batch& b, stream_t st);  // FAST, few advancing facets
-int launch_initial_mean(const DevSolve& s, void* mean_out, stream_t st);
-// T0 = ((1-A) mean / (eps sigma))^0.25 (x^0.25 exact to libm through pq in REFERENCE)
-int launch_fill_initial(const DevSolve& s, const void* mean, const PowTab& pq, stream_t st);
+// T0 = ((1-A) mean / (eps sigma))^0.25 (x^0.25 exact to libm through pq in REFERENCE), and W of FAST
+int launch_initial(const DevSolve& s, const PowTab& pq, int sms, stream_t st);
 int launch_energy_balance(const DevSolve& s, stream_t st);
 
 // disk-integrated flux (atpm_flux.cu)

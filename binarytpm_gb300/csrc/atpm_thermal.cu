@@ -25,6 +25,8 @@
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 #include "atpm_column.cuh"
 #include "atpm_gather.cuh"
 #include "atpm_internal.h"
@@ -606,39 +608,115 @@ __global__ void k_advance(Batch b) {
 }
 
 // ------------------------------------------------------------- initial state
+// initialisetemperatures (main.cpp:1439-1467): the facet's mean absorbed flux,
+// summed in step order, -> T0 = ((1 - A) mean / (eps sigma))^0.25 everywhere in
+// its column and at every step; FAST's W (BF16 tiles and FP32 rows) with it.
+// A block owns 64 facets and a span of steps.  Its threads bring E in through
+// shared memory, kInitSteps steps at a time with the next ones in flight, and
+// one thread a facet sums them: a thread a facet on its own waited for E 720
+// times over.  W is constant over the steps, so it is packed once and stored
+// 16 bytes a lane.  Bound by the stores; FAST, 21,760 facets x 720 steps with
+// the W kernels 199 -> 77 us a call, 1,280 facets 53 -> 25.
+constexpr int kInitFacets = 64, kInitSteps = 32;
+
 template <int MODE>
-__global__ void k_initial_mean(DevSolve sv, void* out) {
+__global__ void __launch_bounds__(256) k_initial(DevSolve sv, PowTab pq) {
     using A = Ar<MODE>;
     using R = typename A::R;
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= sv.nf) return;
+    constexpr int PER = kInitFacets * kInitSteps / 256;  // elements a thread brings in at a time
+    __shared__ R e[kInitSteps][kInitFacets];
+    __shared__ R t0[kInitFacets];
+    __shared__ float w0[kInitFacets];
+    __shared__ __align__(16) __nv_bfloat16 wt[2][kInitFacets];
+    const int nf = sv.nf, ntau = sv.ntau, f0 = blockIdx.x * kInitFacets;
+    const int col = threadIdx.x % kInitFacets, row = threadIdx.x / kInitFacets, f = f0 + col;
+    constexpr int ROWS = 256 / kInitFacets;
     const R* E = static_cast<const R*>(sv.E);
-    const R inv = A::div(R(1), (R)sv.ntau);
-    R t = R(0);
-    for (int s = 0; s < sv.ntau; ++s) t = A::add(t, A::mul(inv, E[(size_t)s * sv.nf + f]));
-    static_cast<R*>(out)[f] = t;
-}
-
-// initialisetemperatures (main.cpp:1455-1462): the facet's mean absorbed
-// flux -> T0 = ((1 - A) mean / (eps sigma))^0.25 everywhere in its column
-template <int MODE>
-__global__ void k_fill_initial(DevSolve sv, const void* mean, PowTab pq) {
-    using R = typename Ar<MODE>::R;
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= sv.nf) return;
-    const R m = static_cast<const R*>(mean)[f];
-    R v;
-    if constexpr (MODE == MODE_FP64) {
-        v = sqrt(sqrt(__ddiv_rn(__dmul_rn(sv.oma_d, m), sv.es_d)));
-    } else {
-        const float x = __fdiv_rn(__fmul_rn(sv.oma, m), sv.es);
-        v = (MODE == MODE_REF) ? libm_qroot(pq, x, sv.status) : dev_qroot(x);  // powf(x, 0.25f)
+    R next[PER];
+    auto fetch = [&](int s0) {
+#pragma unroll
+        for (int j = 0; j < PER; ++j) {
+            const int s = s0 + row + j * ROWS;
+            next[j] = (f < nf && s < ntau) ? __ldg(E + (size_t)s * nf + f) : R(0);
+        }
+    };
+    const R inv = A::div(R(1), (R)ntau);
+    R m = R(0);
+    fetch(0);
+    for (int s0 = 0; s0 < ntau; s0 += kInitSteps) {
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < PER; ++j) e[row + j * ROWS][col] = next[j];
+        __syncthreads();
+        fetch(s0 + kInitSteps);
+        if (row == 0) {
+            if (s0 + kInitSteps <= ntau) {
+#pragma unroll
+                for (int j = 0; j < kInitSteps; ++j) m = A::add(m, A::mul(inv, e[j][col]));
+            } else {
+                for (int j = 0; s0 + j < ntau; ++j) m = A::add(m, A::mul(inv, e[j][col]));
+            }
+        }
     }
-    R* temp = static_cast<R*>(sv.temp);
-    R* S0 = static_cast<R*>(sv.stemp0);
-    R* S1 = static_cast<R*>(sv.stemp1);
-    for (int i = 0; i <= sv.nx; ++i) temp[(size_t)i * sv.nf + f] = v;
-    for (int s = 0; s < sv.ntau; ++s) { S0[(size_t)s * sv.nf + f] = v; S1[(size_t)s * sv.nf + f] = v; }
+    if (row == 0) {
+        R v = R(0);
+        if (f < nf) {
+            if constexpr (MODE == MODE_FP64) {
+                v = sqrt(sqrt(__ddiv_rn(__dmul_rn(sv.oma_d, m), sv.es_d)));
+            } else {
+                const float x = __fdiv_rn(__fmul_rn(sv.oma, m), sv.es);
+                v = (MODE == MODE_REF) ? libm_qroot(pq, x, sv.status) : dev_qroot(x);  // powf(x, 0.25f)
+            }
+        }
+        t0[col] = v;
+        if constexpr (MODE == MODE_FAST) {
+            const float w = f < nf ? fast_w(sv.es_w, v) : 0.0f;
+            const __nv_bfloat16 hi = __float2bfloat16_rn(w);
+            w0[col] = w;
+            wt[0][col] = hi;
+            wt[1][col] = w_lo(w, hi);
+        }
+    }
+    __syncthreads();
+    // this block's steps [b0, b1): whole multiples of 32 up to the last
+    const int span = ((ntau + 31) / 32 + gridDim.y - 1) / gridDim.y * 32;
+    const int b0 = blockIdx.y * span, b1 = min(ntau, b0 + span);
+    const R v = t0[col];
+    if (f < nf) {
+        R* S0 = static_cast<R*>(sv.stemp0);
+        R* S1 = static_cast<R*>(sv.stemp1);
+        for (int s = b0 + row; s < b1; s += ROWS) {
+            S0[(size_t)s * nf + f] = v;
+            S1[(size_t)s * nf + f] = v;
+        }
+        R* temp = static_cast<R*>(sv.temp);
+        if (blockIdx.y == 0)
+            for (int i = row; i <= sv.nx; i += ROWS) temp[(size_t)i * nf + f] = v;
+    }
+    if constexpr (MODE == MODE_FAST) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        if (sv.Wb) {  // eight lanes a step's row of 64 facets, swizzled
+            uint4* Wb = static_cast<uint4*>(sv.Wb) + (size_t)blockIdx.x * sv.tc_nchunks * sv.tc_n * 16;
+            const uint4* hi = reinterpret_cast<const uint4*>(wt[0]);
+            const uint4* lo = reinterpret_cast<const uint4*>(wt[1]);
+            for (int s = b0 + threadIdx.x / 8; s < b1; s += 32) {
+                const int n = s % sv.tc_n, at = lane & 7;
+                uint4* d = Wb + (size_t)(s / sv.tc_n) * sv.tc_n * 16 + n * 8 + at;
+                d[0] = hi[at ^ (n & 7)];
+                d[sv.tc_n * 8] = lo[at ^ (n & 7)];
+            }
+        }
+        if (sv.W32)
+            for (int r = warp; r < min(kInitFacets, nf - f0); r += 8) {
+                float* d = sv.W32 + (size_t)(f0 + r) * sv.w32_ld;
+                const float w = w0[r];
+                for (int s = b0 + 4 * lane; s < b1; s += 128) {
+                    if (s + 4 <= b1) *reinterpret_cast<float4*>(d + s) = make_float4(w, w, w, w);
+                    else
+                        for (int u = s; u < b1; ++u) d[u] = w;
+                }
+            }
+    }
 }
 
 // FP64 energy balance of the current revolution: sums over facets and steps
@@ -746,24 +824,17 @@ int launch_revolution(const Batch& b, stream_t st) {
     return 0;
 }
 
-int launch_initial_mean(const DevSolve& s, void* out, stream_t stv) {
+// the steps are split between blocks until there are two a SM: a block that
+// stores all of them takes 32 us a call at 1,280 facets x 720 steps, against
+// 25 us split; with four or eight a SM 5,440 facets take 39 and 53 us, with two 38
+int launch_initial(const DevSolve& s, const PowTab& pq, int sms, stream_t stv) {
     cudaStream_t st = static_cast<cudaStream_t>(stv);
-    const int g = (s.nf + 127) / 128;
+    const int g = (s.nf + kInitFacets - 1) / kInitFacets;
+    const dim3 grid((unsigned)g, (unsigned)std::max(1, std::min((s.ntau + 31) / 32, 2 * sms / g)));
     switch (s.mode) {
-        case MODE_REF: k_initial_mean<MODE_REF><<<g, 128, 0, st>>>(s, out); break;
-        case MODE_FP64: k_initial_mean<MODE_FP64><<<g, 128, 0, st>>>(s, out); break;
-        default: k_initial_mean<MODE_FAST><<<g, 128, 0, st>>>(s, out); break;
-    }
-    return cudaGetLastError() == cudaSuccess ? 0 : 2;
-}
-
-int launch_fill_initial(const DevSolve& s, const void* mean, const PowTab& pq, stream_t stv) {
-    cudaStream_t st = static_cast<cudaStream_t>(stv);
-    const int g = (s.nf + 127) / 128;
-    switch (s.mode) {
-        case MODE_REF: k_fill_initial<MODE_REF><<<g, 128, 0, st>>>(s, mean, pq); break;
-        case MODE_FP64: k_fill_initial<MODE_FP64><<<g, 128, 0, st>>>(s, mean, pq); break;
-        default: k_fill_initial<MODE_FAST><<<g, 128, 0, st>>>(s, mean, pq); break;
+        case MODE_REF: k_initial<MODE_REF><<<grid, 256, 0, st>>>(s, pq); break;
+        case MODE_FP64: k_initial<MODE_FP64><<<grid, 256, 0, st>>>(s, pq); break;
+        default: k_initial<MODE_FAST><<<grid, 256, 0, st>>>(s, pq); break;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
