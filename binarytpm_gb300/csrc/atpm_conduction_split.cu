@@ -311,7 +311,7 @@ __global__ void __launch_bounds__(32) k_conduction_split(Batch b) {
     else column_split<MODE, NX, L>(sv, b, fc, live, sm);
 }
 
-// FAST: the facets k_tail_mode counted, as warps of 32 / L facets of one solve
+// FAST: the facets k_prepare counted, as warps of 32 / L facets of one solve
 // each (the active-facet list where one is kept for this revolution, else the
 // facet range)
 template <int NX, int L>
@@ -397,7 +397,7 @@ int launch_conduction_split(const Batch& b, stream_t stv) {
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 
-// FAST: runs the revolutions that k_tail_mode gives it, returns at once in the
+// FAST: runs the revolutions that k_prepare gives it, returns at once in the
 // others
 int launch_conduction_few(const Batch& b, stream_t stv) {
     cudaStream_t st = static_cast<cudaStream_t>(stv);

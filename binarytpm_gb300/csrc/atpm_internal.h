@@ -122,7 +122,7 @@ __device__ __forceinline__ float libm_qroot(const PowTab& t, float x, int* statu
 }
 #endif
 
-// per-solve control words (device memory, updated by the advance kernel)
+// per-solve control words (device memory, updated by k_converge)
 struct Ctl {
     int rev;        // next revolution index
     int active;     // 1 while the revolution loop runs
@@ -132,8 +132,8 @@ struct Ctl {
 
 // act_cnt beyond the lists: lanes per facet of the split sweep (batch leader; 0:
 // the thread-per-facet kernels run), its warps in all (batch leader), and this
-// solve's first warp
-enum : int { ACT_LANES = 4, ACT_WARPS = 5, ACT_START = 6, ACT_N = 7 };
+// solve's first warp; tickets of k_converge's blocks (batch leader)
+enum : int { ACT_LANES = 4, ACT_WARPS = 5, ACT_START = 6, ACT_TICKET = 7, ACT_N = 8 };
 
 struct DevSolve {
     int nf, nv, ntau, nx, revcap, mode;
@@ -161,11 +161,11 @@ struct DevSolve {
     uint8_t* hot;            // [nf] some |stemp1-stemp0| >= TACC this revolution
     // facets still active after each convergence test (FAST, freeze on),
     // double-buffered by revolution parity: k_converge of revolution r fills
-    // list (r+1)&1, the conduction of r+1 reads it, k_advance of r+1 clears it
+    // list (r+1)&1, the conduction of r+1 reads it, the end of r+1 clears it
     uint8_t* rb_act;         // [ceil(nf/128)] some facet of the 128-facet row block active (FAST)
     int* act_list;           // [2][nf]
     int* act_cnt;            // [ACT_N]: counts of the two lists, the revolution each list is for, then
-                             // this revolution's split sweep (k_tail_mode)
+                             // this revolution's split sweep (k_prepare), and the convergence test's ticket
     int* counts;             // [revcap] numconverged after each revolution
     int* status;             // ST_* bits
     Ctl* ctl;
@@ -278,7 +278,7 @@ struct Batch {
     const int4* qmap;        // tensor-core work items {solve, row block, step chunk, 0}
     int nq;
     int4* tc_list;           // [nq] this launch's items whose row block has an active facet
-    int* tc_work;            // [2] list length, next ticket (zeroed before every launch)
+    int* tc_work;            // [2] list length, next ticket (k_prepare)
     int tc_nmax;             // largest step chunk in the batch
     int cond_variant;        // FAST conduction register/occupancy variant (1, 2, 3)
     int tc_stages;           // tensor-core pipeline depth (0: deepest that fits)
@@ -292,7 +292,7 @@ struct Batch {
 };
 // deepest tensor-core pipeline that fits shared memory for step chunk N
 int tc_max_stages(int N);
-int launch_revolution(const Batch& b, stream_t st);  // W, Q, conduction, convergence, advance
+int launch_revolution(const Batch& b, stream_t st);  // W, Q, conduction, convergence
 // per solve: control word (4), status, counts of the last `window` revolutions
 int launch_progress(const Batch& b, int window, int* out, stream_t st);
 int kernels_per_revolution(const Batch& b);          // kernels launch_revolution starts
@@ -312,7 +312,7 @@ int launch_rem_fill(const DevSolve& s, int nkb, const int* slot, const int* rptr
 int launch_tc_rowneed(const DevSolve& s, int nkb, unsigned* need, stream_t st);
 int launch_tc_fill(const DevSolve& s, int nkb, const int* slot, const int* lo_of, void* tiles, void* lo_tiles,
                    stream_t st);
-// part 0 W, 1 Q, 2 conduction, 3 convergence, 4 advance
+// part 0 preparation and W, 1 Q, 2 conduction, 3 convergence and advance (4: none)
 int launch_revolution_part(const Batch& b, int part, stream_t st);
 // REFERENCE / FP64 conduction of one revolution (atpm_conduction_split.cu)
 int launch_conduction_split(const Batch& b, stream_t st);

@@ -30,7 +30,7 @@
 // with one bulk copy (cp.async.bulk) into a shared-memory stage ring.  The
 // product kernel is persistent (one CTA per SM) and warp-specialised: a
 // producer warp takes work items (row block x step chunk) by ticket from the
-// list k_tc_compact builds before each launch and streams their tiles, an MMA
+// list k_prepare builds before each launch and streams their tiles, an MMA
 // warp issues tcgen05.mma (M = 128, N = step chunk, K = 16) into one of two
 // TMEM accumulators, and four epilogue warps drain the other with
 // tcgen05.ld and write Q coalesced along facets.  All-zero 16-wide K slices
@@ -349,26 +349,6 @@ int launch_rem_fill(const DevSolve& s, int nkb, const int* slot, const int* rptr
     const size_t threads = (size_t)s.nf * 32;
     k_rem_fill<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(s, nkb, slot, rptr, ridx, rvf, rrow);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
-}
-
-// Work items whose row block has an active facet, compacted before every
-// launch (in map order within each warp), so tickets are spent on work only.
-__global__ void __launch_bounds__(128) k_tc_compact(Batch b) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    bool use = false;
-    int4 it = make_int4(0, 0, 0, 0);
-    if (i < b.nq) {
-        it = b.qmap[i];
-        const DevSolve& sv = b.tab[it.x];
-        const bool everyone = !sv.freeze || sv.ti == 0.0f;
-        use = sv.ctl->active && sv.tc_tiles && (everyone || sv.rb_act[it.y]);
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, use);
-    const int lane = threadIdx.x & 31;
-    int base = 0;
-    if (lane == 0 && m) base = atomicAdd(&b.tc_work[0], __popc(m));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (use) b.tc_list[base + __popc(m & ((1u << lane) - 1u))] = it;
 }
 
 // Persistent, warp-specialised: one CTA per SM.  Work items are handed out
@@ -760,10 +740,6 @@ int launch_spmm_tc(const Batch& b, stream_t stv) {
             return 2;
         attr_set.fetch_or(bit, std::memory_order_release);
     }
-    // the list length and the ticket counter start at zero for every launch
-    // (a memset node when the revolution is captured in a graph)
-    if (cudaMemsetAsync(b.tc_work, 0, 2 * sizeof(int), st) != cudaSuccess) return 2;
-    k_tc_compact<<<(b.nq + 127) / 128, 128, 0, st>>>(b);
     const int grid = b.nq < b.sms ? b.nq : b.sms;  // one persistent CTA per SM
     // The remainder first: the product's epilogue adds its sums.  (Side by side
     // on two streams the two hardly overlapped, the product's shared memory

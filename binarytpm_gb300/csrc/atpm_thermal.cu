@@ -12,12 +12,12 @@
 //   k_conduction   depth column in registers, NTAU steps, Newton BC -- A1
 //                  (FAST: over the active-facet list once at most half a
 //                  solve is active)
-//   k_tail_mode, k_conduction_few   FAST revolutions with few advancing facets:
+//   k_prepare, k_conduction_few   FAST revolutions with few advancing facets:
 //                  several lanes per facet (atpm_conduction_split.cu, as the
 //                  REFERENCE and FP64 sweeps)
 //   k_converge     shape_converged (main.cpp:1876-1909)             -- A4
 //                  (+ the active-facet lists and row-block activity)
-//   k_advance      revolution counter / stop rule (main.cpp:2522-2539)
+//   advance        revolution counter / stop rule (main.cpp:2522-2539)
 //
 // All of them read the per-solve control word and return at once for solves
 // that have stopped, so the same launch sequence (or a captured graph of it)
@@ -415,13 +415,13 @@ __device__ __forceinline__ void column_revolution_fast2(const DevSolve& sv, int 
 }
 
 // How a FAST revolution's depth sweep runs, decided once per revolution from
-// the facets that advance (one warp over the solves): with few of them the
+// the facets that advance (one warp, over the solves): with few of them the
 // lane-split sweep takes every solve (k_conduction_few; its warps are dealt
 // out here, solve by solve), else the thread-per-facet kernels do.  The answer
 // goes to the batch's first solve, where all of them read it: exactly one of
 // the forms advances each facet.
-__global__ void k_tail_mode(Batch b) {
-    const int lane = threadIdx.x;
+__device__ __forceinline__ void tail_mode(const Batch& b) {
+    const int lane = threadIdx.x & 31;
     auto advancing = [&](int i) {
         if (i >= b.n) return 0;
         const DevSolve& s = b.tab[i];
@@ -451,6 +451,74 @@ __global__ void k_tail_mode(Batch b) {
     if (lane == 0) {
         b.tab[0].act_cnt[ACT_LANES] = lanes;
         b.tab[0].act_cnt[ACT_WARPS] = start;
+    }
+}
+
+// What a FAST revolution needs to know before it runs, in one block: how its
+// depth sweep runs, and the product's work items whose row block has an active
+// facet, in map order, so that tickets are spent on work only.  A kernel for
+// each and a memset of the counters cost a few us apiece in revolutions of
+// some 140 (single solves, late revolutions): with the end of the revolution in
+// k_converge, 1,280 facets 140.5 -> 137.5 us.
+constexpr int kPrepItems = 8;  // items a thread looks at in one pass
+
+__global__ void __launch_bounds__(1024) k_prepare(Batch b) {
+    __shared__ int at[kPrepItems * 32];
+    __shared__ int count;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (warp == 31) tail_mode(b);
+    if (b.nq == 0) return;
+    int base = 0;
+    for (int i0 = 0; i0 < b.nq; i0 += 1024 * kPrepItems) {
+        int4 it[kPrepItems];
+        unsigned m[kPrepItems];
+#pragma unroll
+        for (int k = 0; k < kPrepItems; ++k) {
+            const int i = i0 + k * 1024 + threadIdx.x;
+            if (i < b.nq) it[k] = b.qmap[i];
+        }
+#pragma unroll
+        for (int k = 0; k < kPrepItems; ++k) {
+            bool use = false;
+            if (i0 + k * 1024 + threadIdx.x < b.nq) {
+                const DevSolve& sv = b.tab[it[k].x];
+                const bool everyone = !sv.freeze || sv.ti == 0.0f;
+                use = sv.ctl->active && sv.tc_tiles && (everyone || sv.rb_act[it[k].y]);
+            }
+            m[k] = __ballot_sync(0xffffffffu, use);
+            if (lane == 0) at[k * 32 + warp] = __popc(m[k]);
+        }
+        __syncthreads();
+        if (warp == 0) {  // exclusive sums of the counts, kPrepItems consecutive ones a lane
+            int c[kPrepItems], sum = 0;
+#pragma unroll
+            for (int k = 0; k < kPrepItems; ++k) {
+                c[k] = at[lane * kPrepItems + k];
+                sum += c[k];
+            }
+            int x = sum;
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) count = x;
+            x += base - sum;
+#pragma unroll
+            for (int k = 0; k < kPrepItems; ++k) {
+                at[lane * kPrepItems + k] = x;
+                x += c[k];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kPrepItems; ++k)
+            if ((m[k] >> lane) & 1u) b.tc_list[at[k * 32 + warp] + __popc(m[k] & ((1u << lane) - 1u))] = it[k];
+        base += count;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        b.tc_work[0] = base;  // list length
+        b.tc_work[1] = 0;     // next ticket
     }
 }
 
@@ -546,7 +614,26 @@ __global__ void __launch_bounds__(64, 4) k_conduction_pairs(Batch b) {
 }
 
 // -------------------------------------------------------------- convergence
-__global__ void __launch_bounds__(128) k_converge(Batch b) {
+// the end of a solve's revolution
+__device__ __forceinline__ void advance(const DevSolve& sv) {
+    Ctl* ctl = sv.ctl;
+    if (!ctl->active) return;
+    const int rev = ctl->rev;
+    if (rev > 5) {
+        const int n = __ldcg(&sv.counts[rev]);
+        ctl->numconv = n;
+        ctl->converged = (n == sv.nf) ? 1 : 0;
+    } else {
+        sv.counts[rev] = ctl->numconv;
+    }
+    // read by this revolution's conduction; k_converge of rev + 1 refills it
+    sv.act_cnt[rev & 1] = 0;
+    sv.act_cnt[2 + (rev & 1)] = -1;
+    ctl->rev = rev + 1;
+    if (ctl->converged || rev + 1 >= sv.revcap || (*sv.status & ST_NONFINITE)) ctl->active = 0;
+}
+
+__device__ __forceinline__ void converge(const Batch& b) {
     const int2 fb = b.fmap[blockIdx.x];
     const DevSolve& sv = b.tab[fb.x];
     if (!sv.ctl->active) return;
@@ -586,25 +673,22 @@ __global__ void __launch_bounds__(128) k_converge(Batch b) {
     }
 }
 
-__global__ void k_advance(Batch b) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= b.n) return;
-    const DevSolve& sv = b.tab[i];
-    Ctl* ctl = sv.ctl;
-    if (!ctl->active) return;
-    const int rev = ctl->rev;
-    if (rev > 5) {
-        const int n = sv.counts[rev];
-        ctl->numconv = n;
-        ctl->converged = (n == sv.nf) ? 1 : 0;
-    } else {
-        sv.counts[rev] = ctl->numconv;
+// The convergence test, and with the last block to finish the end of the
+// revolution for every solve (a kernel of its own took 3 to 5 us).  The ticket
+// counter, of the batch's first solve, wraps to zero with the last block.
+__global__ void __launch_bounds__(128) k_converge(Batch b) {
+    __shared__ bool last;
+    converge(b);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        unsigned* ticket = reinterpret_cast<unsigned*>(&b.tab[0].act_cnt[ACT_TICKET]);
+        last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
     }
-    // read by this revolution's conduction; k_converge of rev + 1 refills it
-    sv.act_cnt[rev & 1] = 0;
-    sv.act_cnt[2 + (rev & 1)] = -1;
-    ctl->rev = rev + 1;
-    if (ctl->converged || rev + 1 >= sv.revcap || (*sv.status & ST_NONFINITE)) ctl->active = 0;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int i = threadIdx.x; i < b.n; i += blockDim.x) advance(b.tab[i]);
 }
 
 // ------------------------------------------------------------- initial state
@@ -763,9 +847,10 @@ bool conduction_nx_supported(int nx) {
 
 template <int MODE>
 static int launch_rev_part(const Batch& b, int part, cudaStream_t st) {
-    // FAST + tensor cores: the conduction sweep keeps W current (store_w), so
-    // part 0 has nothing to do
-    if (MODE == MODE_FAST && b.nq > 0 && part < 2) return part == 0 ? 0 : launch_spmm_tc(b, st);
+    if (MODE == MODE_FAST && part == 0) k_prepare<<<1, 1024, 0, st>>>(b);
+    // FAST + tensor cores: the conduction sweep keeps W current (store_w)
+    if (MODE == MODE_FAST && b.nq > 0 && part == 0) return cudaGetLastError() == cudaSuccess ? 0 : 2;
+    if (MODE == MODE_FAST && b.nq > 0 && part == 1) return launch_spmm_tc(b, st);
     switch (part) {
         case 0: if (b.nw > 0) k_selfheat_w<MODE><<<b.nw, dim3(32, 8), 0, st>>>(b); break;
         case 1: {
@@ -776,7 +861,6 @@ static int launch_rev_part(const Batch& b, int part, cudaStream_t st) {
         }
         case 2:
             if (MODE != MODE_FAST) return launch_conduction_split(b, st);
-            k_tail_mode<<<1, 32, 0, st>>>(b);
             switch (b.nx) {
 #define NX_CASE(N)                                                                       \
     case N:                                                                               \
@@ -791,7 +875,7 @@ static int launch_rev_part(const Batch& b, int part, cudaStream_t st) {
             }
             return launch_conduction_few(b, st);
         case 3: k_converge<<<b.nfb, 128, 0, st>>>(b); break;
-        case 4: k_advance<<<(b.n + 127) / 128, 128, 0, st>>>(b); break;
+        case 4: break;  // the end of the revolution: k_converge's last block
         default: return 1;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
@@ -809,11 +893,11 @@ int launch_revolution_part(const Batch& b, int part, stream_t stv) {
 
 int kernels_per_revolution(const Batch& b) {
     const bool tc = b.mode == MODE_FAST && b.nq > 0;
-    // k_tc_compact + k_spmm_tc (+ k_spmm_rem), or W + Q
-    const int selfheat = tc ? 2 + (b.rem_nmb > 0 ? 1 : 0) : (b.nw > 0 ? 2 : 0);
-    // + k_tail_mode, k_conduction_few (+ k_conduction_pairs)
+    // k_spmm_tc (+ k_spmm_rem), or W + Q
+    const int selfheat = tc ? 1 + (b.rem_nmb > 0 ? 1 : 0) : (b.nw > 0 ? 2 : 0);
+    // k_prepare, k_conduction, k_conduction_few (+ k_conduction_pairs)
     const int conduction = b.mode == MODE_FAST ? (b.cond_variant == 4 ? 4 : 3) : 1;
-    return selfheat + conduction + 2;                    // + k_converge, k_advance
+    return selfheat + conduction + 1;                    // + k_converge
 }
 
 int launch_revolution(const Batch& b, stream_t st) {
