@@ -10,7 +10,7 @@
 //                        sub-facet against the analytic crater rim, every
 //                        (facet, step) in one launch
 //   k_crater_scatter     roughness_single/multiple_scattering (216-304):
-//                        one block per (facet, step) batch, the 100x100
+//                        one block per batch of a facet's steps, the 100x100
 //                        crater view-factor matrix staged in shared memory
 //   k_crater_revolution  finite_difference + boundary_condition (377-490)
 //                        for a whole revolution in ONE launch: a block owns a
@@ -28,27 +28,12 @@
 // runs.  FAST precision contracts and reorders.
 #include <cuda_runtime.h>
 
+#include "atpm_crater_rim.cuh"
 #include "atpm_internal.h"
 
 namespace atpm {
 
 namespace {
-
-template <int MODE> struct Ca;
-template <> struct Ca<MODE_REF> {
-    static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
-    static __device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b); }
-    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
-    static __device__ __forceinline__ float div(float a, float b) { return __fdiv_rn(a, b); }
-    static __device__ __forceinline__ float sqrt_(float a) { return __fsqrt_rn(a); }
-};
-template <> struct Ca<MODE_FAST> {
-    static __device__ __forceinline__ float add(float a, float b) { return a + b; }
-    static __device__ __forceinline__ float sub(float a, float b) { return a - b; }
-    static __device__ __forceinline__ float mul(float a, float b) { return a * b; }
-    static __device__ __forceinline__ float div(float a, float b) { return a / b; }
-    static __device__ __forceinline__ float sqrt_(float a) { return sqrtf(a); }
-};
 
 __device__ __forceinline__ float cpow4_exact(const PowTab& t, float x, int* st) {
     // x^4 corrected to this host's libm powf (atpm_powtab.cpp)
@@ -63,99 +48,166 @@ __device__ __forceinline__ float cpow4(const PowTab& t, float x, int* st) {
 
 }  // namespace
 
-// sfcpartialshadow: each thread owns one (facet, step, sub-facet)
+// sfcpartialshadow: a block takes kRimDirs consecutive (facet, step) Sun
+// directions at a time, a thread one sub-facet in all of them.  A sub-facet
+// that is dark already has nothing to lose and is skipped.  Bound by
+// instruction issue; one direction at a time, with its square root for every
+// point, 160 facets x 360 steps took 665 us in REFERENCE, now 298; 200 x 720 in
+// FAST 1,105 and 660.
 template <int MODE>
 __global__ void __launch_bounds__(128) k_crater_shadow(CraterDev c) {
     using A = Ca<MODE>;
-    const int nsf = c.nsf;
+    __shared__ RimShared r;
+    __shared__ float dir[2][kRimDirs][3];  // direction and slope
+    __shared__ int lit[2][kRimDirs];
+    const int nsf = c.nsf, j = threadIdx.x;
     const long long n = (long long)c.nf * c.ntau;
-    const int j = threadIdx.x;
-    for (long long fs = blockIdx.x; fs < n; fs += gridDim.x) {
-        if (c.shadow[fs] != 1) continue;  // block-uniform
-        if (j >= nsf) continue;
-        const float* iv = c.illumvec + 3 * fs;
-        // sun vector normalised by its x-y length (GPU_code.cu:177-181)
-        const float s = A::sqrt_(A::add(A::mul(iv[0], iv[0]), A::mul(iv[1], iv[1])));
-        const float sv0 = A::div(iv[0], s), sv1 = A::div(iv[1], s), sv2 = A::div(iv[2], s);
-        const float a = A::div(fabsf(sv2), A::sqrt_(A::add(A::mul(sv0, sv0), A::mul(sv1, sv1))));
-        float sh = c.sfc_shadow[fs * nsf + j];
-        const float* v2 = c.cverts + 3 * c.cfac[3 * j + 2];
-        const float* t0 = c.ctri + 6 * j;
-        const float* t1 = t0 + 3;
-        const float R = 10.0f;
-        for (int p = 0; p != 100; ++p) {
-            const float m0 = c.cmult[2 * p], m1 = c.cmult[2 * p + 1];
-            float mp[3];
-#pragma unroll
-            for (int k = 0; k < 3; ++k) mp[k] = A::add(A::add(v2[k], A::mul(m0, t0[k])), A::mul(m1, t1[k]));
-            const float tc1 = A::add(A::mul(A::mul(-1.0f, sv1), mp[0]), A::mul(sv0, mp[1]));
-            const float rad = A::sqrt_(A::sub(A::mul(R, R), A::mul(tc1, tc1)));
-            const float tc0 = A::sub(A::add(A::mul(sv0, mp[0]), A::mul(sv1, mp[1])), rad);
-            if (mp[2] <= A::mul(a, tc0) && sh != 0.0f) sh = A::sub(sh, A::div(1.0f, 100.0f));
-            if (sh < 0.0f) sh = 0.0f;
+    rim_open<MODE>(r, c);
+    Rim<MODE> rim;
+    if (j < nsf) rim.load(c, r, j);
+    int turn = 0;
+    for (long long fs0 = (long long)blockIdx.x * kRimDirs; fs0 < n; fs0 += (long long)gridDim.x * kRimDirs, turn ^= 1) {
+        if (threadIdx.x < kRimDirs) {
+            const long long fs = fs0 + threadIdx.x;
+            const bool use = fs < n && c.shadow[fs] == 1;
+            lit[turn][threadIdx.x] = use;
+            if (use) {
+                const float* iv = c.illumvec + 3 * fs;
+                // sun vector normalised by its x-y length (GPU_code.cu:177-181)
+                const float s = A::sqrt_(A::add(A::mul(iv[0], iv[0]), A::mul(iv[1], iv[1])));
+                const float sv0 = A::div(iv[0], s), sv1 = A::div(iv[1], s), sv2 = A::div(iv[2], s);
+                dir[turn][threadIdx.x][0] = sv0;
+                dir[turn][threadIdx.x][1] = sv1;
+                dir[turn][threadIdx.x][2] = A::div(fabsf(sv2), A::sqrt_(A::add(A::mul(sv0, sv0), A::mul(sv1, sv1))));
+            }
         }
-        c.sfc_shadow[fs * nsf + j] = sh;
+        __syncthreads();  // the other turn's directions are overwritten only after the next one
+        if (j >= nsf) continue;
+        float sh[kRimDirs], w0[kRimDirs], w1[kRimDirs], a[kRimDirs];
+        bool any = false;
+#pragma unroll
+        for (int d = 0; d < kRimDirs; ++d) {
+            const bool use = lit[turn][d];
+            sh[d] = use ? c.sfc_shadow[(fs0 + d) * nsf + j] : 0.0f;
+            any = any || sh[d] != 0.0f;
+            w0[d] = use ? dir[turn][d][0] : 0.0f;
+            w1[d] = use ? dir[turn][d][1] : 0.0f;
+            a[d] = use ? dir[turn][d][2] : 1.0f;
+        }
+        if (!any) continue;
+        int m[kRimDirs];
+        rim.count(r, w0, w1, a, m);
+#pragma unroll
+        for (int d = 0; d < kRimDirs; ++d)
+            if (sh[d] != 0.0f)
+                c.sfc_shadow[(fs0 + d) * nsf + j] = sh[d] == 1.0f ? r.left[m[d]] : rim_take<MODE>(sh[d], m[d]);
     }
 }
 
-// single (multiple == 0) or single + Jacobi multiple scattering of one
-// (facet, step) per block iteration
+// single (multiple == 0) or single + Jacobi multiple scattering of kScatSteps
+// steps of a facet per block iteration: a view factor is read once for all of
+// them, and two barriers an iteration serve them all.  A step that has
+// converged keeps its values while the others go on.  Bound by shared-memory
+// reads; one step at a time 160 facets x 360 steps took 495 us in REFERENCE, now
+// 307; 200 x 720 in FAST 1,164 and 607.
+constexpr int kScatSteps = 4;
+
 template <int MODE>
 __global__ void __launch_bounds__(128) k_crater_scatter(CraterDev c, float solar, float acc, int multiple, int cap) {
     using A = Ca<MODE>;
-    extern __shared__ float sm[];
+    extern __shared__ __align__(16) float sm[];
     const int nsf = c.nsf;
-    float* Vs = sm;                 // nsf*nsf
-    float* ill = Vs + nsf * nsf;    // nsf
-    float* pold = ill + nsf;        // nsf
-    __shared__ int more;
+    float4* vals = reinterpret_cast<float4*>(sm);  // nsf: illumination, then the last iterate, of the four steps
+    float* Vs = sm + 4 * nsf;                      // nsf * nsf
+    __shared__ int more[2];
     for (int k = threadIdx.x; k < nsf * nsf; k += blockDim.x) Vs[k] = c.V[k];
-    __syncthreads();
-    const long long n = (long long)c.nf * c.ntau;
+    if (threadIdx.x < 2) more[threadIdx.x] = 0;
+    const int per = (c.ntau + kScatSteps - 1) / kScatSteps;
+    const long long n = (long long)c.nf * per;
     const int j = threadIdx.x;
-    for (long long fs = blockIdx.x; fs < n; fs += gridDim.x) {
-        const int f = (int)(fs / c.ntau);
+    for (long long g = blockIdx.x; g < n; g += gridDim.x) {
+        const int f = (int)(g / per), s0 = (int)(g % per) * kScatSteps, ns = min(kScatSteps, c.ntau - s0);
         const float alb = c.albedo[f];
-        const size_t o = (size_t)fs * nsf + j;
-        float solarpower = 0.0f, tot = 0.0f;
-        if (j < nsf) {
-            const float sh = c.sfc_shadow[o], ia = c.illumangle[o], gi = c.RGI[o];
-            ill[j] = A::add(A::mul(A::mul(solar, sh), ia), gi);
-            solarpower = A::add(A::mul(A::mul(solar, ia), sh), gi);
+        const size_t o = ((size_t)f * c.ntau + s0) * nsf + j;
+        float power[kScatSteps], tot[kScatSteps], w[kScatSteps];
+#pragma unroll
+        for (int d = 0; d < kScatSteps; ++d) {
+            power[d] = tot[d] = 0.0f;
+            if (j < nsf && d < ns) {
+                const size_t od = o + (size_t)d * nsf;
+                const float sh = c.sfc_shadow[od], ia = c.illumangle[od], gi = c.RGI[od];
+                tot[d] = A::add(A::mul(A::mul(solar, sh), ia), gi);
+                power[d] = A::add(A::mul(A::mul(solar, ia), sh), gi);
+            }
         }
+        __syncthreads();  // the last steps' values are read
+        if (j < nsf) vals[j] = make_float4(tot[0], tot[1], tot[2], tot[3]);
         __syncthreads();
+        auto terms = [&](int i, float v) {
+            const float4 x = vals[i];
+            w[0] = A::mul(v, x.x);
+            w[1] = A::mul(v, x.y);
+            w[2] = A::mul(v, x.z);
+            w[3] = A::mul(v, x.w);
+        };
         if (j < nsf) {
-            tot = ill[j];
-            for (int i = 0; i != nsf; ++i) tot = A::add(tot, A::mul(A::mul(Vs[i * nsf + j], alb), ill[i]));
-            if (tot <= 0.0f) tot = 0.0f;
+#pragma unroll 4
+            for (int i = 0; i < nsf; ++i) {
+                terms(i, A::mul(Vs[i * nsf + j], alb));
+#pragma unroll
+                for (int d = 0; d < kScatSteps; ++d) tot[d] = A::add(tot[d], w[d]);
+            }
+#pragma unroll
+            for (int d = 0; d < kScatSteps; ++d)
+                if (tot[d] <= 0.0f) tot[d] = 0.0f;
         }
         if (multiple) {
-            float pnew = 0.0f;
-            if (j < nsf) pold[j] = A::mul(alb, tot);
+            float old[kScatSteps], next[kScatSteps] = {};
             __syncthreads();
+#pragma unroll
+            for (int d = 0; d < kScatSteps; ++d) old[d] = A::mul(alb, tot[d]);
+            if (j < nsf) vals[j] = make_float4(old[0], old[1], old[2], old[3]);
+            __syncthreads();
+            int going = (1 << ns) - 1;  // uniform: steps that have not converged
             for (int it = 0; it < cap; ++it) {
-                if (threadIdx.x == 0) more = 0;
-                float sum = 0.0f;
+                float sum[kScatSteps] = {};
                 if (j < nsf) {
-                    for (int i = 0; i != nsf; ++i) sum = A::add(sum, A::mul(Vs[i * nsf + j], pold[i]));
-                    pnew = A::mul(alb, A::add(solarpower, sum));
+#pragma unroll 4
+                    for (int i = 0; i < nsf; ++i) {
+                        terms(i, Vs[i * nsf + j]);
+#pragma unroll
+                        for (int d = 0; d < kScatSteps; ++d) sum[d] = A::add(sum[d], w[d]);
+                    }
                 }
-                __syncthreads();
+                __syncthreads();  // the iterate and the last flags are read
+                int moved = 0;
                 if (j < nsf) {
-                    const float d = A::sub(pnew, pold[j]);
-                    if (fabsf(d) > acc) more = 1;
-                    pold[j] = pnew;
+#pragma unroll
+                    for (int d = 0; d < kScatSteps; ++d)
+                        if ((going >> d) & 1) {
+                            next[d] = A::mul(alb, A::add(power[d], sum[d]));
+                            if (fabsf(A::sub(next[d], old[d])) > acc) moved |= 1 << d;
+                            old[d] = next[d];
+                        }
+                    vals[j] = make_float4(old[0], old[1], old[2], old[3]);
                 }
+                moved = __reduce_or_sync(0xffffffffu, moved);
+                if ((threadIdx.x & 31) == 0 && moved) atomicOr(&more[it & 1], moved);
+                if (threadIdx.x == 0) more[(it + 1) & 1] = 0;
                 __syncthreads();
-                const int m = more;
-                __syncthreads();
-                if (!m) break;
+                going = more[it & 1];
+                if (!going) break;
                 if (it + 1 == cap && threadIdx.x == 0) atomicOr(c.status, ST_SCATTER_CAP);
             }
-            tot = A::div(pnew, alb);
+#pragma unroll
+            for (int d = 0; d < kScatSteps; ++d) tot[d] = A::div(next[d], alb);
+            __syncthreads();
+            if (threadIdx.x < 2) more[threadIdx.x] = 0;  // the next steps begin with the flags of iteration 0
         }
-        if (j < nsf) c.RI[o] = tot;
-        __syncthreads();
+        if (j < nsf)
+#pragma unroll
+            for (int d = 0; d < kScatSteps; ++d)
+                if (d < ns) c.RI[o + (size_t)d * nsf] = tot[d];
     }
 }
 
@@ -537,11 +589,20 @@ int crater_launch(int what, const CraterDev& c, const PowTab& p4, const PowTab& 
     const int grid_fs = 152 * 8;
     switch (what) {
         case 0:  // partial shadow
-            if (c.mode == MODE_FAST) k_crater_shadow<MODE_FAST><<<grid_fs, 128, 0, st>>>(c);
-            else k_crater_shadow<MODE_REF><<<grid_fs, 128, 0, st>>>(c);
+        {
+            // one wave, as every block sets its sub-points up
+            int dev = 0, sms = 0, per = 0;
+            const void* k = c.mode == MODE_FAST ? (const void*)k_crater_shadow<MODE_FAST> : (const void*)k_crater_shadow<MODE_REF>;
+            if (cudaGetDevice(&dev) != cudaSuccess ||
+                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, 128, 0) != cudaSuccess)
+                return 2;
+            if (c.mode == MODE_FAST) k_crater_shadow<MODE_FAST><<<sms * per, 128, 0, st>>>(c);
+            else k_crater_shadow<MODE_REF><<<sms * per, 128, 0, st>>>(c);
             break;
+        }
         case 1: {  // scattering: fargs = {solar, acc, multiple}
-            const size_t sm = smv + 2 * c.nsf * 4;
+            const size_t sm = smv + (size_t)kScatSteps * c.nsf * 4;
             cudaFuncSetAttribute(k_crater_scatter<MODE_REF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             cudaFuncSetAttribute(k_crater_scatter<MODE_FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
             if (c.mode == MODE_FAST)
