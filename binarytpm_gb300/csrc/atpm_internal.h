@@ -278,7 +278,7 @@ struct Batch {
     const int4* qmap;        // tensor-core work items {solve, row block, step chunk, 0}
     int nq;
     int4* tc_list;           // [nq] this launch's items whose row block has an active facet
-    int* tc_work;            // [2] list length, next ticket (k_prepare)
+    int* tc_work;            // [3] list length, next ticket, parts of an item (k_prepare)
     int tc_nmax;             // largest step chunk in the batch
     int cond_variant;        // FAST conduction register/occupancy variant (1, 2, 3)
     int tc_stages;           // tensor-core pipeline depth (0: deepest that fits)

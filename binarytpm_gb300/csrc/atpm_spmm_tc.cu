@@ -55,7 +55,7 @@ namespace {
 
 constexpr int TC_M = 128;        // facets per row block (TMEM lanes)
 constexpr int TC_K = 64;         // facets per column block (one 128-byte swizzle row of BF16)
-constexpr int TC_STAGES = 4;   // upper bound; the ring depth follows the stage size
+constexpr int TC_STAGES = 6;   // upper bound; the ring depth follows the stage size
 constexpr long long WAIT_CYCLES = 2000000000LL;
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -166,7 +166,7 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
 }
 
-// ring depth: as many stages (<= 4) as fit in 220 KB of shared memory;
+// ring depth: as many stages (<= 6) as fit in 220 KB of shared memory;
 // a stage holds A_hi, A_lo (16 KB each) and B_hi, B_lo (N x 128 B each)
 __host__ __device__ inline int tc_stages(int N) {
     const int stage = (TC_M * TC_K * 4 + N * TC_K * 4 + 1023) & ~1023;
@@ -363,7 +363,9 @@ int launch_rem_fill(const DevSolve& s, int nkb, const int* slot, const int* rptr
 //   warps 2-5        epilogue: TMEM quadrant (warp & 3) -> Q, then arrive on
 //                    tempty[buffer]; the issuer's next-but-one item waits on it
 // Every item's products accumulate in the single-item order, so Q does not
-// depend on which CTA computed it.
+// depend on which CTA computed it.  A launch of few items deals each of them out
+// by steps (k_prepare): its tiles' copies and its sums' way out are then shared by
+// several SMs.
 constexpr int TC_THREADS = 192;
 constexpr int TC_QUEUE = 4;  // queued work items
 // Tiles accumulated in TMEM before the partial sum goes to Q: the tensor
@@ -374,6 +376,13 @@ constexpr int TC_QUEUE = 4;  // queued work items
 // and the epilogue adds the segments into Q in order with round-to-nearest.
 constexpr int TC_SEG = 64;
 
+// a queued item's segment and, of its chunk's groups of 16 steps, the first and
+// how many
+__device__ __forceinline__ int tc_part(int seg, int first, int groups) { return seg | first << 20 | groups << 25; }
+__device__ __forceinline__ int part_seg(int p) { return p & 0xfffff; }
+__device__ __forceinline__ int part_first(int p) { return p >> 20 & 31; }
+__device__ __forceinline__ int part_groups(int p) { return p >> 25 & 31; }
+
 __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
     extern __shared__ __align__(1024) unsigned char dyn[];
     __shared__ __align__(8) uint64_t full[TC_STAGES], empty[TC_STAGES], tfull[2], tempty[2], fin;
@@ -381,11 +390,14 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
     __shared__ int4 qitem[TC_QUEUE];
     __shared__ uint32_t tmem_base;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // one stage layout for the launch, sized for the largest chunk of the batch
-    const int Nmax = b.tc_nmax;
+    // one stage layout for the launch, sized for the largest part of a chunk:
+    // smaller parts leave room for more stages
+    const int nsub = b.tc_work[2];
+    const int Nmax = (b.tc_nmax / 16 + nsub - 1) / nsub * 16;
     const uint32_t a_bytes = TC_M * TC_K * 2;
     const uint32_t stage_bytes = (2 * a_bytes + (uint32_t)Nmax * TC_K * 2 * 2 + 1023) & ~1023u;
-    int S = (b.tc_stages > 0 && b.tc_stages < tc_stages(Nmax)) ? b.tc_stages : tc_stages(Nmax);
+    int S = tc_stages(Nmax);
+    if (nsub == 1 && b.tc_stages > 0 && b.tc_stages < S) S = b.tc_stages;
     {
         uint32_t dsz;
         asm("mov.u32 %0, %%dynamic_smem_size;" : "=r"(dsz));
@@ -431,21 +443,25 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
         const int nlist = b.tc_work[0];
         for (;;) {
             const int g = atomicAdd(&b.tc_work[1], 1);
-            const bool stop = g >= nlist;
-            const int4 it = stop ? make_int4(-1, 0, 0, 0) : b.tc_list[g];
+            const bool stop = g >= nlist * nsub;
+            const int4 it = stop ? make_int4(-1, 0, 0, 0) : b.tc_list[g / nsub];
+            // this part's groups of 16 steps
+            const int groups = stop ? 1 : b.tab[it.x].tc_n / 16, per = (groups + nsub - 1) / nsub;
+            const int g0 = stop ? 0 : g % nsub * per, gn = min(per, groups - g0);
+            if (gn <= 0) continue;
             const int tall = stop ? 0 : b.tab[it.x].tc_ptr[it.y + 1] - b.tab[it.x].tc_ptr[it.y];
             const int nseg = stop ? 1 : max(1, (tall + TC_SEG - 1) / TC_SEG);
             for (int seg = 0; seg < nseg && ok; ++seg) {
                 // queue the item's segment (or the stop item)
                 if (!mbar_wait(&qempty[qs], qph ^ 1u)) { ok = false; break; }
-                qitem[qs] = make_int4(it.x, it.y, it.z, seg);
+                qitem[qs] = make_int4(it.x, it.y, it.z, tc_part(seg, g0, gn));
                 mbar_arrive(&qfull[qs]);
                 if (++qs == TC_QUEUE) { qs = 0; qph ^= 1u; }
                 if (stop) break;
                 const DevSolve& sv = b.tab[it.x];
                 const int N = sv.tc_n, c = it.z;
                 const int t0 = sv.tc_ptr[it.y] + seg * TC_SEG, T = min(TC_SEG, tall - seg * TC_SEG);
-                const uint32_t b_bytes = (uint32_t)N * TC_K * 2 * 2;
+                const uint32_t w_bytes = (uint32_t)gn * 16 * TC_K * 2;  // of W_hi, and of W_lo
                 const __nv_bfloat16* tiles = static_cast<const __nv_bfloat16*>(sv.tc_tiles);
                 const __nv_bfloat16* lo_tiles = static_cast<const __nv_bfloat16*>(sv.tc_lo_tiles);
                 const __nv_bfloat16* Wb = static_cast<const __nv_bfloat16*>(sv.Wb);
@@ -454,11 +470,16 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
                     unsigned char* sa = base + (size_t)slot * stage_bytes;
                     const int kb = sv.tc_col[t0 + i] & 0xffffff;
                     const int lo = sv.tc_lo[t0 + i];
-                    mbar_expect_tx(&full[slot], a_bytes + (lo >= 0 ? a_bytes : 0u) + b_bytes);
+                    mbar_expect_tx(&full[slot], a_bytes + (lo >= 0 ? a_bytes : 0u) + 2 * w_bytes);
                     bulk_g2s(sa, tiles + (size_t)(t0 + i) * (TC_M * TC_K), a_bytes, &full[slot]);
                     if (lo >= 0) bulk_g2s(sa + a_bytes, lo_tiles + (size_t)lo * (TC_M * TC_K), a_bytes, &full[slot]);
-                    bulk_g2s(sa + 2 * a_bytes, Wb + ((size_t)kb * sv.tc_nchunks + c) * (size_t)2 * N * TC_K, b_bytes,
-                             &full[slot]);
+                    const __nv_bfloat16* w = Wb + ((size_t)kb * sv.tc_nchunks + c) * (size_t)2 * N * TC_K + g0 * 16 * TC_K;
+                    if (gn * 16 == N) {
+                        bulk_g2s(sa + 2 * a_bytes, w, 2 * w_bytes, &full[slot]);
+                    } else {
+                        bulk_g2s(sa + 2 * a_bytes, w, w_bytes, &full[slot]);
+                        bulk_g2s(sa + 2 * a_bytes + w_bytes, w + (size_t)N * TC_K, w_bytes, &full[slot]);
+                    }
                     last_ph[slot] = (int)ph;
                     if (++slot == (uint32_t)S) { slot = 0; ph ^= 1u; }
                 }
@@ -479,10 +500,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
             const int4 w = qitem[qs];
             if (w.x < 0) break;
             const DevSolve& sv = b.tab[w.x];
-            const int N = sv.tc_n;
+            const int N = part_groups(w.w) * 16, seg = part_seg(w.w);
             const int tall = sv.tc_ptr[w.y + 1] - sv.tc_ptr[w.y];
-            const int t0 = sv.tc_ptr[w.y] + w.w * TC_SEG, T = max(0, min(TC_SEG, tall - w.w * TC_SEG));
-            const uint32_t b_bytes = (uint32_t)N * TC_K * 2 * 2;
+            const int t0 = sv.tc_ptr[w.y] + seg * TC_SEG, T = max(0, min(TC_SEG, tall - seg * TC_SEG));
+            const uint32_t w_bytes = (uint32_t)N * TC_K * 2;
             const uint32_t ab = item_no & 1u, use_no = item_no >> 1;
             if (!mbar_wait(&tempty[ab], (use_no & 1u) ^ 1u)) { ok = false; break; }
             tc_fence_after();
@@ -494,7 +515,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
                 tc_fence_after();
                 const uint32_t sa = smem_u32(base + (size_t)slot * stage_bytes);
                 const uint64_t ad = sw128_desc(sa), al = sw128_desc(sa + a_bytes);
-                const uint64_t bh = sw128_desc(sa + 2 * a_bytes), bl = sw128_desc(sa + 2 * a_bytes + b_bytes / 2);
+                const uint64_t bh = sw128_desc(sa + 2 * a_bytes), bl = sw128_desc(sa + 2 * a_bytes + w_bytes);
                 const bool has_lo = sv.tc_lo[t0 + i] >= 0;
                 // K slices without an entry are zero in both A tiles: their
                 // products would add exact zeros, so they are not issued
@@ -531,7 +552,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
             const int4 w = qitem[qs];
             if (w.x < 0) break;
             const DevSolve& sv = b.tab[w.x];
-            const int N = sv.tc_n, nf = sv.nf, ntau = sv.ntau, nc = w.z;
+            const int N = part_groups(w.w) * 16, seg = part_seg(w.w), nf = sv.nf, ntau = sv.ntau;
+            const int sw = w.z * sv.tc_n + part_first(w.w) * 16;  // the part's first step
             const int T = sv.tc_ptr[w.y + 1] - sv.tc_ptr[w.y];
             float* Q = static_cast<float*>(sv.Q);
             const uint32_t ab = item_no & 1u, use_no = item_no >> 1;
@@ -543,13 +565,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
             const int f = w.y * TC_M + q * 32 + lane;
             // the last segment adds the remainder's sums of the rows that
             // have entries in it (k_spmm_rem)
-            const bool rem = f < nf && sv.rem_ptr && (w.w + 1) * TC_SEG >= T &&
+            const bool rem = f < nf && sv.rem_ptr && (seg + 1) * TC_SEG >= T &&
                              __ldg(&sv.rem_ptr[f]) != __ldg(&sv.rem_ptr[f + 1]);
             const float* R = static_cast<const float*>(sv.W) + (size_t)(f < nf ? f : 0) * gather_ld(ntau);
             if (T == 0) {  // no tile in this row block
                 if (f < nf)
                     for (int n = 0; n < N; ++n) {
-                        const int s = nc * N + n;
+                        const int s = sw + n;
                         if (s < ntau) Q[(size_t)s * nf + f] = rem ? R[s] : 0.0f;
                     }
             } else {
@@ -557,30 +579,35 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_spmm_tc(Batch b) {
                 // (round to nearest); a batch's loads all issue before its
                 // stores
                 const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16) + ab * kBufCols;
-                for (int c0 = 0; c0 < N; c0 += 16) {
+#pragma unroll 1
+                for (int c0 = 0; c0 < N; c0 += 16) {  // N is a multiple of 16
                     float v[16];
                     tc_ld16(tbase + (uint32_t)c0, v);
+                    const int s0 = sw + c0;
                     if (f < nf) {
-                        float prev[16];
+                        float* d = Q + (size_t)s0 * nf + f;
                         float4 more[4];
+                        if (rem) {
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const int s = nc * N + c0 + 4 * j;  // a multiple of 4: N is one of 16
-                            if (rem && s < ntau) more[j] = __ldg(reinterpret_cast<const float4*>(R + s));
+                            for (int j = 0; j < 4; ++j)
+                                if (s0 + 4 * j < ntau) more[j] = __ldg(reinterpret_cast<const float4*>(R + s0) + j);
+                        }
+                        if (seg > 0) {
+                            float prev[16];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) prev[j] = s0 + j < ntau ? __ldcg(d + (size_t)j * nf) : 0.0f;
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) v[j] = prev[j] + v[j];
+                        }
+                        if (rem) {
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) v[j] += reinterpret_cast<const float*>(more)[j];
                         }
 #pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int s = nc * N + c0 + j;
-                            prev[j] = (w.w > 0 && c0 + j < N && s < ntau) ? __ldcg(&Q[(size_t)s * nf + f]) : 0.0f;
-                        }
-#pragma unroll
-                        for (int j = 0; j < 16; ++j) {
-                            const int s = nc * N + c0 + j;
-                            float x = w.w == 0 ? v[j] : prev[j] + v[j];
-                            if (rem) x += reinterpret_cast<const float*>(more)[j];
-                            if (c0 + j < N && s < ntau) Q[(size_t)s * nf + f] = x;
-                        }
+                        for (int j = 0; j < 16; ++j)
+                            if (s0 + j < ntau) d[(size_t)j * nf] = v[j];
                     }
+                    __syncwarp();  // the next tensor-memory load is the whole warp's
                 }
             }
             tc_fence_before();
@@ -740,7 +767,8 @@ int launch_spmm_tc(const Batch& b, stream_t stv) {
             return 2;
         attr_set.fetch_or(bit, std::memory_order_release);
     }
-    const int grid = b.nq < b.sms ? b.nq : b.sms;  // one persistent CTA per SM
+    const int parts = b.nq * (b.tc_nmax / 16);
+    const int grid = parts < b.sms ? parts : b.sms;  // one persistent CTA per SM
     // The remainder first: the product's epilogue adds its sums.  (Side by side
     // on two streams the two hardly overlapped, the product's shared memory
     // leaving no room, and the sums needed a pass over Q of their own.)

@@ -460,40 +460,41 @@ __device__ __forceinline__ void tail_mode(const Batch& b) {
 // each and a memset of the counters cost a few us apiece in revolutions of
 // some 140 (single solves, late revolutions): with the end of the revolution in
 // k_converge, 1,280 facets 140.5 -> 137.5 us.
-constexpr int kPrepItems = 8;  // items a thread looks at in one pass
+// A small block, which starts beside the other group's kernels: one of 1,024
+// threads waited for a whole SM and held the sweep of eight inertias up 6 %.
+constexpr int kPrepThreads = 256, kPrepWarps = kPrepThreads / 32;
+constexpr int kPrepItems = 16;  // items a thread looks at in one pass
 
-__global__ void __launch_bounds__(1024) k_prepare(Batch b) {
-    __shared__ int at[kPrepItems * 32];
+__global__ void __launch_bounds__(kPrepThreads) k_prepare(Batch b) {
+    constexpr int PER = kPrepItems * kPrepWarps / 32;
+    __shared__ int at[kPrepItems * kPrepWarps];
     __shared__ int count;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (warp == 31) tail_mode(b);
+    if (warp == kPrepWarps - 1) tail_mode(b);
     if (b.nq == 0) return;
     int base = 0;
-    for (int i0 = 0; i0 < b.nq; i0 += 1024 * kPrepItems) {
-        int4 it[kPrepItems];
-        unsigned m[kPrepItems];
-#pragma unroll
+    for (int i0 = 0; i0 < b.nq; i0 += kPrepThreads * kPrepItems) {
+        unsigned mine = 0;  // the items of this thread that are in
+#pragma unroll 8
         for (int k = 0; k < kPrepItems; ++k) {
-            const int i = i0 + k * 1024 + threadIdx.x;
-            if (i < b.nq) it[k] = b.qmap[i];
-        }
-#pragma unroll
-        for (int k = 0; k < kPrepItems; ++k) {
+            const int i = i0 + k * kPrepThreads + threadIdx.x;
             bool use = false;
-            if (i0 + k * 1024 + threadIdx.x < b.nq) {
-                const DevSolve& sv = b.tab[it[k].x];
+            if (i < b.nq) {
+                const int4 it = b.qmap[i];
+                const DevSolve& sv = b.tab[it.x];
                 const bool everyone = !sv.freeze || sv.ti == 0.0f;
-                use = sv.ctl->active && sv.tc_tiles && (everyone || sv.rb_act[it[k].y]);
+                use = sv.ctl->active && sv.tc_tiles && (everyone || sv.rb_act[it.y]);
             }
-            m[k] = __ballot_sync(0xffffffffu, use);
-            if (lane == 0) at[k * 32 + warp] = __popc(m[k]);
+            const unsigned m = __ballot_sync(0xffffffffu, use);
+            if (lane == 0) at[k * kPrepWarps + warp] = __popc(m);
+            mine |= use ? 1u << k : 0u;
         }
         __syncthreads();
-        if (warp == 0) {  // exclusive sums of the counts, kPrepItems consecutive ones a lane
-            int c[kPrepItems], sum = 0;
+        if (warp == 0) {  // exclusive sums of the counts, PER consecutive ones a lane
+            int c[PER], sum = 0;
 #pragma unroll
-            for (int k = 0; k < kPrepItems; ++k) {
-                c[k] = at[lane * kPrepItems + k];
+            for (int k = 0; k < PER; ++k) {
+                c[k] = at[lane * PER + k];
                 sum += c[k];
             }
             int x = sum;
@@ -504,21 +505,31 @@ __global__ void __launch_bounds__(1024) k_prepare(Batch b) {
             if (lane == 31) count = x;
             x += base - sum;
 #pragma unroll
-            for (int k = 0; k < kPrepItems; ++k) {
-                at[lane * kPrepItems + k] = x;
+            for (int k = 0; k < PER; ++k) {
+                at[lane * PER + k] = x;
                 x += c[k];
             }
         }
         __syncthreads();
-#pragma unroll
-        for (int k = 0; k < kPrepItems; ++k)
-            if ((m[k] >> lane) & 1u) b.tc_list[at[k * 32 + warp] + __popc(m[k] & ((1u << lane) - 1u))] = it[k];
+#pragma unroll 8
+        for (int k = 0; k < kPrepItems; ++k) {
+            const bool use = (mine >> k) & 1u;
+            const unsigned m = __ballot_sync(0xffffffffu, use);
+            if (use)
+                b.tc_list[at[k * kPrepWarps + warp] + __popc(m & ((1u << lane) - 1u))] =
+                    b.qmap[i0 + k * kPrepThreads + threadIdx.x];
+        }
         base += count;
         __syncthreads();
     }
     if (threadIdx.x == 0) {
         b.tc_work[0] = base;  // list length
         b.tc_work[1] = 0;     // next ticket
+        // parts an item is dealt out in: as many as the SMs take in one wave
+        // (a second wave reads every V tile again).  us a revolution whole and
+        // dealt out: 90.2 and 80.6 at 320 facets x 300 steps, 132.6 and 130 at
+        // 2,740 x 400, 137.6 and 134.3 at 1,280 x 720; half a wave 80, 132 and 137.5.
+        b.tc_work[2] = max(1, min(b.tc_nmax / 16, base ? b.sms / base : 1));
     }
 }
 
@@ -847,7 +858,7 @@ bool conduction_nx_supported(int nx) {
 
 template <int MODE>
 static int launch_rev_part(const Batch& b, int part, cudaStream_t st) {
-    if (MODE == MODE_FAST && part == 0) k_prepare<<<1, 1024, 0, st>>>(b);
+    if (MODE == MODE_FAST && part == 0) k_prepare<<<1, kPrepThreads, 0, st>>>(b);
     // FAST + tensor cores: the conduction sweep keeps W current (store_w)
     if (MODE == MODE_FAST && b.nq > 0 && part == 0) return cudaGetLastError() == cudaSuccess ? 0 : 2;
     if (MODE == MODE_FAST && b.nq > 0 && part == 1) return launch_spmm_tc(b, st);
