@@ -23,10 +23,12 @@
 // All of it is FP64, on a part whose FP64 rate is 1/64 of FP32, so FP64
 // operations are what it costs.  The positions are the stage's, operand by
 // operand (its body lies 1e11 m away from an origin while its shape keeps its
-// own units, so their rounding shows in the normals); from them on, cosines come
-// from one reciprocal square root instead of a facet frame, acos and cos, and a
-// wavelength costs one exp and one reciprocal: 13.0 -> 4.0 ms for 21,760 facets,
-// 720 steps and three wavelengths.
+// own units, so their rounding shows in the normals and, for an observer near the
+// body, in the view vector); from them on, cosines come from one reciprocal square
+// root instead of a facet frame, acos and cos, and a wavelength costs one exp and
+// one reciprocal: 13.0 -> 4.2 ms for 21,760 facets, 720 steps and three
+// wavelengths.  A cosine within kSure of 0 or 1 is the stage's to judge
+// (stage_view): there its rounding decides whether a facet or sub-facet counts.
 //
 // The rough-surface sum (observe, wise_main.cpp:695-727) replaces each
 // facet's own term by its crater's: the sub-facets with a visible fraction
@@ -113,6 +115,45 @@ __global__ void __launch_bounds__(256) k_flux_flags(const int32_t* src, uint8_t*
     }
 }
 
+// what the cosines here and the stage's may differ by (each a few operations of
+// 2^-53 on terms of at most 1), with room to spare
+constexpr double kSure = 1e-14;
+
+__device__ __forceinline__ int exponent(double x) { return __double2hiint(x) >> 20 & 0x7ff; }
+
+// x / 3 correctly rounded: the product with the rounded 1/3, corrected by its exact
+// residual (P. Markstein, IBM J. Res. Dev. 34, 1990), on a part where a division
+// takes some ten FP64 operations
+__device__ __forceinline__ double third(double x) {
+    const double q = __dmul_rn(x, 1.0 / 3.0);
+    return __fma_rn(__fma_rn(-3.0, q, x), 1.0 / 3.0, q);
+}
+
+// the stage's own view of a facet in its operand order (wise_main.cpp:555-645):
+// the view vector in the facet's frame (rows x^, y, n) and its length; returns the
+// angle to the normal, NaN where the cosine rounds above 1
+__device__ __noinline__ double stage_view(const DevSolve& s, const FluxArgs& a, int f, int step, double (&v)[3],
+                                          double& d) {
+    const Facet t(s, a, f, step);
+    const double nn = __dsqrt_rn(dot3(t.n, t.n)), xx = __dsqrt_rn(dot3(t.edge, t.edge));
+    double n[3], x[3], ov[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        n[k] = __ddiv_rn(t.n[k], nn);
+        x[k] = __ddiv_rn(t.edge[k], xx);
+        ov[k] = __dsub_rn(__ddiv_rn(t.sum[k], 3.0), a.obs[k]);
+    }
+    const double y[3] = {__dsub_rn(__dmul_rn(n[1], x[2]), __dmul_rn(n[2], x[1])),
+                         __dsub_rn(__dmul_rn(n[2], x[0]), __dmul_rn(n[0], x[2])),
+                         __dsub_rn(__dmul_rn(n[0], x[1]), __dmul_rn(n[1], x[0]))};
+    v[0] = -dot3(x, ov);
+    v[1] = -dot3(y, ov);
+    v[2] = -dot3(n, ov);
+    d = __dsqrt_rn(dot3(v, v));
+    return acos(__ddiv_rn(v[2], __dsqrt_rn(dot3(ov, ov))));
+}
+constexpr double kRight = 3.141592653589793 / 2.0;
+
 // (2hc^2 / lambda^5) * (1 / (exp(hc / (lambda k T)) - 1)), 0 where that is NaN
 __device__ __forceinline__ double planck(const FluxArgs& a, int l, double inv_t) {
     const double b = a.b1[l] / (exp(a.hl[l] * inv_t) - 1.0);
@@ -135,12 +176,21 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux_partial(DevSolve s, FluxA
         const Facet t(s, a, f, step);
         double ov[3];  // from the facet to the observer
 #pragma unroll
-        for (int k = 0; k < 3; ++k) ov[k] = a.obs[k] - t.sum[k] * (1.0 / 3.0);
+        for (int k = 0; k < 3; ++k) ov[k] = __dsub_rn(a.obs[k], third(t.sum[k]));
         const double oo = dot3(ov, ov), nn = dot3(t.n, t.n), no = dot3(t.n, ov);
-        // cosine toward the observer; above 1 the stage's acos is NaN and the
-        // facet contributes nothing
-        const double c = no > 0.0 ? no * rsqrt(nn * oo) : -1.0;
-        if (c > 0.0 && c <= 1.0) {
+        // cosine toward the observer; |cosine| < kSure by the exponents
+        const bool edge_on = 2 * exponent(no) < exponent(nn) + exponent(oo) - 88;
+        double c = no > 0.0 ? no * rsqrt(nn * oo) : -1.0;
+        bool seen = c > 0.0;
+        if (edge_on || (__double2hiint(c) >= 0x3fefffff && c > 1.0 - kSure)) {
+            double v[3], d;
+            const double angle = stage_view(s, a, f, step, v, d);
+            // NaN passes the stage's horizon test; its own term is then dropped,
+            // a crater's terms have their own angles
+            seen = !(angle > kRight) && (ROUGH || angle == angle);
+            c = cos(angle);
+        }
+        if (seen) {
             weight = a.eps * a.area[f] / oo;
             if constexpr (!ROUGH) {
                 weight *= c;
@@ -176,13 +226,19 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux_partial(DevSolve s, FluxA
         for (int i = 0; i < 32; ++i) {
             const double* v = view[warp * 32 + i];
             if (v[3] == 0.0) continue;
-            const size_t base =
-                ((size_t)(blockIdx.x * kFluxThreads + warp * 32 + i) * s.ntau + step) * (size_t)a.nsf;
+            const int facet = blockIdx.x * kFluxThreads + warp * 32 + i;
+            const size_t base = ((size_t)facet * s.ntau + step) * (size_t)a.nsf;
             for (int j = lane; j < a.nsf; j += 32) {
                 const double vis = (double)a.sub_vis[base + j];
                 const double* g = a.sub_geo + 4 * j;
-                const double c = v[0] * g[0] + v[1] * g[1] + v[2] * g[2];
-                if (!(vis > 0.0) || !(fabs(c) <= 1.0)) continue;
+                double c = v[0] * g[0] + v[1] * g[1] + v[2] * g[2];
+                if (!(vis > 0.0)) continue;
+                if (fabs(c) > 1.0 - kSure) {  // the stage's acos of a ratio above 1 is NaN: no term
+                    double w[3], d;
+                    stage_view(s, a, facet, step, w, d);
+                    c = __ddiv_rn(dot3(w, g), d);
+                }
+                if (!(fabs(c) <= 1.0)) continue;
                 const double m = v[3] * g[3] * vis * c, inv_t = 1.0 / (double)a.sub_T[base + j];
 #pragma unroll
                 for (int l = 0; l < kMaxFluxWavelengths; ++l)
