@@ -359,9 +359,14 @@ __device__ __forceinline__ float edge_of(float2 a, float2 b, float2 q, float sig
     return e;
 }
 
-// 1: q lies in the triangle, 0: it does not, 2: within the margin of an edge
+// 1: q lies in the triangle, 0: it does not, 2: within the margin of an edge, or
+// the triangle is no wider than the margin: its orientation, on which every edge's
+// side rests, is then a matter of rounding (an edge-on facet ten times as long as
+// its short edge would hide nothing)
 __device__ __forceinline__ int locate(const Tri& t, float2 q, float margin) {
-    const float area = (t.q1.x - t.q0.x) * (t.q2.y - t.q0.y) - (t.q1.y - t.q0.y) * (t.q2.x - t.q0.x);
+    const float ax = t.q1.x - t.q0.x, ay = t.q1.y - t.q0.y, bx = t.q2.x - t.q0.x, by = t.q2.y - t.q0.y;
+    const float area = ax * by - ay * bx;
+    if (fabsf(area) <= margin * (fabsf(ax) + fabsf(ay) + fabsf(bx) + fabsf(by))) return 2;
     const float sign = area < 0.0f ? -1.0f : 1.0f;
     float c0, c1, c2;
     const float e0 = edge_of(t.q0, t.q1, q, sign, margin, c0), e1 = edge_of(t.q1, t.q2, q, sign, margin, c1),
