@@ -65,9 +65,11 @@ struct Proj {
     float scale;      // distance of the body centre
     float pad;        // box padding (km)
     float margin;     // beyond this from a decision FP32 decides (km)
+    float lift;       // most a midpoint's distance exceeds the body's and its depth (km)
     float2* uv;       // [nv][ntau]
     float* w;         // [nv][ntau] depth behind the body centre along c
-    unsigned* stats;  // [0] max |u|,|v| (float bits), [1] max box extent, [2] bad-projection flag, [3] max |w|
+    unsigned* stats;  // [0] max |u|,|v| (float bits), [1] max box extent, [2] bad-projection flag, [3] max |w|,
+                      // [4] max -w
     float4* wbox;     // [windows][nf] union of each facet's padded boxes over 32 steps
 };
 
@@ -105,10 +107,12 @@ __global__ void __launch_bounds__(256) k_geom_vertices(GeomArgs a, Proj p) {
     const float m = 1.0f / (1.0f + w / p.scale), u = x * m, t = y * m;
     p.uv[i] = make_float2(u, t);
     p.w[i] = w;
-    const unsigned lat = warp_max(__float_as_uint(fmaxf(fabsf(u), fabsf(t)))), dep = warp_max(__float_as_uint(fabsf(w)));
+    const unsigned lat = warp_max(__float_as_uint(fmaxf(fabsf(u), fabsf(t)))), dep = warp_max(__float_as_uint(fabsf(w))),
+                   front = warp_max(__float_as_uint(fmaxf(-w, 0.0f)));
     if ((threadIdx.x & 31) == (unsigned)(__ffs(__activemask()) - 1)) {
         if (lat > __ldcg(&p.stats[0])) atomicMax(&p.stats[0], lat);
         if (dep > __ldcg(&p.stats[3])) atomicMax(&p.stats[3], dep);
+        if (front > __ldcg(&p.stats[4])) atomicMax(&p.stats[4], front);
     }
 }
 
@@ -326,20 +330,35 @@ __global__ void __launch_bounds__(256) k_shadow_all(GeomArgs a) {
 }
 
 // ------------------------------------------------------------- culled drivers
-// a projected facet: its corners and its midpoint's depth
+// a projected facet: its corners and their depths
 struct Tri {
     float2 q0, q1, q2;
-    float w;
+    float w0, w1, w2;
+};
+// a facet's midpoint: its projection, and its distance from the origin less the
+// body's
+struct Mid {
+    float2 q;
+    float r;
 };
 
 __device__ __forceinline__ Tri load_tri(const GeomArgs& a, const Proj& p, int f, int s) {
     const int* fv = a.s.fac + 3 * f;
     const size_t i0 = (size_t)fv[0] * a.s.ntau + s, i1 = (size_t)fv[1] * a.s.ntau + s, i2 = (size_t)fv[2] * a.s.ntau + s;
-    return {p.uv[i0], p.uv[i1], p.uv[i2], (p.w[i0] + p.w[i1] + p.w[i2]) * (1.0f / 3.0f)};
+    return {p.uv[i0], p.uv[i1], p.uv[i2], p.w[i0], p.w[i1], p.w[i2]};
 }
 
-__device__ __forceinline__ float2 middle(const Tri& t) {
-    return make_float2((t.q0.x + t.q1.x + t.q2.x) * (1.0f / 3.0f), (t.q0.y + t.q1.y + t.q2.y) * (1.0f / 3.0f));
+// With corners at depths w_i the midpoint projects to the mean of theirs weighted
+// by scale + w_i, and lies (scale + w) sqrt(1 + t) from the origin, t the square of
+// its projection over scale.  Both hold at any distance: plain means and the depth
+// itself leave them by the square of the body's size over the distance, which an
+// observer close by would need a margin of whole facets for.
+__device__ __forceinline__ Mid middle(const Proj& p, const Tri& t) {
+    const float inv = 1.0f / p.scale, p0 = 1.0f + t.w0 * inv, p1 = 1.0f + t.w1 * inv, p2 = 1.0f + t.w2 * inv;
+    const float m = 1.0f / (p0 + p1 + p2), w = (t.w0 + t.w1 + t.w2) * (1.0f / 3.0f);
+    const float x = (t.q0.x * p0 + t.q1.x * p1 + t.q2.x * p2) * m, y = (t.q0.y * p0 + t.q1.y * p1 + t.q2.y * p2) * m;
+    const float u = x * inv, v = y * inv, sq = u * u + v * v;
+    return {make_float2(x, y), w + (p.scale + w) * (sq / (1.0f + sqrtf(1.0f + sq)))};
 }
 
 __device__ __forceinline__ float4 tri_box(const Tri& t, float pad) {
@@ -375,11 +394,11 @@ __device__ __forceinline__ int locate(const Tri& t, float2 q, float margin) {
     return (e0 > c0 && e1 > c1 && e2 > c2) ? 1 : 2;
 }
 
-// whether g, at depth gw behind h at hw, is the one tested against the other:
-// the farther, and on equal distances the higher index where `ties`
-__device__ __forceinline__ bool behind(const GeomArgs& a, const Proj& p, int g, int h, int s, float gw, float hw,
+// whether g, at distance gr from the origin, is the one tested against h at hr: the
+// farther, and on equal distances the higher index where `ties`
+__device__ __forceinline__ bool behind(const GeomArgs& a, const Proj& p, int g, int h, int s, float gr, float hr,
                                        bool ties) {
-    const float d = gw - hw;
+    const float d = gr - hr;
     if (d > p.margin) return true;
     if (d < -p.margin) return false;
     const int o = exact_order(a.g.hp, a.s.fac, a.s.ntau, g, h, s);  // sign of |g| - |h|
@@ -420,8 +439,10 @@ __device__ __forceinline__ void count_tests(unsigned long long* ctr, unsigned n)
 // entries at a time, a lane each, are held against the box around the warp's
 // lit points; the entries left are tested one by one, a lane per step.  Taking
 // every entry in turn was bound by the loop's instructions (7.2 ms
-// for 21,760 facets, 5.8 M entries, 720 steps; 1.2 ms now).
-__global__ void __launch_bounds__(256) k_shadow_dep_cull(GeomArgs a, Proj p) {
+// for 21,760 facets, 5.8 M entries, 720 steps; 1.2 ms now).  Three CTAs an SM
+// rather than the two its free choice of registers leaves: 0.200 against 0.217 ms
+// for 5,840 facets and 360 steps.
+__global__ void __launch_bounds__(256, 3) k_shadow_dep_cull(GeomArgs a, Proj p) {
     const int nf = a.s.nf, ntau = a.s.ntau;
     const int g = blockIdx.y * blockDim.y + threadIdx.y;
     const int lane = threadIdx.x, s = blockIdx.x * 32 + lane;
@@ -432,8 +453,8 @@ __global__ void __launch_bounds__(256) k_shadow_dep_cull(GeomArgs a, Proj p) {
     const int sc = valid ? s : ntau - 1;
     const size_t o = (size_t)g * ntau + sc;
     bool lit = valid && a.s.shadow[o] == 1;
-    const Tri tg = load_tri(a, p, g, sc);
-    const float2 q = middle(tg);
+    const Mid mg = middle(p, load_tri(a, p, g, sc));
+    const float2 q = mg.q;
     unsigned ntest = 0;
     // the box around this warp's lit points (empty when none is lit)
     float4 qb = lit ? make_float4(q.x, q.x, q.y, q.y) : make_float4(INFINITY, -INFINITY, INFINITY, -INFINITY);
@@ -454,7 +475,10 @@ __global__ void __launch_bounds__(256) k_shadow_dep_cull(GeomArgs a, Proj p) {
             const int h = __shfl_sync(0xffffffffu, mine, __ffs(left) - 1);
             if (!lit) continue;
             const Tri th = load_tri(a, p, h, s);
-            if (!in_box(q, tri_box(th, p.pad)) || !behind(a, p, g, h, s, tg.w, th.w, false)) continue;
+            if (!in_box(q, tri_box(th, p.pad))) continue;
+            // h's distance is its mean depth and up to `lift`: the depth settles most
+            const float d = mg.r - (th.w0 + th.w1 + th.w2) * (1.0f / 3.0f);
+            if (d < -p.margin || (d <= p.margin + p.lift && !behind(a, p, g, h, s, mg.r, middle(p, th).r, false))) continue;
             ++ntest;
             int hit = locate(th, q, p.margin);
             if (hit == 2) hit = exact_test(a.g.hp, a.s.fac, ntau, g, h, s) == 0;
@@ -472,7 +496,8 @@ struct GridArgs {
     int s0, ns;     // steps of this chunk
     int* start;     // [ns][G*G + 1] first entry of each cell
     int* cursor;    // [ns][G*G]
-    float4* tri;    // [ns][nf][2] corners, midpoint depth, lit flag
+    float4* tri;    // [ns][nf][2] corners, midpoint distance, lit flag
+    float2* mid;    // [ns][nf] midpoints
     int* who;       // [ns][kCover nf] facets by cell
 };
 constexpr int kCover = 9;  // a box of at most two cells' size touches at most 3 x 3 cells
@@ -561,9 +586,11 @@ __global__ void __launch_bounds__(256) k_grid_fill(GeomArgs a, Proj p, GridArgs 
     if (i >= (long long)nf * gr.ns) return;
     const int f = (int)(i / gr.ns), k = (int)(i % gr.ns), s = gr.s0 + k;
     const Tri t = load_tri(a, p, f, s);
+    const Mid m = middle(p, t);
     float4* d = gr.tri + 2 * ((size_t)k * nf + f);
     d[0] = make_float4(t.q0.x, t.q0.y, t.q1.x, t.q1.y);
-    d[1] = make_float4(t.q2.x, t.q2.y, t.w, a.s.shadow[(size_t)f * ntau + s] == 1 ? 1.0f : 0.0f);
+    d[1] = make_float4(t.q2.x, t.q2.y, m.r, a.s.shadow[(size_t)f * ntau + s] == 1 ? 1.0f : 0.0f);
+    gr.mid[(size_t)k * nf + f] = m.q;
     const float4 b = tri_box(t, p.pad);
     int* cu = gr.cursor + (size_t)k * gr.G * gr.G;
     const size_t first = (size_t)k * kCover * nf;
@@ -572,10 +599,11 @@ __global__ void __launch_bounds__(256) k_grid_fill(GeomArgs a, Proj p, GridArgs 
     });
 }
 
-__device__ __forceinline__ Tri stored_tri(const float4* t, float* lit) {
+// corners (no depths) and the midpoint's distance
+__device__ __forceinline__ Tri stored_tri(const float4* t, float* r) {
     const float4 x = __ldg(t), y = __ldg(t + 1);
-    *lit = y.w;
-    return {make_float2(x.x, x.y), make_float2(x.z, x.w), make_float2(y.x, y.y), y.z};
+    *r = y.z;
+    return {make_float2(x.x, x.y), make_float2(x.z, x.w), make_float2(y.x, y.y)};
 }
 
 // all pairs over the grid: a facet's box is filed in every cell it touches, so
@@ -592,10 +620,9 @@ __global__ void __launch_bounds__(256, 4) k_shadow_grid(GeomArgs a, Proj p, Grid
     if (i >= (long long)nf * gr.ns) return;
     const int k = (int)(i / nf), g = (int)(i % nf), s = gr.s0 + k;
     const float4* tri = gr.tri + 2 * (size_t)k * nf;
-    float lit;
-    const Tri tg = stored_tri(tri + 2 * (size_t)g, &lit);
-    if (lit == 0.0f) return;  // dark already
-    const float2 q = middle(tg);
+    const float4 own = __ldg(tri + 2 * (size_t)g + 1);
+    if (own.w == 0.0f) return;  // dark already
+    const float2 q = __ldg(gr.mid + (size_t)k * nf + g);
     const int* st = gr.start + (size_t)k * (gr.G * gr.G + 1) + cell_of(gr, q.y) * gr.G + cell_of(gr, q.x);
     const size_t first = (size_t)k * kCover * nf;
     const int* who = gr.who + first;
@@ -605,9 +632,9 @@ __global__ void __launch_bounds__(256, 4) k_shadow_grid(GeomArgs a, Proj p, Grid
     for (int j = st[0]; j < end; ++j) {
         const int h = next;
         if (j + 1 < end) next = __ldg(who + j + 1);
-        float unused;
-        const Tri th = stored_tri(tri + 2 * (size_t)h, &unused);
-        if (!in_box(q, tri_box(th, p.pad)) || h == g || !behind(a, p, g, h, s, tg.w, th.w, true)) continue;
+        float hr;
+        const Tri th = stored_tri(tri + 2 * (size_t)h, &hr);
+        if (!in_box(q, tri_box(th, p.pad)) || h == g || !behind(a, p, g, h, s, own.z, hr, true)) continue;
         ++ntest;
         int hit = locate(th, q, p.margin);
         if (hit == 2) hit = exact_test(a.g.hp, a.s.fac, ntau, g, h, s) == 0;
@@ -663,24 +690,26 @@ int launch_shadow_culled(const DevSolve& s, const GeomWork& g, bool all_pairs, s
     Proj p{};
     if (!make_frame(g, p)) return -1;
     const long long nft = (long long)s.nf * s.ntau;
-    unsigned stats[4] = {0, 0, 0, 0};
+    unsigned stats[5] = {};
     auto read_stats = [&]() {
-        return cudaMemcpyAsync(stats, p.stats, 16, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
+        return cudaMemcpyAsync(stats, p.stats, sizeof stats, cudaMemcpyDeviceToHost, st) == cudaSuccess &&
                cudaStreamSynchronize(st) == cudaSuccess;
     };
     if (!read_stats()) return 2;
     if (stats[2]) return -1;  // a vertex too far off the body direction: no projection
-    float umax, wmax;
+    float umax, wmax, front;
     memcpy(&umax, &stats[0], 4);
     memcpy(&wmax, &stats[3], 4);
-    // What FP32 may not decide (km): some 16 ulps of the largest coordinate, a
-    // good part of a metre per 1e11 km for the FP64 test's own rounding (1.5 mm
-    // at 1 AU, where its positions have ulps of 0.03 mm), and the perspective's
-    // second order over the body, by which a midpoint's projection and order
-    // leave the mean of its corners'.  The boxes are padded by a centimetre
-    // besides.
-    const float size = umax > wmax ? umax : wmax, bend = 4.0f * size * size / p.scale;
-    p.margin = 2e-6f * size + 1e-14f * p.scale + bend;
+    memcpy(&front, &stats[4], 4);
+    // What FP32 may not decide (km): some 16 ulps of the largest coordinate, as the
+    // perspective enlarges them (scale over the nearest vertex's depth, and the
+    // body's size over its distance, 1 for all but the closest observers), and a
+    // good part of a metre per 1e11 km for the FP64 test's own rounding (1.5 mm at
+    // 1 AU, where its positions have ulps of 0.03 mm).  The boxes are padded by a
+    // centimetre besides.
+    const float size = umax > wmax ? umax : wmax, wide = 1.0f + size / p.scale;
+    p.margin = std::min(size, 2e-6f * size * wide * wide / (1.0f - front / p.scale)) + 1e-14f * p.scale;
+    p.lift = size * wide * (size / p.scale);
     p.pad = 1e-5f + p.margin;
     int rc = 0;
     if (!all_pairs) {
@@ -711,14 +740,16 @@ int launch_shadow_culled(const DevSolve& s, const GeomWork& g, bool all_pairs, s
         const int sc = (int)std::max<size_t>(
             1, std::min<size_t>((size_t)s.ntau, std::min<size_t>((64u << 20) / (n + 1), (1u << 30) / (entries * 4))));
         const size_t b_st = al256((size_t)sc * (n + 1) * 4), b_cu = al256((size_t)sc * n * 4),
-                     b_tri = al256((size_t)sc * s.nf * 2 * sizeof(float4)), b_who = al256(sc * entries * 4);
+                     b_tri = al256((size_t)sc * s.nf * 2 * sizeof(float4)), b_who = al256(sc * entries * 4),
+                     b_mid = al256((size_t)sc * s.nf * sizeof(float2));
         void* gm = nullptr;
-        if (cudaMallocAsync(&gm, b_st + b_cu + b_tri + b_who, st) != cudaSuccess) return 2;
+        if (cudaMallocAsync(&gm, b_st + b_cu + b_tri + b_who + b_mid, st) != cudaSuccess) return 2;
         char* t = static_cast<char*>(gm);
         gr.start = reinterpret_cast<int*>(t);
         gr.cursor = reinterpret_cast<int*>(t + b_st);
         gr.tri = reinterpret_cast<float4*>(t + b_st + b_cu);
         gr.who = reinterpret_cast<int*>(t + b_st + b_cu + b_tri);
+        gr.mid = reinterpret_cast<float2*>(t + b_st + b_cu + b_tri + b_who);
         for (int s0 = 0; s0 < s.ntau && !rc; s0 += sc) {
             gr.s0 = s0;
             gr.ns = std::min(sc, s.ntau - s0);
@@ -797,7 +828,7 @@ int launch_geometry(const DevSolve& s, const GeomWork& g, stream_t stv) {
     const long long nvt = (long long)s.nv * s.ntau, nft = (long long)s.nf * s.ntau;
     Proj p{};
     if (!make_frame(g, p)) p.uv = nullptr;
-    if (p.uv && cudaMemsetAsync(p.stats, 0, 16, st) != cudaSuccess) return 2;
+    if (p.uv && cudaMemsetAsync(p.stats, 0, 5 * sizeof(unsigned), st) != cudaSuccess) return 2;
     k_geom_vertices<<<(unsigned)((nvt + 255) / 256), 256, 0, st>>>(a, p);
     if (s.mode == MODE_FP64) k_geom_facets<MODE_FP64><<<(unsigned)((nft + 255) / 256), 256, 0, st>>>(a);
     else if (s.mode == MODE_FAST) k_geom_facets<MODE_FAST><<<(unsigned)((nft + 255) / 256), 256, 0, st>>>(a);

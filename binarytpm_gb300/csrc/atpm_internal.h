@@ -226,7 +226,7 @@ struct GeomWork {
     // the culled drivers' projection (null: not wanted)
     void* uv;        // [nv][ntau] float2
     float* depth;    // [nv][ntau]
-    unsigned* stats; // [4]
+    unsigned* stats; // [5]
     // the plain drivers' arrays (null until launch_geometry_arrays is wanted)
     double* hm;      // [nf][ntau][3] heliocentric facet midpoints
     double* nrm;     // [nf][ntau][3] unit normals
