@@ -586,6 +586,9 @@ int crater_launch(int what, const CraterDev& c, const PowTab& p4, const PowTab& 
                   void* p1, stream_t stv) {
     cudaStream_t st = static_cast<cudaStream_t>(stv);
     const size_t smv = (size_t)c.nsf * c.nsf * 4;
+    // dynamic shared memory of the largest crater (128 sub-facets): the limit belongs
+    // to a function, not to a launch, so every thread sets the same one
+    constexpr int kSharedLimit = (128 * 128 + kScatSteps * 128) * 4;
     const int grid_fs = 152 * 8;
     switch (what) {
         case 0:  // partial shadow
@@ -603,8 +606,8 @@ int crater_launch(int what, const CraterDev& c, const PowTab& p4, const PowTab& 
         }
         case 1: {  // scattering: fargs = {solar, acc, multiple}
             const size_t sm = smv + (size_t)kScatSteps * c.nsf * 4;
-            cudaFuncSetAttribute(k_crater_scatter<MODE_REF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            cudaFuncSetAttribute(k_crater_scatter<MODE_FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            cudaFuncSetAttribute(k_crater_scatter<MODE_REF>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit);
+            cudaFuncSetAttribute(k_crater_scatter<MODE_FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit);
             if (c.mode == MODE_FAST)
                 k_crater_scatter<MODE_FAST><<<grid_fs, 128, sm, st>>>(c, fargs[0], fargs[1], (int)fargs[2], 10000);
             else
@@ -623,8 +626,8 @@ int crater_launch(int what, const CraterDev& c, const PowTab& p4, const PowTab& 
 #undef NX_CASE
         case 3: {  // equilibrium: fargs = {es}
             const size_t sm = smv + c.nsf * 4;
-            cudaFuncSetAttribute(k_crater_equilibrium<MODE_REF>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-            cudaFuncSetAttribute(k_crater_equilibrium<MODE_FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+            cudaFuncSetAttribute(k_crater_equilibrium<MODE_REF>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit);
+            cudaFuncSetAttribute(k_crater_equilibrium<MODE_FAST>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSharedLimit);
             if (c.mode == MODE_FAST) k_crater_equilibrium<MODE_FAST><<<c.nf, 128, sm, st>>>(c, p4, pq, fargs[0]);
             else k_crater_equilibrium<MODE_REF><<<c.nf, 128, sm, st>>>(c, p4, pq, fargs[0]);
             break;

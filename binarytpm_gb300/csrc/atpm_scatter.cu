@@ -476,8 +476,10 @@ namespace {
 template <int MODE, int STEPS>
 int launch_levels(const DevSolve& s, const GsPlan& plan, void* work, cudaStream_t st, int cap) {
     const size_t smem = (size_t)s.nf * STEPS * sizeof(typename Sa<MODE>::R);
-    if (cudaFuncSetAttribute(k_multi_levels<MODE, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-        cudaSuccess)
+    // the limit belongs to the function, not to the launch: every thread sets the
+    // same one, or a small shape's would refuse a large one's launch
+    if (cudaFuncSetAttribute(k_multi_levels<MODE, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kGsSharedBytes) != cudaSuccess)
         return 2;
     k_multi_levels<MODE, STEPS><<<(s.ntau + STEPS - 1) / STEPS, 1024, smem, st>>>(s, plan, work, cap);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;

@@ -260,7 +260,7 @@ int launch_tc_rowneed(const DevSolve& s, int nkb, unsigned* need, stream_t stv) 
     int warps = (int)std::min<size_t>(8, kMax / per_warp);
     const size_t smem = per_warp * warps;
     if (smem > 48 * 1024 &&
-        cudaFuncSetAttribute(k_tc_rowneed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+        cudaFuncSetAttribute(k_tc_rowneed, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax) != cudaSuccess)
         return 2;
     k_tc_rowneed<<<(unsigned)((s.nf + warps - 1) / warps), warps * 32, smem, st>>>(s, nkb, need);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
