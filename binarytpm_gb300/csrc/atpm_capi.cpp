@@ -1598,7 +1598,7 @@ LoopOut revolution_loop(atpm_solve* const* solves, int n, const Batch& b, cudaGr
     }
     cudaError_t e = cudaSuccess;
     int chunk = 4;
-    while (e == cudaSuccess && done_revs < maxcap) {
+    for (;;) {  // once at least: the autotuner may have run every revolution
         const int k = std::min(chunk, maxcap - done_revs);
         for (int j = 0; j < k && e == cudaSuccess; ++j) e = cudaGraphLaunch(gx, lead->st);
         o.launches += (int64_t)k * kernels_per_revolution(b);
@@ -1609,8 +1609,9 @@ LoopOut revolution_loop(atpm_solve* const* solves, int n, const Batch& b, cudaGr
         for (int i = 0; i < n && e == cudaSuccess; ++i)
             e = cudaMemcpyAsync(&ctl[i], solves[i]->ds.ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, lead->st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(lead->st);
+        if (e != cudaSuccess) break;
         for (int i = 0; i < n; ++i) any = any || ctl[i].active;
-        if (!any) break;
+        if (!any || done_revs >= maxcap) break;
         chunk = std::min(chunk * 2, 32);
     }
     if (e != cudaSuccess) {
