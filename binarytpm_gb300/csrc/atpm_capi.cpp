@@ -626,16 +626,18 @@ Batch make_batch(atpm_context* ctx, const DevSolve* tab, int n, const int4* wm, 
     b.tail_limit = warp_tail_per_sm() * ctx->sm_count;
     b.few_limit = std::max(b.tail_limit, kFewPerSm * ctx->sm_count);
     b.sms = ctx->sm_count;
+    b.facets = 0;
     b.rem_nmb = 0;
     b.rem_ntau = 0;
     return b;
 }
 
-// the remainder kernel's grid: the largest row-block count and step count of
-// the solves that have a sparse remainder
-void set_remainder_grid(Batch& b, atpm_solve* const* solves, int n) {
+// the batch's facets in all, and the remainder kernel's grid: the largest
+// row-block count and step count of the solves that have a sparse remainder
+void set_sizes(Batch& b, atpm_solve* const* solves, int n) {
     for (int i = 0; i < n; ++i) {
         const DevSolve& d = solves[i]->ds;
+        b.facets += d.nf;
         if (!d.rem_ptr) continue;
         b.rem_nmb = std::max(b.rem_nmb, (d.nf + 127) / 128);
         b.rem_ntau = std::max(b.rem_ntau, d.ntau);
@@ -650,7 +652,7 @@ atpm_status make_batch_for(atpm_solve* const* solves, int n, Batch* out, void** 
         *out = make_batch(s0->ctx, s0->ds_dev, 1, s0->wmap, s0->nw, s0->fmap, s0->nfb, s0->P.precision, s0->P.nx);
         set_tc_map(*out, s0->qmap, (size_t)s0->nq);
         out->tc_nmax = s0->ds.tc_n;
-        set_remainder_grid(*out, solves, n);
+        set_sizes(*out, solves, n);
         return ATPM_OK;
     }
     std::vector<DevSolve> tab(n);
@@ -679,7 +681,7 @@ atpm_status make_batch_for(atpm_solve* const* solves, int n, Batch* out, void** 
                       reinterpret_cast<int2*>(t + bt + bw), (int)fm.size(), s0->P.precision, s0->P.nx);
     set_tc_map(*out, reinterpret_cast<int4*>(t + bt + bw + bf), qm.size());
     out->tc_nmax = nmax;
-    set_remainder_grid(*out, solves, n);
+    set_sizes(*out, solves, n);
     return ATPM_OK;
 }
 
@@ -700,7 +702,7 @@ atpm_status capture_graph(atpm_solve* s, const Batch& b, cudaGraphExec_t* out) {
 }
 
 // Autotuner for FAST batches.  Its knobs change launch configurations only,
-// never results: the conduction variant (k_conduction<FAST, NX, 1|2|3>: one
+// never results: the conduction variant (k_conduction<NX, 1|2|3>: one
 // source, three register budgets; 4: the paired-facet sweep) and the
 // tensor-core pipeline depth.  The first time a kind of batch (precision,
 // NX, step chunk, size class, number of groups) runs, its first kTuneRevs
@@ -711,15 +713,34 @@ atpm_status capture_graph(atpm_solve* s, const Batch& b, cudaGraphExec_t* out) {
 // issue slots to the other group's product therefore shows up as the faster
 // revolution, which the sweep's own duration does not show.  The fastest
 // candidates are kept in the context for every later batch of that kind.
-uint64_t tune_key(const Batch& b, int groups) {
+//
+// Neither knob reaches every batch.  With few enough facets the lane-split sweep
+// runs every revolution and there is no variant to choose; with few enough
+// product items they are dealt out in parts at a depth of their own (k_prepare).
+// Such batches are kinds of their own, which keep the default of the knob they
+// lack: timing it would choose by noise, and for larger batches of the same size
+// class (8,300 and 16,000 facets), which do have it, at 2.09 against 1.52 ms.
+struct TuneKind {
+    bool variants, depths;
+};
+TuneKind tune_kind(const std::vector<Batch>& bs) {
+    TuneKind k{false, false};
+    for (const Batch& b : bs) {
+        k.variants = k.variants || !few_always(b);
+        k.depths = k.depths || 2 * b.nq > b.sms || (b.nq > 0 && b.tc_nmax < 32);
+    }
+    return k;
+}
+uint64_t tune_key(const Batch& b, int groups, TuneKind kind) {
     int cls = 0;
     while ((1 << cls) < b.nfb && cls < 40) ++cls;  // facet blocks, power-of-two class
     return (uint64_t)b.mode | ((uint64_t)b.nx << 4) | ((uint64_t)b.tc_nmax << 12) | ((uint64_t)cls << 24) |
-           ((uint64_t)(b.nq > 0) << 32) | ((uint64_t)(groups > 1) << 33);
+           ((uint64_t)(b.nq > 0) << 32) | ((uint64_t)(groups > 1) << 33) | ((uint64_t)kind.variants << 34) |
+           ((uint64_t)kind.depths << 35);
 }
 
-// revolutions the autotuner times: conduction variants 1-4 at the deepest
-// tensor-core pipeline, then variant 4 one stage shallower
+// revolutions the autotuner times: conduction variants 1-4 (where there is one to
+// choose) at the deepest tensor-core pipeline, then variant 4 one stage shallower
 constexpr int kTuneRevs = 5;
 
 bool tune_log() {
@@ -732,7 +753,8 @@ atpm_status autotune(const std::vector<atpm_solve*>& leads, std::vector<Batch>& 
     atpm_solve* s0 = leads[0];
     atpm_context* c = s0->ctx;
     const int ng = (int)bs.size();
-    const uint64_t key = tune_key(bs[0], ng);
+    const TuneKind kind = tune_kind(bs);
+    const uint64_t key = tune_key(bs[0], ng, kind);
     auto apply = [&](int v, int d) {
         for (Batch& b : bs) {
             b.cond_variant = v;
@@ -754,8 +776,10 @@ atpm_status autotune(const std::vector<atpm_solve*>& leads, std::vector<Batch>& 
         return ATPM_OK;
     }
     const int smax = bs[0].nq > 0 ? tc_max_stages(bs[0].tc_nmax) : 0;
-    const int cand_v[kTuneRevs] = {1, 2, 3, 4, 4};
-    const int cand_d[kTuneRevs] = {smax, smax, smax, smax, smax > 2 ? smax - 1 : smax};
+    const int less = kind.depths && smax > 2 ? smax - 1 : smax;
+    int cand_v[kTuneRevs] = {1, 2, 3, 4, 4};
+    if (!kind.variants) std::fill(cand_v, cand_v + kTuneRevs, cond_variant());
+    const int cand_d[kTuneRevs] = {smax, smax, smax, smax, less};
     // per revolution: start and end on the leader's stream, the end of every other group
     const int nev = kTuneRevs * (1 + ng);
     std::vector<cudaEvent_t> ev(nev, nullptr);
@@ -788,17 +812,18 @@ atpm_status autotune(const std::vector<atpm_solve*>& leads, std::vector<Batch>& 
     if (e != cudaSuccess) return fail(ATPM_E_CUDA, "autotune: %s", cudaGetErrorString(e));
     // variant 4 unless another revolution was faster; ties keep it
     int best = 3;
-    for (int r = 0; r < 3; ++r)
+    for (int r = 0; r < 3 && kind.variants; ++r)
         if (rv[r] < rv[best]) best = r;
     atpm_tune_choice ch;
     ch.cond_variant = cand_v[best];
-    ch.tc_stages = (smax > 2 && rv[4] < rv[3]) ? smax - 1 : 0;
+    ch.tc_stages = (less < smax && rv[4] < rv[3]) ? less : 0;
     for (int r = 0; r < kTuneRevs; ++r) ch.rev_ms[r] = rv[r];
     if (tune_log())
         std::fprintf(stderr,
-                     "atpm autotune: %d group(s), revolution ms v1 %.4f v2 %.4f v3 %.4f v4 %.4f v4/depth-1 %.4f "
+                     "atpm autotune: %d group(s), revolution ms v%d %.4f v%d %.4f v%d %.4f v%d %.4f v%d/depth %d %.4f "
                      "-> variant %d depth %d\n",
-                     ng, rv[0], rv[1], rv[2], rv[3], rv[4], ch.cond_variant, ch.tc_stages);
+                     ng, cand_v[0], rv[0], cand_v[1], rv[1], cand_v[2], rv[2], cand_v[3], rv[3], cand_v[4], less, rv[4],
+                     ch.cond_variant, ch.tc_stages);
     {
         std::lock_guard<std::mutex> lk(c->mu);
         c->tune[key] = ch;
@@ -918,7 +943,7 @@ atpm_status batch_plan(atpm_solve* const* solves, int n, BatchPlan& plan, cudaSt
                         reinterpret_cast<int2*>(t + h.bt + h.bw), (int)h.fm.size(), s0->P.precision, s0->P.nx);
     set_tc_map(plan.b, reinterpret_cast<int4*>(t + h.bt + h.bw + h.bf), h.qm.size());
     plan.b.tc_nmax = h.nmax;
-    set_remainder_grid(plan.b, solves, n);
+    set_sizes(plan.b, solves, n);
     plan.solves.assign(solves, solves + n);
     return ATPM_OK;
 }
@@ -979,7 +1004,7 @@ atpm_status batch_step(atpm_solve* const* solves, int n, int k, void* table, cud
                          reinterpret_cast<int2*>(t + h.bt + h.bw), (int)h.fm.size(), s0->P.precision, s0->P.nx);
     set_tc_map(b, reinterpret_cast<int4*>(t + h.bt + h.bw + h.bf), h.qm.size());
     b.tc_nmax = h.nmax;
-    set_remainder_grid(b, solves, n);
+    set_sizes(b, solves, n);
     for (int r = 0; r < k; ++r)
         if (launch_revolution(b, st)) return fail(ATPM_E_CUDA, "batched revolution launch");
     return ATPM_OK;

@@ -286,10 +286,13 @@ struct Batch {
                              // solves at most half active sweep the list of their active facets
     int tail_limit;          // advancing facets of the batch up to which 16 lanes share a facet,
     int few_limit;           // and up to which 4 do
+    int facets;              // of all its solves
     int sms;                 // SMs of the device (persistent tensor-core grid)
     int rem_nmb, rem_ntau;   // largest row-block count / steps of the batch's solves with a
                              // sparse remainder (0: none; the remainder kernel's grid)
 };
+// the lane-split sweep runs every FAST revolution of the batch
+inline bool few_always(const Batch& b) { return b.warp_tail && b.facets <= b.few_limit; }
 // deepest tensor-core pipeline that fits shared memory for step chunk N
 int tc_max_stages(int N);
 int launch_revolution(const Batch& b, stream_t st);  // W, Q, conduction, convergence

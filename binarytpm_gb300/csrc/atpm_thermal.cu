@@ -856,6 +856,9 @@ bool conduction_nx_supported(int nx) {
     return false;
 }
 
+// some revolution has the paired sweep
+static bool pairs_run(const Batch& b) { return b.cond_variant == 4 && !few_always(b); }
+
 template <int MODE>
 static int launch_rev_part(const Batch& b, int part, cudaStream_t st) {
     if (MODE == MODE_FAST && part == 0) k_prepare<<<1, kPrepThreads, 0, st>>>(b);
@@ -878,7 +881,7 @@ static int launch_rev_part(const Batch& b, int part, cudaStream_t st) {
         if (b.cond_variant >= 3) k_conduction<N, 3><<<b.nfb, 128, 0, st>>>(b);            \
         else if (b.cond_variant == 2) k_conduction<N, 2><<<b.nfb, 128, 0, st>>>(b);       \
         else k_conduction<N, 1><<<b.nfb, 128, 0, st>>>(b);                                \
-        if (b.cond_variant == 4) k_conduction_pairs<N><<<b.nfb, 64, 0, st>>>(b);          \
+        if (pairs_run(b)) k_conduction_pairs<N><<<b.nfb, 64, 0, st>>>(b);                 \
         break;
                 NX_LIST(NX_CASE)
 #undef NX_CASE
@@ -907,7 +910,7 @@ int kernels_per_revolution(const Batch& b) {
     // k_spmm_tc (+ k_spmm_rem), or W + Q
     const int selfheat = tc ? 1 + (b.rem_nmb > 0 ? 1 : 0) : (b.nw > 0 ? 2 : 0);
     // k_prepare, k_conduction, k_conduction_few (+ k_conduction_pairs)
-    const int conduction = b.mode == MODE_FAST ? (b.cond_variant == 4 ? 4 : 3) : 1;
+    const int conduction = b.mode == MODE_FAST ? (pairs_run(b) ? 4 : 3) : 1;
     return selfheat + conduction + 1;                    // + k_converge
 }
 

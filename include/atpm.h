@@ -266,10 +266,13 @@ ATPM_API atpm_status atpm_selftest_bounded_wait(int32_t device, int64_t limit_cy
  * the plain drivers ran (ATPM_SHADOW_CULL=0). */
 ATPM_API atpm_status atpm_last_shadow_stats(atpm_solve* s, double* shadow_ms, int64_t* rays, int64_t* exact_tests);
 /* Launch configuration of the last atpm_batch_run led by s (FAST): the
- * conduction register/occupancy variant (1-3), the tensor-core pipeline
- * depth, and whether that run timed the candidates (the autotuner does so
- * on the first three revolutions of the first batch of each kind; its
- * choices never change results).  ATPM_AUTOTUNE=0 turns it off. */
+ * conduction variant (1-4: three register budgets of the thread-per-facet
+ * sweep, two facets a thread) of its revolutions with more advancing facets
+ * than the lane-split sweep takes, the tensor-core pipeline depth, and
+ * whether that run timed the candidates (the autotuner does so on the first
+ * five revolutions of the first batch of each kind; its choices never change
+ * results, and a kind without a use for one of the two keeps its default).
+ * ATPM_AUTOTUNE=0 turns it off. */
 ATPM_API atpm_status atpm_last_run_config(atpm_solve* s, int32_t* cond_variant, int32_t* tc_stages, int32_t* tuned);
 /* Device time (ms, CUDA events on the solve's stream) of the last atpm_run /
  * atpm_batch_run revolution loop, and launches issued inside it. */
