@@ -593,6 +593,7 @@ atpm_status ensure_gs_plan(atpm_solve* s) {
         gs->plan.off = reinterpret_cast<const int*>(m + b_rows);
         gs->plan.mid = reinterpret_cast<const int*>(m + b_rows + b_off);
         gs->plan.levels = levels;
+        gs->plan.listed = (int)rows.size();
     }
     s->gs = gs;
     return ATPM_OK;

@@ -255,6 +255,7 @@ struct GsPlan {
     const int* off;    // [levels + 1] first row of each level
     const int* mid;    // [nf] first entry above the facet
     int levels;
+    int listed;        // facets with a list
 };
 constexpr size_t kGsSharedBytes = 220 * 1024;  // one CTA's values (k_multi_levels)
 int launch_multiple_scattering(const DevSolve& s, const GsPlan& plan, void* work, stream_t st);

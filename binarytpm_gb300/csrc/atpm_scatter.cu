@@ -11,8 +11,8 @@
 //                     from the last sweep) until every |change| <= accuracy;
 //                     one warp per step, lanes fetch 32 list entries at once
 //                     and the two partial sums are accumulated in list order
-//                     (unsorted lists, very large shapes, and the
-//                     no-allocation entry point)
+//                     (unsorted lists, lists that chain facet to facet, very
+//                     large shapes, and the no-allocation entry point)
 //   k_multi_levels    the same sweeps with every facet whose lower neighbours
 //                     are done swept together
 //   k_multi_jacobi    FAST precision: Jacobi sweeps of every facet and step at
@@ -473,25 +473,41 @@ int multiple_scattering_jacobi(const DevSolve& s, void* work, cudaStream_t st, i
 }  // namespace
 
 namespace {
+// -1: not launched, the facet-by-facet kernel is faster
 template <int MODE, int STEPS>
 int launch_levels(const DevSolve& s, const GsPlan& plan, void* work, cudaStream_t st, int cap) {
+    const auto kernel = k_multi_levels<MODE, STEPS>;
     const size_t smem = (size_t)s.nf * STEPS * sizeof(typename Sa<MODE>::R);
     // the limit belongs to the function, not to the launch: every thread sets the
     // same one, or a small shape's would refuse a large one's launch
-    if (cudaFuncSetAttribute(k_multi_levels<MODE, STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)kGsSharedBytes) != cudaSuccess)
+    int dev = 0, sms = 0, per = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGsSharedBytes) != cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, 1024, smem) != cudaSuccess || per < 1)
         return 2;
-    k_multi_levels<MODE, STEPS><<<(s.ntau + STEPS - 1) / STEPS, 1024, smem, st>>>(s, plan, work, cap);
+    // A level costs a barrier in every wave of CTAs, a facet of the other kernel a
+    // warp's turn, and they cost about the same: lists that chain facet to facet go
+    // facet by facet.  ms by levels and by facets, 720 steps, 2 neighbours either
+    // side of a facet: 5,440 facets (one wave) 9.9 and 8.6 in 5,440 levels, 6.0 and
+    // 8.6 in 2,720; 12,000 (two waves) 37 and 20 in 12,000, 22 and 20 in 6,000;
+    // 20,480 (three) 98 and 36 in 20,480, 53 and 36 in 10,240; 16 neighbours,
+    // 20,480 facets 54 and 53 in 6,826, 36 and 54 in 5,120.
+    const long long grid = (s.ntau + STEPS - 1) / STEPS, waves = (grid + (long long)sms * per - 1) / ((long long)sms * per);
+    if (6 * waves * plan.levels > 5ll * plan.listed) return -1;
+    kernel<<<(unsigned)grid, 1024, smem, st>>>(s, plan, work, cap);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 // as many steps a CTA (lanes a facet) as their values fit shared memory
 template <int MODE>
 int launch_gauss_seidel(const DevSolve& s, const GsPlan& plan, void* work, cudaStream_t st, int cap) {
     const size_t most = kGsSharedBytes / sizeof(typename Sa<MODE>::R) / (size_t)s.nf;
-    if (plan.rows && most >= 8) return launch_levels<MODE, 8>(s, plan, work, st, cap);
-    if (plan.rows && most >= 4) return launch_levels<MODE, 4>(s, plan, work, st, cap);
-    if (plan.rows && most >= 2) return launch_levels<MODE, 2>(s, plan, work, st, cap);
-    if (plan.rows && most >= 1) return launch_levels<MODE, 1>(s, plan, work, st, cap);
+    int rc = -1;
+    if (plan.rows && most >= 8) rc = launch_levels<MODE, 8>(s, plan, work, st, cap);
+    else if (plan.rows && most >= 4) rc = launch_levels<MODE, 4>(s, plan, work, st, cap);
+    else if (plan.rows && most >= 2) rc = launch_levels<MODE, 2>(s, plan, work, st, cap);
+    else if (plan.rows && most >= 1) rc = launch_levels<MODE, 1>(s, plan, work, st, cap);
+    if (rc >= 0) return rc;
     k_multi_gs<MODE><<<s.ntau, 32, 0, st>>>(s, work, cap);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
