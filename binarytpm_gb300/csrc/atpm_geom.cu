@@ -70,7 +70,7 @@ struct Proj {
     float* w;         // [nv][ntau] depth behind the body centre along c
     unsigned* stats;  // [0] max |u|,|v| (float bits), [1] max box extent, [2] bad-projection flag, [3] max |w|,
                       // [4] max -w
-    float4* wbox;     // [windows][nf] union of each facet's padded boxes over 32 steps
+    float4* wbox;     // [windows][nf] union of each facet's padded boxes over 32 steps (or null)
 };
 
 __device__ __forceinline__ unsigned warp_max(unsigned v) { return __reduce_max_sync(__activemask(), v); }
@@ -464,12 +464,12 @@ __global__ void __launch_bounds__(256, 3) k_shadow_dep_cull(GeomArgs a, Proj p) 
         qb.z = fminf(qb.z, __shfl_xor_sync(0xffffffffu, qb.z, o2));
         qb.w = fmaxf(qb.w, __shfl_xor_sync(0xffffffffu, qb.w, o2));
     }
-    const float4* wb = p.wbox + (size_t)blockIdx.x * nf;  // this warp's step window
+    const float4* wb = p.wbox ? p.wbox + (size_t)blockIdx.x * nf : nullptr;  // this warp's step window
     for (int k0 = d0; k0 < d1; k0 += 32) {
         if (!__any_sync(0xffffffffu, lit)) break;
         const bool have = k0 + lane < d1;
         const int mine = have ? __ldg(&a.s.dep_idx[k0 + lane]) : 0;
-        const float4 u = __ldg(wb + mine);
+        const float4 u = wb ? __ldg(wb + mine) : make_float4(-INFINITY, INFINITY, -INFINITY, INFINITY);
         unsigned left = __ballot_sync(0xffffffffu, have && !(u.x > qb.y || u.y < qb.x || u.z > qb.w || u.w < qb.z));
         for (; left; left &= left - 1) {
             const int h = __shfl_sync(0xffffffffu, mine, __ffs(left) - 1);
@@ -715,12 +715,15 @@ int launch_shadow_culled(const DevSolve& s, const GeomWork& g, bool all_pairs, s
     if (!all_pairs) {
         const int nw = (s.ntau + 31) / 32;
         void* wm = nullptr;
-        if (cudaMallocAsync(&wm, (size_t)nw * s.nf * sizeof(float4), st) != cudaSuccess) return 2;
-        p.wbox = static_cast<float4*>(wm);
         const dim3 blk(32, 8), grd(nw, (s.nf + 7) / 8);
-        k_window_box<<<grd, blk, 0, st>>>(a, p);
+        if (cudaMallocAsync(&wm, (size_t)nw * s.nf * sizeof(float4), st) == cudaSuccess) {
+            p.wbox = static_cast<float4*>(wm);
+            k_window_box<<<grd, blk, 0, st>>>(a, p);
+        } else {
+            cudaGetLastError();  // without window boxes: the per-step tests alone (same flags)
+        }
         k_shadow_dep_cull<<<grd, blk, 0, st>>>(a, p);
-        cudaFreeAsync(wm, st);
+        if (wm) cudaFreeAsync(wm, st);
     } else {
         k_grid_extent<<<(unsigned)((nft + 255) / 256), 256, 0, st>>>(a, p);
         if (!read_stats()) return 2;

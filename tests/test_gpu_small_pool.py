@@ -1,0 +1,72 @@
+"""Calls whose scratch memory only makes them faster, with device memory for less
+than that: they go on without it, with the same results."""
+import contextlib
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+GRANULE = 32 << 20  # a pool's limit is rounded up to whole ones
+
+
+class _Location(C.Structure):
+    _fields_ = [("type", C.c_int), ("id", C.c_int)]
+
+
+class _PoolProps(C.Structure):  # CUmemPoolProps
+    _fields_ = [("alloc_type", C.c_int), ("handle_types", C.c_int), ("location", _Location), ("security", C.c_void_p),
+                ("max_size", C.c_size_t), ("usage", C.c_ushort), ("reserved", C.c_ubyte * 54)]
+
+
+@contextlib.contextmanager
+def _room(size):
+    """Device 0's stream-ordered allocations come from a pool with `size` bytes left."""
+    cu = C.CDLL("libcuda.so.1")
+
+    def ok(rc):
+        assert rc == 0, rc
+
+    pool, before, filler = C.c_void_p(), C.c_void_p(), C.c_void_p()
+    props = _PoolProps(1, 0, _Location(1, 0), None, GRANULE, 0)
+    ok(cu.cuMemPoolCreate(C.byref(pool), C.byref(props)))
+    ok(cu.cuMemAllocFromPoolAsync(C.byref(filler), C.c_size_t(GRANULE - size), pool, None))
+    ok(cu.cuStreamSynchronize(None))
+    ok(cu.cuDeviceGetMemPool(C.byref(before), 0))
+    ok(cu.cuDeviceSetMemPool(0, pool))
+    try:
+        yield
+    finally:
+        ok(cu.cuDeviceSetMemPool(0, before))
+        ok(cu.cuMemFreeAsync(filler, None))
+        ok(cu.cuCtxSynchronize())
+        ok(cu.cuMemPoolDestroy(pool))
+
+
+def _problem(nf=80000, ntau=128, **kw):
+    """Many facets over few vertices: whatever goes by facets and steps is large."""
+    from binarytpm_gb300 import problem
+
+    rng = np.random.default_rng(3)
+    facets = np.stack([(np.arange(nf) * k + j) % 41 for j, k in enumerate((1, 3, 7))], 1).astype(np.int32)
+    facets[:, 2] = np.where((facets[:, 2] == facets[:, 0]) | (facets[:, 2] == facets[:, 1]), (facets[:, 2] + 11) % 41,
+                            facets[:, 2])
+    near = np.sort(rng.integers(0, nf, (2000, 5)), axis=1)
+    ptr = np.minimum(5 * np.arange(nf + 1), near.size).astype(np.int32)
+    return problem.Problem(rng.normal(size=(41, 3)), facets, ptr, near.reshape(-1).astype(np.int32),
+                           np.full(near.size, 0.05, np.float32), ntau=ntau, nx=8, **kw)
+
+
+@pytest.mark.parametrize("precision", [0, 2])
+def test_shadowing_without_window_boxes(gpu_ctx, precision):
+    from binarytpm_gb300 import lib
+
+    s = lib.Solve(gpu_ctx, _problem(), precision=precision)
+    s.geometry_shadow()
+    want = s.shadow()
+    with _room(4 << 20):  # projected vertices fit, the boxes of 80,000 facets and 4 windows (5 MB) do not
+        s.geometry_shadow()
+    assert np.array_equal(s.shadow(), want)
+    assert 0 < want[:2000].sum() < want[:2000].size
+    s.close()
