@@ -1805,8 +1805,21 @@ ATPM_API atpm_status atpm_get_shadow(atpm_solve* s, int32_t* out) {
     // page-locked memory)
     const size_t nt = (size_t)s->nf * s->P.ntau;
     void* tmp = nullptr;
-    CK(cudaMallocAsync(&tmp, nt * 4, s->st));
-    cudaError_t e = cudaSuccess;
+    cudaError_t e = cudaMallocAsync(&tmp, nt * 4, s->st);
+    if (e == cudaErrorMemoryAllocation) {
+        // no room for the words: the bytes into the end of the caller's buffer,
+        // widened from its front (word i never reaches past byte i)
+        cudaGetLastError();
+        uint8_t* bytes = reinterpret_cast<uint8_t*>(out) + 3 * nt;
+        CK(cudaMemcpyAsync(bytes, s->ds.shadow, nt, cudaMemcpyDeviceToHost, s->st));
+        CK(cudaStreamSynchronize(s->st));
+        for (size_t i = 0; i < nt; ++i) {
+            const int32_t flag = bytes[i];
+            std::memcpy(reinterpret_cast<uint8_t*>(out) + 4 * i, &flag, 4);
+        }
+        return ATPM_OK;
+    }
+    CK(e);
     if (launch_widen_flags(s->ds.shadow, static_cast<int32_t*>(tmp), nt, s->st)) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, tmp, nt * 4, cudaMemcpyDeviceToHost, s->st);
     cudaFreeAsync(tmp, s->st);

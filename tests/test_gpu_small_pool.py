@@ -70,3 +70,17 @@ def test_shadowing_without_window_boxes(gpu_ctx, precision):
     assert np.array_equal(s.shadow(), want)
     assert 0 < want[:2000].sum() < want[:2000].size
     s.close()
+
+
+@pytest.mark.parametrize("nf,ntau", [(80000, 128), (70001, 127)])
+def test_shadow_flags_without_staging(gpu_ctx, nf, ntau):
+    from binarytpm_gb300 import lib
+
+    s = lib.Solve(gpu_ctx, _problem(nf, ntau, shadowing=0), precision=0)
+    s.geometry_shadow()
+    want = s.shadow()
+    with _room(4 << 20):
+        got = s.shadow()
+    assert np.array_equal(got, want)
+    assert 0 < want.sum() < want.size
+    s.close()
