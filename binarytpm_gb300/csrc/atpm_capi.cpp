@@ -1460,14 +1460,16 @@ ATPM_API atpm_status atpm_scattering(atpm_solve* s) {
         if (rp) return rp;
     }
     void* work = nullptr;
-    CK(cudaMallocAsync(&work, scattering_work_bytes(s->ds, multiple), s->st));
+    const cudaError_t ea = cudaMallocAsync(&work, scattering_work_bytes(s->ds, multiple), s->st);
+    if (ea == cudaErrorMemoryAllocation && !multiple) cudaGetLastError();  // single scattering needs none
+    else CK(ea);
     int rc = launch_single_scattering(s->ds, work, multiple, s->st);
     const char* what = "single scattering launch";
     if (!rc && multiple) {
         rc = launch_multiple_scattering(s->ds, s->gs ? s->gs->plan : GsPlan{}, work, s->st);
         what = "multiple scattering launch";
     }
-    cudaFreeAsync(work, s->st);
+    if (work) cudaFreeAsync(work, s->st);
     if (rc) return fail(ATPM_E_CUDA, "%s", what);
     if (launch_forcing_transpose(s->ds, s->st)) return fail(ATPM_E_CUDA, "forcing transpose launch");
     int st = 0;

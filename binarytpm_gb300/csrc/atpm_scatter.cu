@@ -4,8 +4,9 @@
 //   k_lit_cosine, k_single_rows
 //                     E[f][s] = S cos_f shadow_f + sum_k vf_k S A cos_g shadow_g
 //                     over rows of cos x shadow (atpm_gather.cuh)
-//   k_single_scatter  the same without the rows, for the no-allocation entry
-//                     point: warp = 32 steps of one facet
+//   k_single_scatter  the same without the rows, where there is no memory for
+//                     them and for the no-allocation entry point: warp = 32
+//                     steps of one facet
 //   k_multi_gs        the reference's per-step Gauss-Seidel sweep in facet
 //                     order (values of facets before f in this sweep, after f
 //                     from the last sweep) until every |change| <= accuracy;
@@ -412,6 +413,10 @@ template <int MODE>
 void launch_single(const DevSolve& s, void* work, bool multiple, cudaStream_t st) {
     using R = typename Sa<MODE>::R;
     R* lit = static_cast<R*>(work);
+    if (!lit) {
+        k_single_scatter<MODE><<<dim3((s.ntau + 31) / 32, (s.nf + 7) / 8), dim3(32, 8), 0, st>>>(s);
+        return;
+    }
     const size_t n = rows_words(s);
     R* next = MODE == MODE_FAST && multiple ? lit + n : nullptr;
     const dim3 blk(32, 8);
@@ -421,7 +426,8 @@ void launch_single(const DevSolve& s, void* work, bool multiple, cudaStream_t st
 }
 }  // namespace
 
-// work: scattering_work_bytes, kept for launch_multiple_scattering
+// work: scattering_work_bytes, kept for launch_multiple_scattering (null for single
+// scattering alone where there is no room for it)
 int launch_single_scattering(const DevSolve& s, void* work, bool multiple, stream_t stv) {
     cudaStream_t st = static_cast<cudaStream_t>(stv);
     switch (s.mode) {

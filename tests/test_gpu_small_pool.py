@@ -84,3 +84,29 @@ def test_shadow_flags_without_staging(gpu_ctx, nf, ntau):
     assert np.array_equal(got, want)
     assert 0 < want.sum() < want.size
     s.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1, 2])
+def test_single_scattering_without_rows(gpu_ctx, precision):
+    from binarytpm_gb300 import lib
+
+    s = lib.Solve(gpu_ctx, _problem(shadowing=0, albedo=0.3, multiple_scattering=0), precision=precision)
+    s.geometry_shadow()
+    s.scattering()
+    want = s.illumination()
+    s.set_albedo(0.0)
+    s.scattering()
+    direct = s.illumination()
+    s.set_albedo(0.3)
+    with _room(4 << 20):
+        s.scattering()
+    got = s.illumination()
+    nan = np.isnan(want)  # some facets here have two corners alike
+    assert np.array_equal(np.isnan(got), nan)
+    got, want, direct = got[~nan], want[~nan], direct[~nan]
+    if precision == 2:  # FAST may contract its products either way: two roundings of terms below the sum
+        assert np.all(np.abs(got - want) <= 8 * 2.0 ** -24 * np.abs(want) + 1e-30)
+    else:
+        assert np.array_equal(got, want)
+    assert (want != direct).any()
+    s.close()
