@@ -2023,13 +2023,22 @@ atpm_status disk_flux_impl(atpm_solve* s, const double* observer, const int32_t*
         a.b1[l] = (2.0 * hcon * cvel * cvel) / std::pow(wl, 5.0);
         a.hl[l] = (hcon * cvel) / (wl * kcon);
     }
-    const size_t nt = (size_t)nf * ntau;
     const size_t b_rot = align256(rot.size() * 8), b_part = align256(flux_partial_bytes(s->ds, nwl)),
-                 b_out = align256((size_t)ntau * nwl * 8), b_vis = visibility ? align256(nt) : 0,
-                 b_flags = visibility ? align256(nt * 4) : 0, b_geo = rough ? align256((size_t)rough->nsf * 4 * 8) : 0,
-                 b_hp = align256((size_t)s->nv * ntau * 24), b_area = align256((size_t)nf * 8);
+                 b_out = align256((size_t)ntau * nwl * 8), b_geo = rough ? align256((size_t)rough->nsf * 4 * 8) : 0,
+                 b_area = align256((size_t)nf * 8);
+    // positions and flags of all steps at once, or of as many as there is memory for
+    int ns = ntau;
+    size_t b_hp, b_vis, b_flags;
     void* tmp = nullptr;
-    CK(cudaMallocAsync(&tmp, b_rot + b_part + b_out + b_vis + b_flags + b_geo + b_hp + b_area, s->st));
+    for (;; ns = (ns + 1) / 2) {
+        b_hp = align256((size_t)s->nv * ns * 24);
+        b_vis = visibility ? align256((size_t)nf * ns) : 0;
+        b_flags = visibility ? align256((size_t)nf * ns * 4) : 0;
+        const cudaError_t ea = cudaMallocAsync(&tmp, b_rot + b_part + b_out + b_vis + b_flags + b_geo + b_hp + b_area, s->st);
+        if (ea == cudaSuccess) break;
+        if (ea != cudaErrorMemoryAllocation || ns == 1) CK(ea);
+        cudaGetLastError();
+    }
     char* t = static_cast<char*>(tmp);
     auto take = [&t](size_t bytes) {
         char* p = t;
@@ -2048,12 +2057,19 @@ atpm_status disk_flux_impl(atpm_solve* s, const double* observer, const int32_t*
     }
     if (rough) a.sub_geo = reinterpret_cast<const double*>(take(b_geo));
     cudaError_t e = cudaMemcpyAsync((void*)a.rot, rot.data(), rot.size() * 8, cudaMemcpyHostToDevice, s->st);
-    if (e == cudaSuccess && visibility)
-        e = cudaMemcpyAsync((void*)a.flags, visibility, nt * 4, cudaMemcpyHostToDevice, s->st);
     if (e == cudaSuccess && rough)
         e = cudaMemcpyAsync((void*)a.sub_geo, rough->sub_geo, (size_t)rough->nsf * 4 * 8, cudaMemcpyHostToDevice, s->st);
     int rc = 0;
-    if (e == cudaSuccess) rc = launch_disk_flux(s->ds, a, s->st);
+    for (int end = ntau; end > 0 && e == cudaSuccess && !rc; end = a.s0) {
+        a.s0 = std::max(0, end - ns);
+        a.ns = end - a.s0;
+        if (visibility)
+            e = a.ns == ntau ? cudaMemcpyAsync((void*)a.flags, visibility, (size_t)nf * ntau * 4, cudaMemcpyHostToDevice, s->st)
+                             : cudaMemcpy2DAsync((void*)a.flags, (size_t)a.ns * 4, visibility + a.s0, (size_t)ntau * 4,
+                                                 (size_t)a.ns * 4, nf, cudaMemcpyHostToDevice, s->st);
+        if (e == cudaSuccess) rc = launch_flux_steps(s->ds, a, s->st);
+    }
+    if (e == cudaSuccess && !rc) rc = launch_flux_sum(s->ds, a, s->st);
     if (e == cudaSuccess && !rc) e = cudaMemcpyAsync(flux, a.out, (size_t)ntau * nwl * 8, cudaMemcpyDeviceToHost, s->st);
     cudaFreeAsync(tmp, s->st);
     cudaError_t e2 = cudaStreamSynchronize(s->st);

@@ -51,8 +51,8 @@ __device__ __forceinline__ double temp_at(const DevSolve& s, int f, int step) {
 
 __global__ void __launch_bounds__(256) k_flux_vertices(DevSolve s, FluxArgs a) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)s.nv * s.ntau) return;
-    const int step = (int)(i / s.nv), v = (int)(i % s.nv);
+    if (i >= (long long)s.nv * a.ns) return;
+    const int step = a.s0 + (int)(i / s.nv), v = (int)(i % s.nv);
     const double* e = s.vert + 3 * v;
     const double* rt = (v < a.vsplit) ? a.rot : a.rot2;
     const double c = rt[2 * step], sn = rt[2 * step + 1];
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256) k_flux_vertices(DevSolve s, FluxArgs a) {
 struct Facet {
     double sum[3], edge[3], n[3];
     __device__ __forceinline__ Facet(const DevSolve& s, const FluxArgs& a, int f, int step) {
-        const double* hp = a.hp + (size_t)step * s.nv * 3;
+        const double* hp = a.hp + (size_t)(step - a.s0) * s.nv * 3;
         const int* fv = s.fac + 3 * f;
         const double *h0 = hp + 3 * (size_t)fv[0], *h1 = hp + 3 * (size_t)fv[1], *h2 = hp + 3 * (size_t)fv[2];
         double nc1[3];
@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(256) k_flux_area(DevSolve s, FluxArgs a) {
     a.area[f] = __ddiv_rn(__dsqrt_rn(dot3(t.n, t.n)), 2.0);
 }
 
-// [nf][ntau] words -> [ntau][nf] bytes
+// [nf][steps] words -> [steps][nf] bytes
 __global__ void __launch_bounds__(256) k_flux_flags(const int32_t* src, uint8_t* dst, int nf, int ntau) {
     __shared__ uint8_t t[32][33];
     const int f0 = blockIdx.y * 32, s0 = blockIdx.x * 32;
@@ -166,13 +166,13 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux_partial(DevSolve s, FluxA
     __shared__ double red[kMaxFluxWavelengths][kWarps];
     // rough: each facet's unit view vector in its frame and its weight
     __shared__ double view[ROUGH ? kFluxThreads : 1][4];
-    const int step = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int step = a.s0 + blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int f = blockIdx.x * kFluxThreads + threadIdx.x;
     double term[kMaxFluxWavelengths];
 #pragma unroll
     for (int l = 0; l < kMaxFluxWavelengths; ++l) term[l] = 0.0;
     double weight = 0.0;
-    if (f < s.nf && (!a.visible || a.visible[(size_t)step * s.nf + f])) {
+    if (f < s.nf && (!a.visible || a.visible[(size_t)blockIdx.y * s.nf + f])) {
         const Facet t(s, a, f, step);
         double ov[3];  // from the facet to the observer
 #pragma unroll
@@ -277,17 +277,16 @@ size_t flux_partial_bytes(const DevSolve& s, int nwl) {
     return nblk * s.ntau * nwl * sizeof(double);
 }
 
-int launch_disk_flux(const DevSolve& s, const FluxArgs& a, stream_t stv) {
+int launch_flux_steps(const DevSolve& s, const FluxArgs& a, stream_t stv) {
     cudaStream_t st = static_cast<cudaStream_t>(stv);
     if (a.nwl < 1 || a.nwl > kMaxFluxWavelengths) return 1;
-    const int nblk = (s.nf + kFluxThreads - 1) / kFluxThreads;
-    const dim3 grid(nblk, s.ntau);
-    const long long nvt = (long long)s.nv * s.ntau;
+    const dim3 grid((s.nf + kFluxThreads - 1) / kFluxThreads, a.ns);
+    const long long nvt = (long long)s.nv * a.ns;
     k_flux_vertices<<<(unsigned)((nvt + 255) / 256), 256, 0, st>>>(s, a);
-    k_flux_area<<<(s.nf + 255) / 256, 256, 0, st>>>(s, a);
+    if (a.s0 + a.ns == s.ntau) k_flux_area<<<(s.nf + 255) / 256, 256, 0, st>>>(s, a);
     if (a.visible)
-        k_flux_flags<<<dim3((s.ntau + 31) / 32, (s.nf + 31) / 32), dim3(32, 8), 0, st>>>(
-            a.flags, const_cast<uint8_t*>(a.visible), s.nf, s.ntau);
+        k_flux_flags<<<dim3((a.ns + 31) / 32, (s.nf + 31) / 32), dim3(32, 8), 0, st>>>(
+            a.flags, const_cast<uint8_t*>(a.visible), s.nf, a.ns);
     if (a.sub_T) {
         if (s.mode == MODE_FP64) k_flux_partial<double, true><<<grid, kFluxThreads, 0, st>>>(s, a);
         else k_flux_partial<float, true><<<grid, kFluxThreads, 0, st>>>(s, a);
@@ -295,7 +294,12 @@ int launch_disk_flux(const DevSolve& s, const FluxArgs& a, stream_t stv) {
         if (s.mode == MODE_FP64) k_flux_partial<double, false><<<grid, kFluxThreads, 0, st>>>(s, a);
         else k_flux_partial<float, false><<<grid, kFluxThreads, 0, st>>>(s, a);
     }
-    k_flux_sum<<<(s.ntau * a.nwl + 127) / 128, 128, 0, st>>>(a, s.ntau, nblk);
+    return cudaGetLastError() == cudaSuccess ? 0 : 2;
+}
+
+int launch_flux_sum(const DevSolve& s, const FluxArgs& a, stream_t stv) {
+    const int nblk = (s.nf + kFluxThreads - 1) / kFluxThreads;
+    k_flux_sum<<<(s.ntau * a.nwl + 127) / 128, 128, 0, static_cast<cudaStream_t>(stv)>>>(a, s.ntau, nblk);
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
 }
 

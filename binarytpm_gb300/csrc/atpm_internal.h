@@ -335,9 +335,10 @@ struct FluxArgs {
     double car[3];           // body centre (km)
     double obs[3];           // observer (km)
     double eps;
-    const int32_t* flags;    // [nf][ntau] visibility words, or null (horizon test only)
-    const uint8_t* visible;  // [ntau][nf] their bytes (k_flux_flags), or null
-    double* hp;              // [ntau][nv][3] vertex positions (k_flux_vertices)
+    int s0, ns;              // the steps of this launch
+    const int32_t* flags;    // [nf][ns] visibility words, or null (horizon test only)
+    const uint8_t* visible;  // [ns][nf] their bytes (k_flux_flags), or null
+    double* hp;              // [ns][nv][3] vertex positions (k_flux_vertices)
     double* area;            // [nf] (k_flux_area)
     int nwl;
     double b1[kMaxFluxWavelengths];  // 2 h c^2 / lambda^5
@@ -352,7 +353,10 @@ struct FluxArgs {
     double sub_total;        // sum over sub-facets of area * normal_z
 };
 size_t flux_partial_bytes(const DevSolve& s, int nwl);
-int launch_disk_flux(const DevSolve& s, const FluxArgs& a, stream_t st);
+// the block partials of steps a.s0 .. a.s0 + a.ns - 1, the last steps first (the
+// areas are the last step's); then all steps' sums
+int launch_flux_steps(const DevSolve& s, const FluxArgs& a, stream_t st);
+int launch_flux_sum(const DevSolve& s, const FluxArgs& a, stream_t st);
 // tensor-core self-heating (atpm_spmm_tc.cu)
 int launch_w_bf16_one(const DevSolve& s, stream_t st);
 int launch_spmm_tc(const Batch& b, stream_t st);

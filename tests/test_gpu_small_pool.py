@@ -110,3 +110,24 @@ def test_single_scattering_without_rows(gpu_ctx, precision):
         assert np.array_equal(got, want)
     assert (want != direct).any()
     s.close()
+
+
+@pytest.mark.parametrize("flags", [True, False])
+def test_disk_flux_a_few_steps_at_a_time(gpu_ctx, flags):
+    from binarytpm_gb300 import lib
+
+    nf, ntau = 12000, 701
+    prob = _problem(nf, ntau, shadowing=0)
+    s = lib.Solve(gpu_ctx, prob, precision=0)
+    rng = np.random.default_rng(8)
+    s.set_forcing(np.ones((nf, ntau), np.int32), (600 * rng.random((nf, ntau))).astype(np.float32))
+    s.set_thermal_inertia(100.0)
+    s.initialise_temperatures()
+    seen = (rng.random((nf, ntau)) < 0.7).astype(np.int32) if flags else None
+    observer, wl = (0.9, 0.1, 0.3), (4.6, 11.1)
+    want = s.disk_flux(observer, wl, seen)
+    with _room(1 << 20):  # the block sums take 0.53 MB, the positions 0.69, the flags 42
+        got = s.disk_flux(observer, wl, seen)
+    assert np.array_equal(got, want)
+    assert (want > 0).all()
+    s.close()
