@@ -1075,15 +1075,38 @@ ATPM_API atpm_status atpm_context_destroy(atpm_context* c) {
     return ATPM_OK;
 }
 
+namespace {
+bool wants_shadows(const atpm_params& P, int nnz) { return (P.shadowing == 1 && nnz > 0) || P.shadowing == 2; }
+
+// atpm_geometry_shadow's scratch: vertex positions, rotation tables, the culled
+// drivers' projection, their statistics and test counts
+struct GeomSizes {
+    size_t hp, rot, uv, depth, total;
+};
+GeomSizes geometry_sizes(int nv, int ntau, bool cull) {
+    const size_t nvt = (size_t)nv * ntau;
+    GeomSizes z{align256(nvt * 24), align256((size_t)ntau * 32), cull ? align256(nvt * 8) : 0, cull ? align256(nvt * 4) : 0, 0};
+    z.total = z.hp + z.rot + z.uv + z.depth + 256 + 64 * 8;
+    return z;
+}
+// the plain shadow drivers' midpoints, normals and distances besides
+size_t plain_sizes(size_t nt) { return 2 * align256(nt * 24) + align256(nt * 8); }
+}  // namespace
+
 ATPM_API atpm_status atpm_solve_footprint(const atpm_shape* sh, const atpm_params* P, uint64_t* bytes) {
     atpm_status r = check_shape(sh, P);
     if (r) return r;
     Layout L = layout(sh->nv, sh->nf, sh->dep_ptr[sh->nf], *P);
     const size_t nt = (size_t)sh->nf * P->ntau;
-    const size_t rs = (P->precision == ATPM_FP64) ? 8 : 4;
-    // transient peak: geometry (hp, hm, nrm, dist) or scattering work
-    const size_t geo = (size_t)sh->nv * P->ntau * 24 + nt * 56 + (size_t)P->ntau * 16;
-    const size_t sct = 3 * (nt + 4 * (size_t)sh->nf) * rs;
+    // transient peak: geometry, scattering work or the shadow flags' staging
+    const bool shadows = wants_shadows(*P, sh->dep_ptr[sh->nf]), cull = shadows && shadow_cull_enabled();
+    const size_t geo = geometry_sizes(sh->nv, P->ntau, cull).total +
+                       (cull ? shadow_scratch_bytes(sh->nf, P->ntau, P->shadowing == 2) : shadows ? plain_sizes(nt) : 0);
+    DevSolve d{};
+    d.nf = sh->nf;
+    d.ntau = P->ntau;
+    d.mode = P->precision;
+    const size_t sct = std::max(scattering_work_bytes(d, P->multiple_scattering != 0), align256(nt * 4));
     // FAST with self-heating: this solve's BF16 W tiles (hi + lo; the view-
     // factor tiles are shared with the solve it is cloned from)
     size_t wb = 0;
@@ -1337,25 +1360,23 @@ ATPM_API atpm_status atpm_geometry_shadow(atpm_solve* s) {
     g.vsplit = s->sec_vertex >= 0 ? s->sec_vertex : s->nv;
     if (s->has_position)
         for (int k = 0; k < 3; ++k) g.car[k] = s->position[k];
-    const size_t nt = (size_t)s->nf * ntau, nvt = (size_t)s->nv * ntau;
+    const size_t nt = (size_t)s->nf * ntau;
     // shadow drivers: through the central projection (the same flags);
     // ATPM_SHADOW_CULL=0 runs the plain drivers
-    const bool shadows = (P.shadowing == 1 && s->nnz > 0) || P.shadowing == 2;
-    const bool cull = shadows && shadow_cull_enabled();
-    const size_t b_hp = align256(nvt * 24), b_rot = align256((size_t)ntau * 32), b_uv = cull ? align256(nvt * 8) : 0,
-                 b_w = cull ? align256(nvt * 4) : 0;
+    const bool shadows = wants_shadows(P, s->nnz), cull = shadows && shadow_cull_enabled();
+    const GeomSizes z = geometry_sizes(s->nv, ntau, cull);
     void *tmp = nullptr, *arrays = nullptr;
-    CK(cudaMallocAsync(&tmp, b_hp + b_rot + b_uv + b_w + 256 + 64 * 8, s->st));
+    CK(cudaMallocAsync(&tmp, z.total, s->st));
     char* t = static_cast<char*>(tmp);
     g.hp = reinterpret_cast<double*>(t);
-    g.rot = reinterpret_cast<double*>(t + b_hp);
-    t += b_hp + b_rot;
+    g.rot = reinterpret_cast<double*>(t + z.hp);
+    t += z.hp + z.rot;
     if (cull) {
         g.uv = t;
-        g.depth = reinterpret_cast<float*>(t + b_uv);
+        g.depth = reinterpret_cast<float*>(t + z.uv);
     }
-    g.stats = reinterpret_cast<unsigned*>(t + b_uv + b_w);
-    g.tests = reinterpret_cast<unsigned long long*>(t + b_uv + b_w + 256);
+    g.stats = reinterpret_cast<unsigned*>(t + z.uv + z.depth);
+    g.tests = reinterpret_cast<unsigned long long*>(t + z.uv + z.depth + 256);
     CK(cudaMemsetAsync(g.tests, 0, 64 * 8, s->st));
     g.rot2 = g.rot + 2 * (size_t)ntau;
     cudaError_t e = cudaMemcpyAsync((void*)g.rot, rot.data(), rot.size() * 8, cudaMemcpyHostToDevice, s->st);
@@ -1373,7 +1394,7 @@ ATPM_API atpm_status atpm_geometry_shadow(atpm_solve* s) {
         if (!culled) {
             rc = 0;
             const size_t b_v = align256(nt * 24);
-            e = cudaMallocAsync(&arrays, 2 * b_v + align256(nt * 8), s->st);
+            e = cudaMallocAsync(&arrays, plain_sizes(nt), s->st);
             if (e == cudaSuccess) {
                 char* p = static_cast<char*>(arrays);
                 g.hm = reinterpret_cast<double*>(p);

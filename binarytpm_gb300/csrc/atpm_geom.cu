@@ -62,7 +62,7 @@ struct GeomArgs {
 // to it, coordinates in km at the body's distance
 struct Proj {
     float c[3], e1[3], e2[3];
-    float scale;      // distance of the body centre
+    float scale, inv; // distance of the body centre, and 1 over it
     float pad;        // box padding (km)
     float margin;     // beyond this from a decision FP32 decides (km)
     float lift;       // most a midpoint's distance exceeds the body's and its depth (km)
@@ -354,11 +354,11 @@ __device__ __forceinline__ Tri load_tri(const GeomArgs& a, const Proj& p, int f,
 // itself leave them by the square of the body's size over the distance, which an
 // observer close by would need a margin of whole facets for.
 __device__ __forceinline__ Mid middle(const Proj& p, const Tri& t) {
-    const float inv = 1.0f / p.scale, p0 = 1.0f + t.w0 * inv, p1 = 1.0f + t.w1 * inv, p2 = 1.0f + t.w2 * inv;
-    const float m = 1.0f / (p0 + p1 + p2), w = (t.w0 + t.w1 + t.w2) * (1.0f / 3.0f);
+    const float p0 = 1.0f + t.w0 * p.inv, p1 = 1.0f + t.w1 * p.inv, p2 = 1.0f + t.w2 * p.inv;
+    const float m = __fdividef(1.0f, p0 + p1 + p2), w = (t.w0 + t.w1 + t.w2) * (1.0f / 3.0f);
     const float x = (t.q0.x * p0 + t.q1.x * p1 + t.q2.x * p2) * m, y = (t.q0.y * p0 + t.q1.y * p1 + t.q2.y * p2) * m;
-    const float u = x * inv, v = y * inv, sq = u * u + v * v;
-    return {make_float2(x, y), w + (p.scale + w) * (sq / (1.0f + sqrtf(1.0f + sq)))};
+    const float u = x * p.inv, v = y * p.inv, sq = u * u + v * v;
+    return {make_float2(x, y), w + (p.scale + w) * __fdividef(sq, 1.0f + sqrtf(1.0f + sq))};
 }
 
 __device__ __forceinline__ float4 tri_box(const Tri& t, float pad) {
@@ -674,6 +674,7 @@ bool make_frame(const GeomWork& g, Proj& p) {
         p.e2[k] = (float)e2[k];
     }
     p.scale = (float)n;
+    p.inv = (float)(1.0 / n);
     p.uv = reinterpret_cast<float2*>(g.uv);
     p.w = g.depth;
     p.stats = g.stats;
@@ -681,7 +682,24 @@ bool make_frame(const GeomWork& g, Proj& p) {
 }
 
 size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
+
+constexpr int kMaxGrid = 2048;  // cells a side
+// a step of the all-pairs grid of n cells: entries, corners, midpoints; the cells
+size_t grid_step_bytes(size_t nf, size_t n) {
+    return nf * (kCover * sizeof(int) + 2 * sizeof(float4) + sizeof(float2)) + (2 * n + 1) * sizeof(int);
+}
+// What the grid may take at once, in chunks of steps: all of it for a few cells a
+// facet, up to 1.5 GB (21,760 facets x 720 steps take 1.3 GB; in three chunks of
+// 512 MB they take 1 % longer), one step at least.
+size_t grid_budget(int nf, int ntau) {
+    const size_t all = (size_t)ntau * grid_step_bytes(nf, 4 * (size_t)nf) + (64u << 20);
+    return std::max(std::min<size_t>(all, 1536u << 20), grid_step_bytes(nf, (size_t)kMaxGrid * kMaxGrid));
+}
 }  // namespace
+
+size_t shadow_scratch_bytes(int nf, int ntau, bool all_pairs) {
+    return all_pairs ? grid_budget(nf, ntau) + 5 * 256 : al256((size_t)((ntau + 31) / 32) * nf * sizeof(float4));
+}
 
 // returns 0 when the culled driver ran, -1 when the caller should fall back
 int launch_shadow_culled(const DevSolve& s, const GeomWork& g, bool all_pairs, stream_t stv) {
@@ -733,15 +751,13 @@ int launch_shadow_culled(const DevSolve& s, const GeomWork& g, bool all_pairs, s
         gr.cell = 0.75f * ext + 1e-6f;
         gr.origin = -(umax + 2.0f * p.pad) - gr.cell;
         long long G = (long long)ceilf(2.0f * -gr.origin / gr.cell) + 1;
-        if (G > 2048) {  // a few huge facets: coarser cells, still correct
-            G = 2048;
+        if (G > kMaxGrid) {  // a few huge facets: coarser cells, still correct
+            G = kMaxGrid;
             gr.cell = 2.0f * -gr.origin / 2000.0f;
         }
         gr.G = (int)G;
         const size_t n = (size_t)G * G, entries = (size_t)kCover * s.nf;
-        // steps per chunk: at most ~64 M cells and 1 GB of entries at once
-        const int sc = (int)std::max<size_t>(
-            1, std::min<size_t>((size_t)s.ntau, std::min<size_t>((64u << 20) / (n + 1), (1u << 30) / (entries * 4))));
+        const int sc = (int)std::max<size_t>(1, std::min<size_t>(s.ntau, grid_budget(s.nf, s.ntau) / grid_step_bytes(s.nf, n)));
         const size_t b_st = al256((size_t)sc * (n + 1) * 4), b_cu = al256((size_t)sc * n * 4),
                      b_tri = al256((size_t)sc * s.nf * 2 * sizeof(float4)), b_who = al256(sc * entries * 4),
                      b_mid = al256((size_t)sc * s.nf * sizeof(float2));

@@ -244,6 +244,7 @@ int launch_shadow_allpairs(const DevSolve& s, const GeomWork& g, stream_t st);
 // pairs over a per-step grid); -1: not applicable (body too close to the
 // origin for a central projection), use the above
 int launch_shadow_culled(const DevSolve& s, const GeomWork& g, bool all_pairs, stream_t st);
+size_t shadow_scratch_bytes(int nf, int ntau, bool all_pairs);  // most it allocates
 
 // scattering (atpm_scatter.cu)
 size_t scattering_work_bytes(const DevSolve& s, bool multiple);
