@@ -683,17 +683,22 @@ bool make_frame(const GeomWork& g, Proj& p) {
 
 size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-constexpr int kMaxGrid = 2048;  // cells a side
+// Most cells of a step's grid.  Two small bodies far apart would have millions of
+// empty ones to clear and scan, one block a step: with a cell for every three
+// quarters of the largest box 2,560 facets x 720 steps took 94 ms at 40 km apart
+// and 294 at 400; with the cells kept to a few a facet 3.2 and 4.4 (8 a facet 3.2
+// and 4.2, but 0.81 against 0.71 at 2.5 km; 4 a facet 4.0 and 5.4).
+size_t most_cells(size_t nf) { return 12 * nf + 4096; }
 // a step of the all-pairs grid of n cells: entries, corners, midpoints; the cells
 size_t grid_step_bytes(size_t nf, size_t n) {
     return nf * (kCover * sizeof(int) + 2 * sizeof(float4) + sizeof(float2)) + (2 * n + 1) * sizeof(int);
 }
-// What the grid may take at once, in chunks of steps: all of it for a few cells a
-// facet, up to 1.5 GB (21,760 facets x 720 steps take 1.3 GB; in three chunks of
-// 512 MB they take 1 % longer), one step at least.
+// What the grid may take at once, in chunks of steps: up to 1.5 GB (21,760 facets x
+// 720 steps take 1.3 GB; in three chunks of 512 MB they take 1 % longer), one step
+// at least.
 size_t grid_budget(int nf, int ntau) {
-    const size_t all = (size_t)ntau * grid_step_bytes(nf, 4 * (size_t)nf) + (64u << 20);
-    return std::max(std::min<size_t>(all, 1536u << 20), grid_step_bytes(nf, (size_t)kMaxGrid * kMaxGrid));
+    const size_t all = (size_t)ntau * grid_step_bytes(nf, most_cells(nf) / 3);
+    return std::max(std::min<size_t>(all, 1536u << 20), grid_step_bytes(nf, most_cells(nf)));
 }
 }  // namespace
 
@@ -750,10 +755,11 @@ int launch_shadow_culled(const DevSolve& s, const GeomWork& g, bool all_pairs, s
         GridArgs gr{};
         gr.cell = 0.75f * ext + 1e-6f;
         gr.origin = -(umax + 2.0f * p.pad) - gr.cell;
+        const int most = (int)sqrt((double)most_cells(s.nf));
         long long G = (long long)ceilf(2.0f * -gr.origin / gr.cell) + 1;
-        if (G > kMaxGrid) {  // a few huge facets: coarser cells, still correct
-            G = kMaxGrid;
-            gr.cell = 2.0f * -gr.origin / 2000.0f;
+        if (G > most) {  // coarser cells: a box touches fewer of them
+            G = most;
+            gr.cell = 2.0f * -gr.origin / (float)(most - 2);
         }
         gr.G = (int)G;
         const size_t n = (size_t)G * G, entries = (size_t)kCover * s.nf;
