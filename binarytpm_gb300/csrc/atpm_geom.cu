@@ -73,12 +73,16 @@ struct Proj {
     float4* wbox;     // [windows][nf] union of each facet's padded boxes over 32 steps (or null)
 };
 
-__device__ __forceinline__ unsigned warp_max(unsigned v) { return __reduce_max_sync(__activemask(), v); }
+// the largest of the warp's values, every lane taking part, into *to
+__device__ __forceinline__ void warp_max_to(unsigned* to, unsigned v) {
+    const unsigned most = __reduce_max_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && most > __ldcg(to)) atomicMax(to, most);
+}
 
 __global__ void __launch_bounds__(256) k_geom_vertices(GeomArgs a, Proj p) {
     const int nv = a.s.nv, ntau = a.s.ntau;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)nv * ntau) return;
+    const long long n = (long long)nv * ntau, at = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = at < n ? at : n - 1;  // lanes beyond the end repeat the last vertex
     const int v = (int)(i / ntau), s = (int)(i % ntau);
     const double* e = a.s.vert + 3 * v;
     // a non-synchronous secondary turns at its own rate (its own table)
@@ -103,17 +107,13 @@ __global__ void __launch_bounds__(256) k_geom_vertices(GeomArgs a, Proj p) {
     const float x = ef[0] * p.e1[0] + ef[1] * p.e1[1] + ef[2] * p.e1[2];
     const float y = ef[0] * p.e2[0] + ef[1] * p.e2[1] + ef[2] * p.e2[2];
     const float d = p.scale + w;
-    if (!(d > 0.5f * sqrtf(d * d + x * x + y * y))) { atomicOr(&p.stats[2], 1u); return; }
+    if (!(d > 0.5f * sqrtf(d * d + x * x + y * y))) atomicOr(&p.stats[2], 1u);  // the projection is not used
     const float m = 1.0f / (1.0f + w / p.scale), u = x * m, t = y * m;
     p.uv[i] = make_float2(u, t);
     p.w[i] = w;
-    const unsigned lat = warp_max(__float_as_uint(fmaxf(fabsf(u), fabsf(t)))), dep = warp_max(__float_as_uint(fabsf(w))),
-                   front = warp_max(__float_as_uint(fmaxf(-w, 0.0f)));
-    if ((threadIdx.x & 31) == (unsigned)(__ffs(__activemask()) - 1)) {
-        if (lat > __ldcg(&p.stats[0])) atomicMax(&p.stats[0], lat);
-        if (dep > __ldcg(&p.stats[3])) atomicMax(&p.stats[3], dep);
-        if (front > __ldcg(&p.stats[4])) atomicMax(&p.stats[4], front);
-    }
+    warp_max_to(&p.stats[0], __float_as_uint(fmaxf(fabsf(u), fabsf(t))));
+    warp_max_to(&p.stats[3], __float_as_uint(fabsf(w)));
+    warp_max_to(&p.stats[4], __float_as_uint(fmaxf(-w, 0.0f)));
 }
 
 // a facet's midpoint, unit normal and the midpoint's distance at one step, in
@@ -509,12 +509,10 @@ __device__ __forceinline__ int cell_of(const GridArgs& gr, float x) {
 
 __global__ void __launch_bounds__(256) k_grid_extent(GeomArgs a, Proj p) {
     const int ntau = a.s.ntau;
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)a.s.nf * ntau) return;
+    const long long n = (long long)a.s.nf * ntau, at = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long i = at < n ? at : n - 1;  // lanes beyond the end repeat the last facet
     const float4 b = tri_box(load_tri(a, p, (int)(i / ntau), (int)(i % ntau)), p.pad);
-    const unsigned m = warp_max(__float_as_uint(fmaxf(b.y - b.x, b.w - b.z)));
-    if ((threadIdx.x & 31) == (unsigned)(__ffs(__activemask()) - 1) && m > __ldcg(&p.stats[1]))
-        atomicMax(&p.stats[1], m);
+    warp_max_to(&p.stats[1], __float_as_uint(fmaxf(b.y - b.x, b.w - b.z)));
 }
 
 // the cells a box touches, in turn
