@@ -1382,7 +1382,7 @@ ATPM_API atpm_status atpm_geometry_shadow(atpm_solve* s) {
     cudaError_t e = cudaMemcpyAsync((void*)g.rot, rot.data(), rot.size() * 8, cudaMemcpyHostToDevice, s->st);
     int rc = 0;
     if (e == cudaSuccess) rc = launch_geometry(s->ds, g, s->st);
-    // the shadow drivers' time (events) and exact-test count (culled drivers)
+    // the shadow drivers' time (events) and triangle-test count (culled drivers)
     cudaEvent_t sh0 = nullptr, sh1 = nullptr;
     unsigned long long counts[64] = {};
     bool culled = false;

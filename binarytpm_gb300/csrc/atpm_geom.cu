@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(256) k_window_box(GeomArgs a, Proj p) {
     if (threadIdx.x == 0) p.wbox[(size_t)blockIdx.x * a.s.nf + h] = u;
 }
 
-// adds a thread's exact-test count to the launch's tally: one add per group
+// adds a thread's triangle-test count to the launch's tally: one add per group
 // of lanes leaving together, spread over 64 counters
 __device__ __forceinline__ void count_tests(unsigned long long* ctr, unsigned n) {
     if (!ctr) return;

@@ -437,7 +437,7 @@ class Solve:
         return float(v.value)
 
     def last_shadow_stats(self):
-        """(device ms, rays, exact ray-triangle tests or -1) of the last
+        """(device ms, rays, ray-triangle tests or -1) of the last
         geometry_shadow's shadow drivers."""
         ms, r, t = C.c_double(), C.c_int64(), C.c_int64()
         _ck(load().atpm_last_shadow_stats(self.h, C.byref(ms), C.byref(r), C.byref(t)))
