@@ -1067,6 +1067,10 @@ extern "C++" void atpm_context_release(atpm_context* c) {
     if (c->p4.slots_dev) cudaFree(c->p4.slots_dev);
     if (c->p3.slots_dev) cudaFree(c->p3.slots_dev);
     if (c->pq.slots_dev) cudaFree(c->pq.slots_dev);
+    // what released solves left in the pool goes back to the device (another
+    // context's next solve maps it anew)
+    cudaMemPool_t pool = nullptr;
+    if (cudaDeviceGetDefaultMemPool(&pool, c->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
     delete c;
 }
 

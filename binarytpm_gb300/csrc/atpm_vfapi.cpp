@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstdio>
 #include <vector>
 
@@ -34,6 +35,26 @@ void set_last_error(const char* msg);
 }  // namespace atpm
 
 namespace {
+// What a call leaves in the stream-ordered pool beyond what the pool held before
+// is bounded: the candidates of a large shape take gigabytes, which the context's
+// release threshold would keep from the rest of the process for good.
+struct PoolGrowth {
+    static constexpr uint64_t kKeep = 512ull << 20;
+    cudaMemPool_t pool = nullptr;
+    uint64_t before = 0;
+    PoolGrowth() {
+        int device = 0;
+        if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetMemPool(&pool, device) != cudaSuccess ||
+            cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &before) != cudaSuccess)
+            pool = nullptr;
+    }
+    ~PoolGrowth() {  // after the buffers' own destructors
+        uint64_t now = 0;
+        if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &now) == cudaSuccess &&
+            now > before + kKeep && cudaStreamSynchronize(0) == cudaSuccess)
+            cudaMemPoolTrimTo(pool, before + kKeep);
+    }
+};
 // device memory from the stream-ordered pool (kept by the context's release
 // threshold from call to call), given back with its owner
 struct DevBufs {
@@ -94,6 +115,7 @@ ATPM_API atpm_status atpm_viewfactors_compute(atpm_context* ctx, int32_t nv, int
     float size = 0.0f;  // the largest coordinate: the scale of the positions' rounding
     for (int i = 0; i < 3 * nv; ++i) size = std::max(size, std::fabs(vertices[i]));
     cudaStream_t st = 0;
+    PoolGrowth growth;
     DevBufs B;
     atpm::VfGeom g{};
     g.nv = nv;
