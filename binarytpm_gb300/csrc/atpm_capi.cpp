@@ -40,6 +40,7 @@ atpm_status fail(atpm_status s, const char* fmt, ...) {
     va_start(ap, fmt);
     std::vsnprintf(buf, sizeof(buf), fmt, ap);
     va_end(ap);
+    cudaGetLastError();  // reported here: the next call's launches must not find it again
     g_err = buf;
     return s;
 }
@@ -883,6 +884,7 @@ extern "C" void wire_arena(atpm_solve* s, const Layout& L);
 namespace atpm {
 void set_last_error(const char* msg) { g_err = msg; }
 atpm_status fail_status(atpm_status s, const char* msg) {
+    cudaGetLastError();
     g_err = msg;
     return s;
 }

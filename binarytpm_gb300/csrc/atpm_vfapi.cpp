@@ -83,6 +83,7 @@ struct OnDevice {
 };
 atpm_status vfail(atpm_status s, const char* what, cudaError_t e) {
     char buf[256];
+    cudaGetLastError();
     std::snprintf(buf, sizeof buf, "viewfactors: %s: %s", what, cudaGetErrorString(e));
     atpm::set_last_error(buf);
     return s;

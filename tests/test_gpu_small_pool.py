@@ -131,3 +131,19 @@ def test_disk_flux_a_few_steps_at_a_time(gpu_ctx, flags):
     assert np.array_equal(got, want)
     assert (want > 0).all()
     s.close()
+
+
+@pytest.mark.parametrize("failing", ["scattering", "viewfactors"])
+def test_a_failed_allocation_fails_one_call(gpu_ctx, failing):
+    from binarytpm_gb300 import lib, problem
+
+    s = lib.Solve(gpu_ctx, _problem(shadowing=0, albedo=0.3), precision=0)
+    s.geometry_shadow()
+    v, f = problem.binary_mesh(4, 3, 2)
+    call = {"scattering": s.scattering, "viewfactors": lambda: lib.viewfactors(gpu_ctx, v, f)}[failing]
+    with _room(256 << 10):
+        with pytest.raises(lib.AtpmError):
+            call()
+    s.geometry_shadow()  # what failed is not found again by the next launches
+    call()
+    s.close()
