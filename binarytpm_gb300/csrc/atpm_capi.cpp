@@ -18,6 +18,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <new>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -551,8 +552,9 @@ atpm_status build_tc(atpm_solve* s, const atpm_shape* sh) {
 
 // the Gauss-Seidel order of the solve's lists, once per shape (a host pass
 // over the list entries below each row's facet: 0.4 ms for 5,440 facets and
-// 0.7 M entries)
-atpm_status ensure_gs_plan(atpm_solve* s) {
+// 0.7 M entries).  Without memory for it, here or on the device, there is no plan
+// and the sweeps go facet by facet.
+atpm_status ensure_gs_plan(atpm_solve* s) try {
     if (s->gs || s->P.precision == ATPM_FAST || s->nnz == 0 || (size_t)s->nf * s->rs > kGsSharedBytes) return ATPM_OK;
     const int nf = s->nf;
     std::vector<int> ptr(nf + 1), idx(s->nnz), mid(nf), level(nf, -1);
@@ -584,7 +586,12 @@ atpm_status ensure_gs_plan(atpm_solve* s) {
         for (int c = 0; c < nf; ++c)
             if (level[c] >= 0) rows[at[level[c]]++] = make_int4(c, ptr[c], mid[c], 0);
         const size_t b_rows = align256(rows.size() * sizeof(int4)), b_off = align256(off.size() * 4);
-        CK(pool_alloc(&gs->mem, b_rows + b_off + (size_t)nf * 4, s->st));
+        const cudaError_t ea = pool_alloc(&gs->mem, b_rows + b_off + (size_t)nf * 4, s->st);
+        if (ea == cudaErrorMemoryAllocation) {
+            cudaGetLastError();
+            return ATPM_OK;
+        }
+        if (ea != cudaSuccess) return fail(ATPM_E_CUDA, "Gauss-Seidel order: %s", cudaGetErrorString(ea));
         char* m = static_cast<char*>(gs->mem);
         CK(cudaMemcpyAsync(m, rows.data(), rows.size() * sizeof(int4), cudaMemcpyHostToDevice, s->st));
         CK(cudaMemcpyAsync(m + b_rows, off.data(), off.size() * 4, cudaMemcpyHostToDevice, s->st));
@@ -597,6 +604,8 @@ atpm_status ensure_gs_plan(atpm_solve* s) {
         gs->plan.listed = (int)rows.size();
     }
     s->gs = gs;
+    return ATPM_OK;
+} catch (const std::bad_alloc&) {
     return ATPM_OK;
 }
 
@@ -1482,14 +1491,17 @@ ATPM_API atpm_status atpm_scattering(atpm_solve* s) {
     if (!s) return fail(ATPM_E_INVALID, "null solve");
     CK(cudaSetDevice(s->ctx->device));
     const bool multiple = s->P.multiple_scattering != 0;
-    if (multiple) {
-        atpm_status rp = ensure_gs_plan(s);
-        if (rp) return rp;
-    }
     void* work = nullptr;
     const cudaError_t ea = cudaMallocAsync(&work, scattering_work_bytes(s->ds, multiple), s->st);
     if (ea == cudaErrorMemoryAllocation && !multiple) cudaGetLastError();  // single scattering needs none
-    else CK(ea);
+    else if (ea != cudaSuccess) return fail(ATPM_E_CUDA, "scattering work: %s", cudaGetErrorString(ea));
+    if (multiple) {
+        atpm_status rp = ensure_gs_plan(s);
+        if (rp) {
+            cudaFreeAsync(work, s->st);
+            return rp;
+        }
+    }
     int rc = launch_single_scattering(s->ds, work, multiple, s->st);
     const char* what = "single scattering launch";
     if (!rc && multiple) {
@@ -1848,7 +1860,7 @@ ATPM_API atpm_status atpm_get_shadow(atpm_solve* s, int32_t* out) {
         }
         return ATPM_OK;
     }
-    CK(e);
+    if (e != cudaSuccess) return fail(ATPM_E_CUDA, "shadow flags: %s", cudaGetErrorString(e));
     if (launch_widen_flags(s->ds.shadow, static_cast<int32_t*>(tmp), nt, s->st)) e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, tmp, nt * 4, cudaMemcpyDeviceToHost, s->st);
     cudaFreeAsync(tmp, s->st);
@@ -2063,7 +2075,8 @@ atpm_status disk_flux_impl(atpm_solve* s, const double* observer, const int32_t*
         b_flags = visibility ? align256((size_t)nf * ns * 4) : 0;
         const cudaError_t ea = cudaMallocAsync(&tmp, b_rot + b_part + b_out + b_vis + b_flags + b_geo + b_hp + b_area, s->st);
         if (ea == cudaSuccess) break;
-        if (ea != cudaErrorMemoryAllocation || ns == 1) CK(ea);
+        if (ea != cudaErrorMemoryAllocation || ns == 1)
+            return fail(ATPM_E_CUDA, "disk_flux work: %s", cudaGetErrorString(ea));
         cudaGetLastError();
     }
     char* t = static_cast<char*>(tmp);

@@ -133,6 +133,20 @@ def test_disk_flux_a_few_steps_at_a_time(gpu_ctx, flags):
     s.close()
 
 
+def test_gauss_seidel_without_its_order(gpu_ctx):
+    from binarytpm_gb300 import lib
+
+    got = []
+    for size in (GRANULE // 2, 1_900_000):  # the sweeps take 1.80 MB, the level order 0.23
+        s = lib.Solve(gpu_ctx, _problem(50000, 1, shadowing=0, albedo=0.3), precision=0)
+        s.geometry_shadow()
+        with _room(size):
+            s.scattering()
+        got.append(s.illumination())
+        s.close()
+    assert np.array_equal(got[0], got[1], equal_nan=True)
+
+
 @pytest.mark.parametrize("failing", ["scattering", "viewfactors"])
 def test_a_failed_allocation_fails_one_call(gpu_ctx, failing):
     from binarytpm_gb300 import lib, problem
