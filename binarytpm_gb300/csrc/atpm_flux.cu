@@ -223,27 +223,29 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux_partial(DevSolve s, FluxA
         // (wise_main.cpp:718)
         view[threadIdx.x][3] = weight;
         __syncwarp();
-        for (int i = 0; i < 32; ++i) {
+        // the warp's facets end to end, so that few sub-facets leave no lane idle
+        int i = lane / a.nsf, j = lane % a.nsf;
+        for (; i < 32; j += 32) {
+            for (; j >= a.nsf; j -= a.nsf) ++i;
+            if (i >= 32) break;
             const double* v = view[warp * 32 + i];
             if (v[3] == 0.0) continue;
             const int facet = blockIdx.x * kFluxThreads + warp * 32 + i;
-            const size_t base = ((size_t)facet * s.ntau + step) * (size_t)a.nsf;
-            for (int j = lane; j < a.nsf; j += 32) {
-                const double vis = (double)a.sub_vis[base + j];
-                const double* g = a.sub_geo + 4 * j;
-                double c = v[0] * g[0] + v[1] * g[1] + v[2] * g[2];
-                if (!(vis > 0.0)) continue;
-                if (fabs(c) > 1.0 - kSure) {  // the stage's acos of a ratio above 1 is NaN: no term
-                    double w[3], d;
-                    stage_view(s, a, facet, step, w, d);
-                    c = __ddiv_rn(dot3(w, g), d);
-                }
-                if (!(fabs(c) <= 1.0)) continue;
-                const double m = v[3] * g[3] * vis * c, inv_t = 1.0 / (double)a.sub_T[base + j];
-#pragma unroll
-                for (int l = 0; l < kMaxFluxWavelengths; ++l)
-                    if (l < a.nwl) term[l] += planck(a, l, inv_t) * m;
+            const size_t at = ((size_t)facet * s.ntau + step) * (size_t)a.nsf + j;
+            const double vis = (double)a.sub_vis[at];
+            const double* g = a.sub_geo + 4 * j;
+            double c = v[0] * g[0] + v[1] * g[1] + v[2] * g[2];
+            if (!(vis > 0.0)) continue;
+            if (fabs(c) > 1.0 - kSure) {  // the stage's acos of a ratio above 1 is NaN: no term
+                double w[3], d;
+                stage_view(s, a, facet, step, w, d);
+                c = __ddiv_rn(dot3(w, g), d);
             }
+            if (!(fabs(c) <= 1.0)) continue;
+            const double m = v[3] * g[3] * vis * c, inv_t = 1.0 / (double)a.sub_T[at];
+#pragma unroll
+            for (int l = 0; l < kMaxFluxWavelengths; ++l)
+                if (l < a.nwl) term[l] += planck(a, l, inv_t) * m;
         }
     }
 #pragma unroll
