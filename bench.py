@@ -551,7 +551,7 @@ def main():
         "batched_sweep": sweep,
         "visibility": vis,
         "energy_balance_fp64": energy,
-        "kernels_ms": kern,
+        "kernels_ms": {k: v for k, v in kern.items() if v["ms"] > 0.0},
         "launch_config": launch_config,
         "wall_clock_value": wall_value, "setup_s": setup_s, "nnz_viewfactors": int(prob.nnz),
         "revolutions_per_solve": nrevs[-1],
@@ -863,7 +863,7 @@ FP64_TI = [200.0, 2000.0]
 CONV_ERR_TI = [200.0, 2000.0]
 # executed instructions per facet-step of the FAST sweep by conduction
 # variant (ncu: profiles/conduction_and_spmm_binary_s4s3_fast.md for the
-# scalar k_conduction<FAST,56>, profiles/conduction_pairs_binary_s4s3_8solves.md
+# scalar k_conduction<56>, profiles/conduction_pairs_binary_s4s3_8solves.md
 # for the paired k_conduction_pairs<56>)
 COND_INSTR_PER_FACET_STEP = {1: 327, 2: 327, 3: 327, 4: 188}
 COND_KERNEL = {1: "k_conduction<56,1>", 2: "k_conduction<56,2>", 3: "k_conduction<56,3>",

@@ -385,7 +385,7 @@ void build_tc_items(atpm_solve* const* solves, int n, std::vector<int4>& q) {
 }
 
 // device layout of a batch's tensor-core map: the nq items, then room for the
-// per-launch list of active items (nq), then the two work counters
+// per-launch list of active items (nq), then the three work words
 size_t tc_map_entries(size_t nq) { return nq ? 2 * nq + 1 : 0; }
 void tc_map_extend(std::vector<int4>& q) {
     const size_t nq = q.size();
@@ -631,9 +631,8 @@ Batch make_batch(atpm_context* ctx, const DevSolve* tab, int n, const int4* wm, 
     b.cond_variant = cond_variant();
     b.tc_stages = 0;
     b.warp_tail = warp_tail_enabled() ? 1 : 0;
-    // active facets of the whole batch up to which a revolution runs warp per
-    // facet: about a dozen warps per SM, where one warp per facet still beats
-    // the thread-per-facet sweep's latency-bound last warps
+    // advancing facets of the whole batch up to which a revolution runs with 16
+    // and with 4 lanes a facet (warp_tail_per_sm, kFewPerSm)
     b.tail_limit = warp_tail_per_sm() * ctx->sm_count;
     b.few_limit = std::max(b.tail_limit, kFewPerSm * ctx->sm_count);
     b.sms = ctx->sm_count;
@@ -2254,20 +2253,21 @@ ATPM_API atpm_status atpm_profile_revolution(atpm_solve* const* solves, int32_t 
     void* tmp = nullptr;
     atpm_status rb = make_batch_for(solves, n, &b, &tmp);
     if (rb) return rb;
-    cudaEvent_t ev[6];
-    for (int k = 0; k < 6; ++k) CK(cudaEventCreate(&ev[k]));
+    cudaEvent_t ev[kRevolutionParts + 1];
+    for (cudaEvent_t& x : ev) CK(cudaEventCreate(&x));
     cudaError_t e = cudaEventRecord(ev[0], s0->st);
-    for (int part = 0; part < 5 && e == cudaSuccess; ++part) {
+    for (int part = 0; part < kRevolutionParts && e == cudaSuccess; ++part) {
         if (launch_revolution_part(b, part, s0->st)) e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaEventRecord(ev[part + 1], s0->st);
     }
-    if (e == cudaSuccess) e = cudaEventSynchronize(ev[5]);
-    for (int k = 0; k < 5 && e == cudaSuccess; ++k) {
+    if (e == cudaSuccess) e = cudaEventSynchronize(ev[kRevolutionParts]);
+    for (int k = 0; k < kRevolutionParts && e == cudaSuccess; ++k) {
         float ms = 0.0f;
         e = cudaEventElapsedTime(&ms, ev[k], ev[k + 1]);
         kernel_ms[k] = ms;
     }
-    for (int k = 0; k < 6; ++k) cudaEventDestroy(ev[k]);
+    kernel_ms[kRevolutionParts] = 0.0;  // the advance: the convergence kernel's last block
+    for (cudaEvent_t x : ev) cudaEventDestroy(x);
     if (tmp) cudaFree(tmp);
     if (e != cudaSuccess) return fail(ATPM_E_CUDA, "profile: %s", cudaGetErrorString(e));
     if (facet_steps) *facet_steps = fs;

@@ -75,7 +75,7 @@ template <int MODE> struct Sc {
 
 // FAST arithmetic is written with explicitly rounded operations (the _rn
 // intrinsics are never contracted into a multiply-add), so the scalar, the
-// warp-per-facet and the paired forms of the sweep round alike, operation by
+// lane-split and the paired forms of the sweep round alike, operation by
 // operation, whatever the compiler schedules.
 // eps sigma T^4 (with the IR absorptivity folded into es_w)
 __device__ __forceinline__ float fast_w(float es_w, float t) {
@@ -118,7 +118,7 @@ struct WOut {
 };
 
 // One FTCS node update and one Newton step of the FAST sweep, shared by the
-// thread-per-facet and the warp-per-facet forms so both round alike.
+// thread-per-facet and the lane-split forms so both round alike.
 // (up + dn) - 2 t is formed as one fma: 2 t is exact, so this is the
 // rounding of the plain expression
 __device__ __forceinline__ float ftcs_node(float r, float up, float dn, float t) {

@@ -317,7 +317,8 @@ int launch_rem_fill(const DevSolve& s, int nkb, const int* slot, const int* rptr
 int launch_tc_rowneed(const DevSolve& s, int nkb, unsigned* need, stream_t st);
 int launch_tc_fill(const DevSolve& s, int nkb, const int* slot, const int* lo_of, void* tiles, void* lo_tiles,
                    stream_t st);
-// part 0 preparation and W, 1 Q, 2 conduction, 3 convergence and advance (4: none)
+// part 0 preparation and W, 1 Q, 2 conduction, 3 convergence and advance
+constexpr int kRevolutionParts = 4;
 int launch_revolution_part(const Batch& b, int part, stream_t st);
 // REFERENCE / FP64 conduction of one revolution (atpm_conduction_split.cu)
 int launch_conduction_split(const Batch& b, stream_t st);

@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(128, MINB) k_conduction(Batch b) {
 }
 
 // FAST conduction variant 4: the facet-range sweep (every revolution before
-// the active-list and warp-per-facet forms take over) as pairs of adjacent
+// the active list or the lane-split form takes over) as pairs of adjacent
 // facets, 64 threads per 128-facet block.  Only pairs with both facets
 // active are swept here: k_conduction, launched beside it, takes a facet
 // whose partner is frozen (the freeze flags do not change during the sweep),
@@ -862,7 +862,7 @@ static bool pairs_run(const Batch& b) { return b.cond_variant == 4 && !few_alway
 template <int MODE>
 static int launch_rev_part(const Batch& b, int part, cudaStream_t st) {
     if (MODE == MODE_FAST && part == 0) k_prepare<<<1, kPrepThreads, 0, st>>>(b);
-    // FAST + tensor cores: the conduction sweep keeps W current (store_w)
+    // FAST + tensor cores: the conduction sweep keeps W current
     if (MODE == MODE_FAST && b.nq > 0 && part == 0) return cudaGetLastError() == cudaSuccess ? 0 : 2;
     if (MODE == MODE_FAST && b.nq > 0 && part == 1) return launch_spmm_tc(b, st);
     switch (part) {
@@ -889,7 +889,6 @@ static int launch_rev_part(const Batch& b, int part, cudaStream_t st) {
             }
             return launch_conduction_few(b, st);
         case 3: k_converge<<<b.nfb, 128, 0, st>>>(b); break;
-        case 4: break;  // the end of the revolution: k_converge's last block
         default: return 1;
     }
     return cudaGetLastError() == cudaSuccess ? 0 : 2;
@@ -915,7 +914,7 @@ int kernels_per_revolution(const Batch& b) {
 }
 
 int launch_revolution(const Batch& b, stream_t st) {
-    for (int part = 0; part < 5; ++part) {
+    for (int part = 0; part < kRevolutionParts; ++part) {
         const int rc = launch_revolution_part(b, part, st);
         if (rc) return rc;
     }

@@ -514,6 +514,7 @@ def viewfactors(ctx: Context, vertices, facets, refine: bool = True):
     return ptr, idx, vf, vec, photo
 
 
+# "advance" is part of "converge" and reported as 0
 KERNEL_NAMES = ["selfheat_w", "selfheat_q", "conduction", "converge", "advance"]
 
 

@@ -174,8 +174,10 @@ ATPM_API atpm_status atpm_get_cosillum(atpm_solve* s, float* out);
  * (3905/Thermal/NominalPole/main.cpp:193, 303). */
 ATPM_API atpm_status atpm_get_converged(atpm_solve* s, uint8_t* out /* [nf] */);
 /* One revolution of the given (active) solves with a CUDA event between
- * kernels: kernel_ms[5] = self-heating W, self-heating Q, conduction,
- * convergence, advance.  Advances the solves by one revolution. */
+ * kernels: kernel_ms[5] = self-heating W (FAST: the revolution's
+ * preparation), self-heating Q, conduction, convergence with the end of the
+ * revolution, and 0 (the end was a kernel of its own).  Advances the solves by
+ * one revolution. */
 ATPM_API atpm_status atpm_profile_revolution(atpm_solve* const* solves, int32_t n, double* kernel_ms,
                                              int64_t* facet_steps, int64_t* active_facets);
 /* Self-heating flux Q[s][f] = sum_g V[f][g] eps sigma T_g[s]^4 for the
