@@ -2054,6 +2054,7 @@ atpm_status disk_flux_impl(atpm_solve* s, const double* observer, const int32_t*
     a.obs[1] = a.car[1] - (AUm * observer[0] * std::cos(observer[1]) * std::sin(observer[2]));
     a.obs[2] = a.car[2] - (AUm * observer[0] * std::sin(observer[1]));
     a.eps = emissivity;
+    a.close = P.polar[0] > 2.0 * observer[0];
     const double cvel = 299792458.0, hcon = 6.626068963e-34, kcon = 1.380650424e-23;
     a.nwl = nwl;
     for (int l = 0; l < nwl; ++l) {

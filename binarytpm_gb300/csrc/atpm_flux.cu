@@ -26,7 +26,7 @@
 // own units, so their rounding shows in the normals and, for an observer near the
 // body, in the view vector); from them on, cosines come from one reciprocal square
 // root instead of a facet frame, acos and cos, and a wavelength costs one exp and
-// one reciprocal: 13.0 -> 4.2 ms for 21,760 facets, 720 steps and three
+// one reciprocal: 13.0 -> 4.1 ms for 21,760 facets, 720 steps and three
 // wavelengths.  A cosine within kSure of 0 or 1 is the stage's to judge
 // (stage_view): there its rounding decides whether a facet or sub-facet counts.
 //
@@ -176,7 +176,7 @@ __global__ void __launch_bounds__(kFluxThreads) k_flux_partial(DevSolve s, FluxA
         const Facet t(s, a, f, step);
         double ov[3];  // from the facet to the observer
 #pragma unroll
-        for (int k = 0; k < 3; ++k) ov[k] = __dsub_rn(a.obs[k], third(t.sum[k]));
+        for (int k = 0; k < 3; ++k) ov[k] = __dsub_rn(a.obs[k], a.close ? third(t.sum[k]) : t.sum[k] * (1.0 / 3.0));
         const double oo = dot3(ov, ov), nn = dot3(t.n, t.n), no = dot3(t.n, ov);
         // cosine toward the observer; |cosine| < kSure by the exponents
         const bool edge_on = 2 * exponent(no) < exponent(nn) + exponent(oo) - 88;

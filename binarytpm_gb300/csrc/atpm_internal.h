@@ -337,6 +337,8 @@ struct FluxArgs {
     double car[3];           // body centre (km)
     double obs[3];           // observer (km)
     double eps;
+    bool close;              // midpoints rounded as the stage rounds them: they show in the view vector of an
+                             // observer much nearer than the origin (within 2e-16 of it from afar)
     int s0, ns;              // the steps of this launch
     const int32_t* flags;    // [nf][ns] visibility words, or null (horizon test only)
     const uint8_t* visible;  // [ns][nf] their bytes (k_flux_flags), or null
