@@ -113,7 +113,10 @@ __device__ __forceinline__ void put_row(R* row, int ntau, int s, const R (&x)[N]
 template <int MODE, int N>
 __global__ void __launch_bounds__(256) k_single_rows(DevSolve sv, const typename Sa<MODE>::R* lit,
                                                      typename Sa<MODE>::R* next) {
-    using A = Sa<MODE>;
+    // FAST rounds product and sum apart, as the form without rows does (there the
+    // flag is the sum's factor): a forcing one ulp off moves the revolution in
+    // which a facet counts as converged
+    using A = Sa<MODE == MODE_FP64 ? MODE_FP64 : MODE_REF>;
     using R = typename A::R;
     const int f = (gridDim.y - 1 - blockIdx.y) * blockDim.y + threadIdx.y;
     if (f >= sv.nf) return;  // warp-uniform
@@ -301,7 +304,7 @@ __global__ void __launch_bounds__(1024) k_multi_levels(DevSolve sv, GsPlan plan,
 
 // one Jacobi sweep: pn = alb (sp + sum_k v_k po[g_k]) for every (facet, step),
 // rows of gather_ld(ntau); *more = 1 if some |pn - po| > accuracy.  sp = solar x
-// the lit cosine; the list's sum is two partial sums over every other entry.
+// the lit cosine; the list's sum is two fused partial sums over every other entry.
 template <int N>
 __global__ void __launch_bounds__(256) k_multi_jacobi(DevSolve sv, const float* lit, const float* po, float* pn,
                                                       int* more) {
@@ -315,8 +318,8 @@ __global__ void __launch_bounds__(256) k_multi_jacobi(DevSolve sv, const float* 
                   [&](int i, float c, const float(&x)[N]) {
 #pragma unroll
                       for (int u = 0; u < N; ++u) {
-                          if (i & 1) a1[u] += c * x[u];
-                          else a0[u] += c * x[u];
+                          if (i & 1) a1[u] = __fmaf_rn(c, x[u], a1[u]);
+                          else a0[u] = __fmaf_rn(c, x[u], a0[u]);
                       }
                   });
     if (!ok) return;
@@ -327,7 +330,7 @@ __global__ void __launch_bounds__(256) k_multi_jacobi(DevSolve sv, const float* 
     float v[N];
 #pragma unroll
     for (int u = 0; u < N; ++u) {
-        v[u] = sv.alb * (sv.solar * sp[u] + (a0[u] + a1[u]));
+        v[u] = sv.alb * __fadd_rn(__fmul_rn(sv.solar, sp[u]), a0[u] + a1[u]);  // the sunlight is a rounded term
         moved = moved || (s + u < sv.ntau && fabsf(v[u] - old[u]) > sv.sacc);
     }
     Steps<float, N>::put(pn + o, v);
