@@ -545,7 +545,7 @@ atpm_status build_tc(atpm_solve* s, const atpm_shape* sh) {
     build_tc_items(one, 1, q);
     tc_map_extend(q);
     CK(pool_alloc(reinterpret_cast<void**>(&s->qmap), q.size() * sizeof(int4), s->st));
-    CK(cudaMemcpy(s->qmap, q.data(), q.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(upload(s->qmap, q.data(), q.size() * sizeof(int4), s->st));
     s->nq = (int)q.size();  // map entries (items, list, counters)
     return ATPM_OK;
 }
@@ -683,10 +683,11 @@ atpm_status make_batch_for(atpm_solve* const* solves, int n, Batch* out, void** 
     const size_t bq = align256(std::max<size_t>(qm.size(), 1) * sizeof(int4));
     CK(pool_alloc(tmp, bt + bw + bf + bq, s0->st));
     char* t = static_cast<char*>(*tmp);
-    CK(cudaMemcpy(t, tab.data(), n * sizeof(DevSolve), cudaMemcpyHostToDevice));
-    if (!wm.empty()) CK(cudaMemcpy(t + bt, wm.data(), wm.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(t + bt + bw, fm.data(), fm.size() * sizeof(int2), cudaMemcpyHostToDevice));
-    if (!qm.empty()) CK(cudaMemcpy(t + bt + bw + bf, qm.data(), qm.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(t, tab.data(), n * sizeof(DevSolve), cudaMemcpyHostToDevice, s0->st));
+    if (!wm.empty()) CK(cudaMemcpyAsync(t + bt, wm.data(), wm.size() * sizeof(int4), cudaMemcpyHostToDevice, s0->st));
+    if (!qm.empty())
+        CK(cudaMemcpyAsync(t + bt + bw + bf, qm.data(), qm.size() * sizeof(int4), cudaMemcpyHostToDevice, s0->st));
+    CK(upload(t + bt + bw, fm.data(), fm.size() * sizeof(int2), s0->st));
     *out = make_batch(s0->ctx, reinterpret_cast<DevSolve*>(t), n, reinterpret_cast<int4*>(t + bt), (int)wm.size(),
                       reinterpret_cast<int2*>(t + bt + bw), (int)fm.size(), s0->P.precision, s0->P.nx);
     set_tc_map(*out, reinterpret_cast<int4*>(t + bt + bw + bf), qm.size());
@@ -2280,21 +2281,24 @@ ATPM_API atpm_status atpm_selfheating_flux(atpm_solve* s, float* q) {
     if (!s || !q) return fail(ATPM_E_INVALID, "null argument");
     CK(cudaSetDevice(s->ctx->device));
     Ctl c, on{0, 1, 0, 0};
-    CK(cudaMemcpy(&c, s->ds.ctl, sizeof c, cudaMemcpyDeviceToHost));
-    CK(cudaMemcpy(s->ds.ctl, &on, sizeof on, cudaMemcpyHostToDevice));
+    CK(cudaMemcpyAsync(&c, s->ds.ctl, sizeof c, cudaMemcpyDeviceToHost, s->st));
+    CK(cudaStreamSynchronize(s->st));
+    CK(upload(s->ds.ctl, &on, sizeof on, s->st));
     Batch b;
     void* tmp = nullptr;
     atpm_solve* one[1] = {s};
     atpm_status r = make_batch_for(one, 1, &b, &tmp);
-    if (r) return r;
+    if (r) {
+        upload(s->ds.ctl, &c, sizeof c, s->st);
+        return r;
+    }
     // every row block, frozen facets included: the flux of the current
     // temperatures for every facet, not only the ones still advancing
     CK(cudaMemsetAsync(s->ds.rb_act, 1, (size_t)(s->nf + 127) / 128, s->st));
     int rc = launch_revolution_part(b, 0, s->st);
     if (!rc) rc = launch_w_bf16_one(s->ds, s->st);
     if (!rc) rc = launch_revolution_part(b, 1, s->st);
-    CK(cudaStreamSynchronize(s->st));
-    CK(cudaMemcpy(s->ds.ctl, &c, sizeof c, cudaMemcpyHostToDevice));
+    CK(upload(s->ds.ctl, &c, sizeof c, s->st));
     if (rc) return fail(ATPM_E_CUDA, "self-heating launch");
     int st = 0;
     CK(cudaMemcpy(&st, s->ds.status, 4, cudaMemcpyDeviceToHost));

@@ -125,7 +125,7 @@ ATPM_API atpm_status atpm_crater_create(atpm_context* ctx, int32_t nf, int32_t n
         delete c;
         return cfail(ATPM_E_NOMEM, "allocation", e);
     }
-    cudaMemset(c->mem, 0, total);
+    e = cudaMemsetAsync(c->mem, 0, total, c->st);
     char* p = static_cast<char*>(c->mem);
     void* ptr[32];
     for (int i = 0; i < n; ++i) {
@@ -155,7 +155,11 @@ ATPM_API atpm_status atpm_crater_create(atpm_context* ctx, int32_t nf, int32_t n
             mult[q][0] = (float)k - (2.0f / 3.0f);
             mult[q][1] = (float)l - (1.0f / 3.0f);
         }
-    cudaMemcpy((void*)d.cmult, mult, sizeof mult, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = upload((void*)d.cmult, mult, sizeof mult, c->st);
+    if (e != cudaSuccess) {
+        atpm_crater_destroy(c);
+        return cfail(ATPM_E_CUDA, "setup", e);
+    }
     c->PI = 4.0f * std::atan(1.0f);
     d.PI = c->PI;
     d.numrevs = nullptr;
@@ -213,7 +217,7 @@ ATPM_API atpm_status atpm_crater_set_surface(atpm_crater* c, int32_t nsv, const 
     atpm_status r = atpm_crater_set_model(c, nsv, vertices, facets, tri.data(), viewfactors, rot_period);
     if (r) return r;
     if (!c->cnorm) CC(cudaMalloc((void**)&c->cnorm, (size_t)nsf * 12), "allocation");
-    CC(cudaMemcpy(c->cnorm, nrm.data(), (size_t)nsf * 12, cudaMemcpyHostToDevice), "copy");
+    CC(upload(c->cnorm, nrm.data(), (size_t)nsf * 12, c->st), "copy");
     c->d.cnorm = c->cnorm;
     return ATPM_OK;
 }
@@ -382,7 +386,7 @@ ATPM_API atpm_status atpm_crater_set_revolutions(atpm_crater* c, const float* nu
         if (!(numrevs[f] > 0.0f) || !std::isfinite(numrevs[f]))
             return atpm::fail_status(ATPM_E_INVALID, "crater_set_revolutions: revolutions must be positive");
     if (!c->numrevs) CC(cudaMalloc((void**)&c->numrevs, (size_t)c->nf * 4), "allocation");
-    CC(cudaMemcpy(c->numrevs, numrevs, (size_t)c->nf * 4, cudaMemcpyHostToDevice), "copy");
+    CC(upload(c->numrevs, numrevs, (size_t)c->nf * 4, c->st), "copy");
     c->d.numrevs = c->numrevs;
     return ATPM_OK;
 }
@@ -402,10 +406,10 @@ ATPM_API atpm_status atpm_crater_set_model(atpm_crater* c, int32_t nsv, const fl
         if (facets[i] < 0 || facets[i] >= nsv) return atpm::fail_status(ATPM_E_INVALID, "crater_set_model: facet index");
     CC(cudaSetDevice(c->ctx->device), "device");
     if (viewfactors)
-        CC(cudaMemcpy((void*)c->d.V, viewfactors, (size_t)c->nsf * c->nsf * 4, cudaMemcpyHostToDevice), "model");
-    CC(cudaMemcpy((void*)c->d.cverts, vertices, (size_t)nsv * 12, cudaMemcpyHostToDevice), "model");
-    CC(cudaMemcpy((void*)c->d.cfac, facets, (size_t)c->nsf * 12, cudaMemcpyHostToDevice), "model");
-    CC(cudaMemcpy((void*)c->d.ctri, trivectors, (size_t)c->nsf * 24, cudaMemcpyHostToDevice), "model");
+        CC(upload((void*)c->d.V, viewfactors, (size_t)c->nsf * c->nsf * 4, c->st), "model");
+    CC(upload((void*)c->d.cverts, vertices, (size_t)nsv * 12, c->st), "model");
+    CC(upload((void*)c->d.cfac, facets, (size_t)c->nsf * 12, c->st), "model");
+    CC(upload((void*)c->d.ctri, trivectors, (size_t)c->nsf * 24, c->st), "model");
     c->rot = rot_period;
     c->d.rot_period = rot_period;
     c->have_model = true;
@@ -416,9 +420,9 @@ ATPM_API atpm_status atpm_crater_set_properties(atpm_crater* c, const uint8_t* c
                                                 const float* ti) {
     if (!c) return atpm::fail_status(ATPM_E_INVALID, "null crater");
     CC(cudaSetDevice(c->ctx->device), "device");
-    if (converged) CC(cudaMemcpy(c->d.conv, converged, c->nf, cudaMemcpyHostToDevice), "properties");
-    if (albedo) CC(cudaMemcpy((void*)c->d.albedo, albedo, (size_t)c->nf * 4, cudaMemcpyHostToDevice), "properties");
-    if (ti) CC(cudaMemcpy((void*)c->d.ti, ti, (size_t)c->nf * 4, cudaMemcpyHostToDevice), "properties");
+    if (converged) CC(upload(c->d.conv, converged, c->nf, c->st), "properties");
+    if (albedo) CC(upload((void*)c->d.albedo, albedo, (size_t)c->nf * 4, c->st), "properties");
+    if (ti) CC(upload((void*)c->d.ti, ti, (size_t)c->nf * 4, c->st), "properties");
     return ATPM_OK;
 }
 
@@ -441,7 +445,7 @@ ATPM_API atpm_status atpm_crater_set_array(atpm_crater* c, int32_t which, const 
     void* dst[] = {(void*)c->d.shadow, c->d.sfc_shadow, (void*)c->d.illumvec, (void*)c->d.illumangle, c->d.RI,
                    (void*)c->d.RGI, (void*)c->d.RGH};
     const size_t bytes[] = {fs * 4, fss * 4, fs * 12, fss * 4, fss * 4, fss * 4, fss * 4};
-    CC(cudaMemcpy(dst[which], data, bytes[which], cudaMemcpyHostToDevice), "set_array");
+    CC(upload(dst[which], data, bytes[which], c->st), "set_array");
     return ATPM_OK;
 }
 
@@ -486,9 +490,10 @@ ATPM_API atpm_status atpm_crater_set_array_strided(atpm_crater* c, int32_t which
         return atpm::fail_status(ATPM_E_INVALID, "crater_set_array_strided: bad arguments");
     CC(cudaSetDevice(c->ctx->device), "device");
     if (facet_stride == per)
-        CC(cudaMemcpy(dev, base, per * c->nf, cudaMemcpyHostToDevice), "set_array_strided");
+        CC(upload(dev, base, per * c->nf, c->st), "set_array_strided");
     else
-        CC(cudaMemcpy2D(dev, per, base, facet_stride, per, c->nf, cudaMemcpyHostToDevice), "set_array_strided");
+        CC(cudaMemcpy2DAsync(dev, per, base, facet_stride, per, c->nf, cudaMemcpyHostToDevice, c->st), "set_array_strided");
+    CC(cudaStreamSynchronize(c->st), "set_array_strided");
     return ATPM_OK;
 }
 
@@ -529,9 +534,10 @@ ATPM_API atpm_status atpm_crater_zero_temperatures(atpm_crater* c) {
     if (c->nx == 0) return atpm::fail_status(ATPM_E_STATE, "shadow-only crater");
     CC(cudaSetDevice(c->ctx->device), "device");
     const size_t fss = (size_t)c->nf * c->ntau * c->nsf;
-    CC(cudaMemset(c->d.stemp0, 0, fss * 4), "zero");
-    CC(cudaMemset(c->d.stemp1, 0, fss * 4), "zero");
-    CC(cudaMemset(c->d.temp, 0, (size_t)c->nf * (c->nx + 1) * c->nsf * 4), "zero");
+    CC(cudaMemsetAsync(c->d.stemp0, 0, fss * 4, c->st), "zero");
+    CC(cudaMemsetAsync(c->d.stemp1, 0, fss * 4, c->st), "zero");
+    CC(cudaMemsetAsync(c->d.temp, 0, (size_t)c->nf * (c->nx + 1) * c->nsf * 4, c->st), "zero");
+    CC(cudaStreamSynchronize(c->st), "zero");
     return ATPM_OK;
 }
 

@@ -13,6 +13,17 @@
 #include "../../include/atpm.h"
 #include "atpm_internal.h"
 
+namespace atpm {
+// Host memory onto an object's own stream, there when this returns.  A plain
+// cudaMemcpy goes through the default stream and may return while its last part is
+// still on the way from a staging buffer; the objects' streams are non-blocking and
+// do not wait for that, so a kernel behind it could read what was there before.
+inline cudaError_t upload(void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    const cudaError_t e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    return e == cudaSuccess ? cudaStreamSynchronize(st) : e;
+}
+}  // namespace atpm
+
 // launch configuration chosen by the autotuner for one kind of batch
 struct atpm_tune_choice {
     int cond_variant = 4;  // FAST conduction variant (1-3 register budgets, 4 paired facets)

@@ -150,6 +150,7 @@ int build_pow_table(int e, HostPowTab* out, char* err, size_t errlen) {
         return 1;
     }
     ce = cudaMemcpy(d, slots.data(), slots.size() * sizeof(uint2), cudaMemcpyHostToDevice);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize(0);  // the solves' streams do not wait for the default one
     if (ce != cudaSuccess) {
         cudaFree(d);
         std::snprintf(err, errlen, "cudaMemcpy(pow table): %s", cudaGetErrorString(ce));
