@@ -27,8 +27,9 @@
 // body, in the view vector); from them on, cosines come from one reciprocal square
 // root instead of a facet frame, acos and cos, and a wavelength costs one exp and
 // one reciprocal: 13.0 -> 4.1 ms for 21,760 facets, 720 steps and three
-// wavelengths.  A cosine within kSure of 0 or 1 is the stage's to judge
-// (stage_view): there its rounding decides whether a facet or sub-facet counts.
+// wavelengths.  A cosine within kSure of 0 or 1 is formed by the stage's own
+// sequence (stage_view): there its rounding decides whether a facet or sub-facet
+// counts.
 //
 // The rough-surface sum (observe, wise_main.cpp:695-727) replaces each
 // facet's own term by its crater's: the sub-facets with a visible fraction
